@@ -381,7 +381,7 @@ size_t simpfem_oc_work_bytes(void);
  * rho, dc, dv, vol_w, rho_new: device arrays of n doubles; work: device workspace of
  * at least simpfem_oc_work_bytes() bytes.  *change_host = max |rho_new - rho|,
  * *lambda_host the final multiplier, *steps_host the bisection steps (each may be
- * NULL).  Synchronises the stream once per bisection step. */
+ * NULL).  The bisection is one cooperative launch; the stream is synchronised once. */
 int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
                       double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
                       double* change_host, double* lambda_host, int* steps_host, void* stream);

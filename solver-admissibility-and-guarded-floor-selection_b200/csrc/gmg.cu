@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "gmg_impl.h"
+#include "gridcomm.cuh"
 
 namespace simpfem {
 
@@ -42,6 +43,19 @@ const char* last_error() { return g_err.c_str(); }
 
 // ----------------------------------------------------------------------------
 
+
+int grid_sm_count() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  SF_CUDA(cudaGetDevice(&dev));
+  int v = dev < 64 ? cached[dev].load(std::memory_order_relaxed) : 0;
+  if (v == 0) {
+    SF_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    v = std::min(v, kGridMaxBlocks);
+    if (dev < 64) cached[dev].store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
 
 static size_t dsize(DType t) { return t == F64 ? 8 : (t == F32 ? 4 : 2); }
 
