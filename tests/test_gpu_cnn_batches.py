@@ -1,7 +1,6 @@
 """The floor proposer's tiled convolution kernels (csrc/cnn.cu) at batches where
 their blocks are partly empty: two and four samples share a block of the data
-gradients, a weight-gradient block takes one, four or (beyond 148 samples) several
-samples.
+gradients, four and 32 a step of the weight gradients, whose ring holds four steps.
 
 Small batches: float32 sums of at most 34 * 27 (forward, data) or 4096 * 31 terms
 (weight gradients, added in partial sums) against the float64 oracle:
