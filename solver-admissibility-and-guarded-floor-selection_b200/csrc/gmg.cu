@@ -57,6 +57,19 @@ int grid_sm_count() {
   return v;
 }
 
+bool cooperative_available() {
+  static std::atomic<int> cached[64];  // 0 unknown, 1 no, 2 yes
+  int dev = 0;
+  SF_CUDA(cudaGetDevice(&dev));
+  int v = dev < 64 ? cached[dev].load(std::memory_order_relaxed) : 0;
+  if (v == 0) {
+    SF_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev));
+    v = v ? 2 : 1;
+    if (dev < 64) cached[dev].store(v, std::memory_order_relaxed);
+  }
+  return v == 2;
+}
+
 static size_t dsize(DType t) { return t == F64 ? 8 : (t == F32 ? 4 : 2); }
 
 // ----------------------------------------------------------------------------
@@ -617,6 +630,7 @@ void* smooth(Gmg& G, int l, const void* rhs, const void* x_in) {
 // ----------------------------------------------------------------------------
 // Coarsest solve (dense via explicit Cholesky inverse factor, or fixed Jacobi-PCG)
 static void fixed_pcg_coarse(Gmg& G, int l, const double* b, double* x);
+static int coarse_pcg_count(const Gmg& G) { return G.high ? std::max(G.o.coarse_pcg_iters, 200) : G.o.coarse_pcg_iters; }
 
 void solve_coarsest(Gmg& G, const void* rhs, void* x) {
   const int l = G.L - 1;
@@ -625,6 +639,11 @@ void solve_coarsest(Gmg& G, const void* rhs, void* x) {
   if (G.L == 1) {
     void* r = smooth(G, 0, rhs, nullptr);
     if (r != x) SF_CUDA(launch_copy(G.cyc, n, r, x, G.guard, G.st));
+    return;
+  }
+  if (G.coarse_mode == 2 && G.pcg_rows > 0) {
+    SF_CUDA(launch_pcg_coop(G.cyc, G.pcg_rows, L.g, L.K64.as<double>(), L.dinv64.as<double>(), rhs, x,
+                            G.pz.as<double>(), coarse_pcg_count(G), G.pcomm.p, G.guard, G.st));
     return;
   }
   const double* b64 = (const double*)rhs;
@@ -1011,8 +1030,7 @@ void apply_full(Gmg& G, const double* rhs, double* out, const int* guard) {
 static void fixed_pcg_coarse(Gmg& G, int l, const double* b, double* x) {
   Level& L = G.lv[l];
   const int64_t n = L.g.ndof;
-  int iters = G.o.coarse_pcg_iters;
-  if (G.high) iters = std::max(iters, 200);
+  const int iters = coarse_pcg_count(G);
   double* r = G.pr.as<double>();
   double* z = G.pz.as<double>();
   double* p = G.pp.as<double>();
@@ -1234,8 +1252,16 @@ static void setup_coarsest(Gmg& G) {
   }
   G.coarse_mode = 2;
   const int64_t nd = L.g.ndof;
-  G.pr.alloc(8 * nd);
+  G.pcg_rows = pcg_coop_rows(nd, cooperative_available());
   G.pz.alloc(8 * nd);
+  if (G.pcg_rows > 0) {
+    if (!G.pcomm.p) {
+      G.pcomm.alloc(pcg_coop_comm_bytes());
+      SF_CUDA(cudaMemsetAsync(G.pcomm.p, 0, pcg_coop_comm_bytes(), G.st));
+    }
+    return;
+  }
+  G.pr.alloc(8 * nd);
   G.pp.alloc(8 * nd);
   G.pAp.alloc(8 * nd);
 }

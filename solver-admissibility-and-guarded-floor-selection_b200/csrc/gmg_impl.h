@@ -197,6 +197,8 @@ struct Gmg {
   DevBuf cdinv;          // inverses of the diagonal tiles of the coarsest factor (scratch)
   // iterative coarse (fixed PCG) vectors
   DevBuf pr, pz, pp, pAp;
+  DevBuf pcomm;        // exchange slots of the one-launch form
+  int pcg_rows = 0;    // its rows per lane group; 0: the launched form
 
   DevBuf sc;         // scalar scratch of the corrections
   DevBuf rhs64, out64, tmp64a, tmp64b, tmp64c, tmp64d;  // apply-level FP64 vectors
