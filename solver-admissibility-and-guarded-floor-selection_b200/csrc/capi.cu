@@ -155,9 +155,35 @@ int simpfem_mesh_create(int nelx, int nely, int nelz, const int32_t* free_dofs_h
   if (n_free > 0) SF_CUDA(cudaMemcpy(m.free_idx.p, m.free_h.data(), 4 * n_free, cudaMemcpyHostToDevice));
   m.mask.alloc(m.g.ndof);
   SF_CUDA(cudaMemcpy(m.mask.p, m.mask_h.data(), m.g.ndof, cudaMemcpyHostToDevice));
+  {
+    std::vector<uint8_t> bits(m.g.nn);
+    std::vector<int32_t> info(m.g.nn);
+    int64_t first = 0;
+    for (int64_t nd = 0; nd < m.g.nn; ++nd) {
+      const int b0 = m.mask_h[3 * nd], b1 = m.mask_h[3 * nd + 1], b2 = m.mask_h[3 * nd + 2];
+      bits[nd] = (uint8_t)(b0 | b1 << 1 | b2 << 2);
+      info[nd] = (int32_t)(8 * first) + bits[nd];
+      first += b0 + b1 + b2;
+    }
+    m.nmask.alloc(m.g.nn);
+    SF_CUDA(cudaMemcpy(m.nmask.p, bits.data(), m.g.nn, cudaMemcpyHostToDevice));
+    if (n_free < (int64_t(1) << 28)) {
+      const int64_t pn = (int64_t)(nely + 1) * (nelz + 1);
+      std::vector<int32_t> planes(nelx + 1);
+      for (int p = 0; p <= nelx; ++p) {
+        bool all = true;
+        for (int64_t nd = p * pn; nd < (p + 1) * pn && all; ++nd) all = bits[nd] == 7;
+        planes[p] = all ? info[p * pn] >> 3 : -1;
+      }
+      m.ninfo.alloc(4 * m.g.nn);
+      m.pinfo.alloc(4 * planes.size());
+      SF_CUDA(cudaMemcpy(m.ninfo.p, info.data(), 4 * m.g.nn, cudaMemcpyHostToDevice));
+      SF_CUDA(cudaMemcpy(m.pinfo.p, planes.data(), 4 * planes.size(), cudaMemcpyHostToDevice));
+    }
+  }
   m.init_red();
-  m.sh[0] = default_shape(m.g, 256);
-  m.sh[1] = default_shape(m.g, 512);
+  m.sh[0] = default_shape(F64, m.g);
+  m.sh[1] = default_shape(F32, m.g);
   *out = h;
   SF_API_END
 }
@@ -201,6 +227,11 @@ int simpfem_matvec(simpfem_mesh* mh, int dtype, const void* E, const void* u_fre
   const DType t = api_dtype(dtype);
   if (t == BF16) throw InvalidArg{"simpfem_matvec: dtype must be F64 or F32"};
   const size_t es = t == F64 ? 8 : 4;
+  if (t == F64 && m.ninfo.p && u_free != y_free) {
+    SF_CUDA(launch_fine_compact(m.g, m.sh[0], (const double*)E, m.ninfo.as<int32_t>(), m.pinfo.as<int32_t>(),
+                                (const double*)u_free, (double*)y_free, S(stream)));
+    return SIMPFEM_OK;
+  }
   m.ufull.alloc(8 * m.g.ndof);
   m.yfull.alloc(8 * m.g.ndof);
   SF_CUDA(cudaMemsetAsync(m.ufull.p, 0, es * m.g.ndof, S(stream)));

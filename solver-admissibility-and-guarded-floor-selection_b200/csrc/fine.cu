@@ -7,32 +7,60 @@
 //
 //  * Node indices are computed from (i, j, k); there is no edof table.
 //  * A block owns a (bj-1) x (bk-1) patch of node columns (one halo element
-//    column on the low j and k sides) and sweeps cx node planes along x.  Each
-//    thread computes one element per plane and carries the element's +x face
-//    contribution in registers to the next plane, so every element is
-//    evaluated once per sweep (plus the halo columns).
+//    column on the low j and k sides) and sweeps cx node planes along x, so
+//    every element is evaluated once per sweep (plus the halo columns).
 //  * The element product KE * u_e uses the reflection symmetry of the unit
 //    cube: in the Walsh (+/-1) basis over the element's 2x2x2 nodes the 24x24
-//    unit stiffness is block diagonal with eight 3x3 blocks, so
-//    KE u = H (B (H u)) costs 72 add + 72 FMA + 72 add instead of 576 FMA.
+//    unit stiffness is block diagonal with eight 3x3 blocks, of which six couple
+//    only two of their three modes (an isotropic material; checked when the
+//    stiffness is installed): 48 products instead of 576.  The transform is
+//    separable, so a node plane is transformed along y and z once for the two
+//    element planes it bounds, and the two face sums that meet on it are added
+//    before they are transformed back.
 //  * Per-node sums are reduced in shared memory in a fixed order (no atomics),
 //    and the caller's epilogue (residual, Chebyshev or Jacobi update) is fused
 //    into the store.
 #include <stdio.h>
 
 #include "common.cuh"
+#include "gmg_impl.h"
 
 namespace simpfem {
 
 __constant__ double c_wht64[8][9];
-__constant__ float c_wht32[8][9];
-__constant__ float2 c_wht32x2[8][9];  // c_wht32 duplicated into both lanes of a pair
-__constant__ float c_keb16[576];   // KE rounded to bf16 (stored as float), corner-major order
+__constant__ float2 c_wht32[4][9];   // FP32 blocks 2h and 2h + 1 as the lanes of a pair
+__constant__ float2 c_whtb32[4][9];  // the same for KE with its entries rounded to bf16
 __constant__ double c_kediag[24];  // KE diagonal, corner-major order
 __constant__ double c_kenb[8][9];  // 3x3 node-diagonal blocks of KE per corner
 
 // corner q = dx * 4 + dy * 2 + dz  <->  reference local node (gpu_fem/pub_simp_solver.py:196-207)
 static const int kRefNodeOfCorner[8] = {0, 4, 3, 7, 1, 5, 2, 6};
+
+// Pattern of the Walsh blocks of an isotropic stiffness: blocks 0 and 7 are full,
+// the others couple two modes and leave the third (lone_mode) by itself.
+__host__ __device__ constexpr int lone_mode(int b) { return b == 1 || b == 6 ? 2 : (b == 2 || b == 5 ? 1 : 0); }
+__host__ __device__ constexpr bool block_entry(int b, int r, int c) {
+  return b == 0 || b == 7 || r == c || (r != lone_mode(b) && c != lone_mode(b));
+}
+static bool has_pattern(const WhtBlocks& wb) {
+  double mx = 0.0, off = 0.0;
+  for (int b = 0; b < 8; ++b)
+    for (int i = 0; i < 9; ++i) {
+      const double v = fabs(wb.b[b][i]);
+      mx = v > mx ? v : mx;
+      if (!block_entry(b, i / 3, i % 3)) off = v > off ? v : off;
+    }
+  return off <= 1e-15 * mx;  // a few roundings of the largest entry
+}
+// Whether the stiffness installed on a device has the pattern (FP64 products skip the
+// other entries; the packed FP32 ones pair two blocks and take them all); written
+// with the constants, which all meshes of a device share.
+static std::atomic<int> g_pattern[64];
+static bool pattern_on_device() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return dev < 64 && g_pattern[dev].load(std::memory_order_acquire) != 0;
+}
 
 void set_fine_constants(const double* ke576, const WhtBlocks& wb) {
   // KE in corner-major order: row (q * 3 + c) <- reference row (3 * a(q) + c)
@@ -43,43 +71,41 @@ void set_fine_constants(const double* ke576, const WhtBlocks& wb) {
         for (int c2 = 0; c2 < 3; ++c2)
           kem[(q * 3 + c) * 24 + q2 * 3 + c2] =
               ke576[(3 * kRefNodeOfCorner[q] + c) * 24 + 3 * kRefNodeOfCorner[q2] + c2];
-  float keb[576];
-  for (int i = 0; i < 576; ++i) keb[i] = __bfloat162float(__float2bfloat16_rn((float)kem[i]));
+  // KE with bf16-rounded entries keeps the reflection symmetry (mirrored entries
+  // round alike), so it has Walsh blocks of its own
+  double keb[576];
+  for (int i = 0; i < 576; ++i) keb[i] = (double)__bfloat162float(__float2bfloat16_rn((float)ke576[i]));
+  double boff = 0.0;
+  const WhtBlocks wbb = make_wht_blocks(keb, &boff);
   double kd[24];
   for (int i = 0; i < 24; ++i) kd[i] = kem[i * 24 + i];
   double nb[8][9];
   for (int q = 0; q < 8; ++q)
     for (int r = 0; r < 3; ++r)
       for (int c = 0; c < 3; ++c) nb[q][r * 3 + c] = kem[(q * 3 + r) * 24 + q * 3 + c];
-  float w32[8][9];
-  for (int b = 0; b < 8; ++b)
-    for (int i = 0; i < 9; ++i) w32[b][i] = (float)wb.b[b][i];
+  float2 w32[4][9], wb32[4][9];
+  for (int h = 0; h < 4; ++h)
+    for (int i = 0; i < 9; ++i) {
+      w32[h][i] = make_float2((float)wb.b[2 * h][i], (float)wb.b[2 * h + 1][i]);
+      wb32[h][i] = make_float2((float)wbb.b[2 * h][i], (float)wbb.b[2 * h + 1][i]);
+    }
   SF_CUDA(cudaMemcpyToSymbol(c_wht64, wb.b, sizeof(wb.b)));
   SF_CUDA(cudaMemcpyToSymbol(c_wht32, w32, sizeof(w32)));
-  float2 w32x2[8][9];
-  for (int b = 0; b < 8; ++b)
-    for (int i = 0; i < 9; ++i) w32x2[b][i] = make_float2(w32[b][i], w32[b][i]);
-  SF_CUDA(cudaMemcpyToSymbol(c_wht32x2, w32x2, sizeof(w32x2)));
-  SF_CUDA(cudaMemcpyToSymbol(c_keb16, keb, sizeof(keb)));
+  SF_CUDA(cudaMemcpyToSymbol(c_whtb32, wb32, sizeof(wb32)));
   SF_CUDA(cudaMemcpyToSymbol(c_kediag, kd, sizeof(kd)));
   SF_CUDA(cudaMemcpyToSymbol(c_kenb, nb, sizeof(nb)));
+  int dev = 0;
+  SF_CUDA(cudaGetDevice(&dev));
+  if (dev < 64) g_pattern[dev].store(has_pattern(wb) ? 1 : 0, std::memory_order_release);
 }
 
-template <typename T>
-__device__ __forceinline__ T wht_coef(int b, int i);
-template <>
-__device__ __forceinline__ double wht_coef<double>(int b, int i) { return c_wht64[b][i]; }
-template <>
-__device__ __forceinline__ float wht_coef<float>(int b, int i) { return c_wht32[b][i]; }
-
-template <typename T>
-__device__ __forceinline__ void wht8(T a[8]) {
+__device__ __forceinline__ void wht8(double a[8]) {
 #pragma unroll
   for (int m = 4; m >= 1; m >>= 1) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       if ((q & m) == 0) {
-        T p = a[q], r = a[q | m];
+        const double p = a[q], r = a[q | m];
         a[q] = p + r;
         a[q | m] = p - r;
       }
@@ -87,23 +113,22 @@ __device__ __forceinline__ void wht8(T a[8]) {
   }
 }
 
-// f = E * KE * u for one element, u/f indexed [corner][component].
-template <typename T>
-__device__ __forceinline__ void elem_wht(const T (&u)[8][3], T E, T (&f)[8][3]) {
-  T w[3][8];
+// f = KE * u for one element, u/f indexed [corner][component].
+__device__ __forceinline__ void elem_wht(const double (&u)[8][3], double (&f)[8][3]) {
+  double w[3][8];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) w[c][q] = u[q][c];
     wht8(w[c]);
   }
-  T v[3][8];
+  double v[3][8];
 #pragma unroll
   for (int b = 0; b < 8; ++b) {
-    const T in0 = w[0][b ^ 4], in1 = w[1][b ^ 2], in2 = w[2][b ^ 1];
-    v[0][b ^ 4] = E * (wht_coef<T>(b, 0) * in0 + wht_coef<T>(b, 1) * in1 + wht_coef<T>(b, 2) * in2);
-    v[1][b ^ 2] = E * (wht_coef<T>(b, 3) * in0 + wht_coef<T>(b, 4) * in1 + wht_coef<T>(b, 5) * in2);
-    v[2][b ^ 1] = E * (wht_coef<T>(b, 6) * in0 + wht_coef<T>(b, 7) * in1 + wht_coef<T>(b, 8) * in2);
+    const double in0 = w[0][b ^ 4], in1 = w[1][b ^ 2], in2 = w[2][b ^ 1];
+    v[0][b ^ 4] = c_wht64[b][0] * in0 + c_wht64[b][1] * in1 + c_wht64[b][2] * in2;
+    v[1][b ^ 2] = c_wht64[b][3] * in0 + c_wht64[b][4] * in1 + c_wht64[b][5] * in2;
+    v[2][b ^ 1] = c_wht64[b][6] * in0 + c_wht64[b][7] * in1 + c_wht64[b][8] * in2;
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -113,33 +138,88 @@ __device__ __forceinline__ void elem_wht(const T (&u)[8][3], T E, T (&f)[8][3]) 
   }
 }
 
-// f = E * (KE_bf16 @ bf16(u)) with FP32 accumulation (the reference's BF16 WMMA
-// semantics, gpu_fem/cuda_fused_matvec.py:112-246).
-__device__ __forceinline__ void elem_bf16(const float (&u)[8][3], float E, float (&f)[8][3]) {
-  float ub[24];
+// FP32 runs on the packed pair instructions of sm_100 (half the issue slots), the
+// lanes of a pair being z: the nodes dz = 0, 1 of a corner pair, or the z parities
+// 0, 1 of a transformed value.  Only the z butterflies cross lanes.  Block b pairs
+// value b ^ 4 of component 0 with b ^ 2 of component 1 and b ^ 1 of component 2, so
+// with component 2 kept in swapped lanes blocks 2h and 2h + 1 are one pair.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 zbutterfly(float2 a) { return make_float2(__fadd_rn(a.x, a.y), __fsub_rn(a.x, a.y)); }
+__device__ __forceinline__ float2 swap2(float2 a) { return make_float2(a.y, a.x); }
+
+// The eight blocks: w[c][2 sx + sy] (component 2 swapped) -> v in the same layout.
+// RN: each row is product, fused multiply-add, fused multiply-add; otherwise the
+// order that contracting c0 in0 + c1 in1 + c2 in2 from the left gives.
+template <bool RN, bool BF>
+__device__ __forceinline__ void blocks2(const float2 (&w)[3][4], float2 (&v)[3][4]) {
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
+  for (int h = 0; h < 4; ++h) {
+    const float2 in0 = w[0][h ^ 2], in1 = w[1][h ^ 1], in2 = w[2][h];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) ub[q * 3 + c] = __bfloat162float(__float2bfloat16_rn(u[q][c]));
-#pragma unroll
-  for (int i = 0; i < 24; ++i) {
-    float acc = 0.f;
-#pragma unroll
-    for (int j = 0; j < 24; ++j) acc = fmaf(c_keb16[j * 24 + i], ub[j], acc);
-    f[i / 3][i % 3] = E * acc;
+    for (int r = 0; r < 3; ++r) {
+      const float2* c = BF ? c_whtb32[h] : c_wht32[h];
+      float2 a;
+      if (RN) {
+        a = __fmul2_rn(c[3 * r], in0);
+        a = __ffma2_rn(c[3 * r + 1], in1, a);
+      } else {
+        a = __fmul2_rn(c[3 * r + 1], in1);
+        a = __ffma2_rn(c[3 * r], in0, a);
+      }
+      a = __ffma2_rn(c[3 * r + 2], in2, a);
+      v[r][r == 0 ? h ^ 2 : (r == 1 ? h ^ 1 : h)] = a;
+    }
   }
 }
 
-// Each block stages its (bj+1) x (bk+1) node tile of one x-plane in shared
-// memory: a tile row is 3 (bk+1) consecutive values of u, so the block reads it
-// with coalesced loads, one value per thread and row (no node is read four
-// times).  Thread t loads the values t, t + NT, ... of the flattened tile; the
-// offsets do not depend on the plane and are computed once.
-constexpr int kTileLoads = 6;  // enough for every shape with bj >= 2, bk >= 3; launch checks
-constexpr int kPlaneBufs = 4;  // node-plane tiles: two being read, two in flight
+// f = E * KE * u for one element: lo and hi are its faces at dx = 0 and 1, node pairs
+// [component][dy].  RN: every operation is rounded by itself; otherwise the modulus
+// is contracted into the first back-transform butterfly.
+template <bool RN>
+__device__ __forceinline__ void element_product2(const float2 (&ulo)[3][2], const float2 (&uhi)[3][2], float E,
+                                                 float2 (&flo)[3][2], float2 (&fhi)[3][2]) {
+  float2 w[3][4], v[3][4];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float2 s0 = add2(ulo[q][0], uhi[q][0]), s1 = add2(ulo[q][1], uhi[q][1]);
+    const float2 d0 = sub2(ulo[q][0], uhi[q][0]), d1 = sub2(ulo[q][1], uhi[q][1]);
+    w[q][0] = zbutterfly(add2(s0, s1));
+    w[q][1] = zbutterfly(sub2(s0, s1));
+    w[q][2] = zbutterfly(add2(d0, d1));
+    w[q][3] = zbutterfly(sub2(d0, d1));
+    if (q == 2) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) w[q][s] = swap2(w[q][s]);
+    }
+  }
+  blocks2<RN, false>(w, v);
+  const float2 E2 = make_float2(E, E);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    float2 s[2], d[2];
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const float2 r = __fmul2_rn(E2, v[q][2 + y]);
+      if (RN) {
+        const float2 p = __fmul2_rn(E2, v[q][y]);
+        s[y] = add2(p, r);
+        d[y] = sub2(p, r);
+      } else {
+        s[y] = __ffma2_rn(E2, v[q][y], r);
+        d[y] = __ffma2_rn(E2, v[q][y], make_float2(-r.x, -r.y));
+      }
+    }
+    const float2 a0 = add2(s[0], s[1]), a1 = sub2(s[0], s[1]), b0 = add2(d[0], d[1]), b1 = sub2(d[0], d[1]);
+    flo[q][0] = zbutterfly(q == 2 ? swap2(a0) : a0);
+    flo[q][1] = zbutterfly(q == 2 ? swap2(a1) : a1);
+    fhi[q][0] = zbutterfly(q == 2 ? swap2(b0) : b0);
+    fhi[q][1] = zbutterfly(q == 2 ? swap2(b1) : b1);
+  }
+}
 
-// One element copied global -> shared asynchronously (cp.async; zero-filled when
-// ok is false, reading nothing from src, which is then any valid address).
+// One value copied global -> shared asynchronously (cp.async; zero-filled when ok
+// is false, reading nothing from src, which is then any valid address).
 template <typename T>
 __device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool ok) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -151,17 +231,257 @@ __device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool ok) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;\n" ::); }
 
-template <typename T, int EPI, int KMODE, int MAXT>
-__global__ void __launch_bounds__(MAXT) fine_sweep_kernel(Grid g, SweepShape sh, const T* __restrict__ E,
-                                                          const uint8_t* __restrict__ mask,
-                                                          const T* __restrict__ u, EpiArgs ea) {
+// One face of an element column at a node plane (12 values): with FORM kFaces
+// transformed along z and y -- v[component][2 a + b], a the y and b the z parity
+// (FP32: component 2 with b swapped) --, else its node values v[component][2 dy + dz].
+enum SweepForm { kFaces = 0, kElementRn = 1, kElement = 2 };
+
+template <bool BF, int FORM>
+__device__ __forceinline__ void face_values(const double* r0, const double* r1, double (&v)[3][4], double (&own)[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    own[q] = r0[q];
+    const double n00 = own[q], n01 = r0[3 + q], n10 = r1[q], n11 = r1[3 + q];
+    const double s0 = n00 + n01, d0 = n00 - n01, s1 = n10 + n11, d1 = n10 - n11;
+    v[q][0] = s0 + s1;
+    v[q][1] = d0 + d1;
+    v[q][2] = s0 - s1;
+    v[q][3] = d0 - d1;
+  }
+}
+template <bool BF>
+__device__ __forceinline__ float operand(float v) {  // the BF16 operator rounds its operands
+  return BF ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+}
+template <bool BF, int FORM>
+__device__ __forceinline__ void face_values(const float* r0, const float* r1, float (&v)[3][4], float (&own)[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    own[q] = r0[q];
+    const float2 a = make_float2(operand<BF>(own[q]), operand<BF>(r0[3 + q]));
+    const float2 b = make_float2(operand<BF>(r1[q]), operand<BF>(r1[3 + q]));
+    float2 p = a, m = b;
+    if (FORM == kFaces) {
+      p = zbutterfly(add2(a, b));
+      m = zbutterfly(sub2(a, b));
+      if (q == 2) {
+        p = swap2(p);
+        m = swap2(m);
+      }
+    }
+    v[q][0] = p.x;
+    v[q][1] = p.y;
+    v[q][2] = m.x;
+    v[q][3] = m.y;
+  }
+}
+
+// The element between faces p (low x) and c (high x): its contributions lo and hi to
+// them, in the faces' representation, scaled by the modulus E.
+template <bool DENSE, bool BF, int FORM>
+__device__ __forceinline__ void element_faces(const double (&p)[3][4], const double (&c)[3][4], double E,
+                                              double (&lo)[3][4], double (&hi)[3][4]) {
+  double w[3][8], v[3][8];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      w[q][s] = p[q][s] + c[q][s];
+      w[q][4 + s] = p[q][s] - c[q][s];
+    }
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const double in[3] = {w[0][b ^ 4], w[1][b ^ 2], w[2][b ^ 1]};
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      double acc = 0.0;
+      bool first = true;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (!DENSE && !block_entry(b, r, k)) continue;
+        const double co = c_wht64[b][3 * r + k];
+        acc = first ? co * in[k] : fma(co, in[k], acc);
+        first = false;
+      }
+      v[r][b ^ (4 >> r)] = E * acc;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      lo[q][s] = v[q][s] + v[q][4 + s];
+      hi[q][s] = v[q][s] - v[q][4 + s];
+    }
+}
+template <bool DENSE, bool BF, int FORM>
+__device__ __forceinline__ void element_faces(const float (&p)[3][4], const float (&c)[3][4], float E,
+                                              float (&lo)[3][4], float (&hi)[3][4]) {
+  float2 a[3][2], b[3][2], l[3][2], h[3][2];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      a[q][y] = make_float2(p[q][2 * y], p[q][2 * y + 1]);
+      b[q][y] = make_float2(c[q][2 * y], c[q][2 * y + 1]);
+    }
+  if constexpr (FORM == kFaces) {
+    float2 w[3][4], v[3][4];
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        w[q][y] = add2(a[q][y], b[q][y]);
+        w[q][2 + y] = sub2(a[q][y], b[q][y]);
+      }
+    blocks2<true, BF>(w, v);
+    const float2 E2 = make_float2(E, E);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const float2 r = __fmul2_rn(E2, v[q][2 + y]);
+        l[q][y] = __ffma2_rn(E2, v[q][y], r);
+        h[q][y] = __ffma2_rn(E2, v[q][y], make_float2(-r.x, -r.y));
+      }
+  } else {
+    element_product2<FORM == kElementRn>(a, b, E, l, h);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      lo[q][2 * y] = l[q][y].x;
+      lo[q][2 * y + 1] = l[q][y].y;
+      hi[q][2 * y] = h[q][y].x;
+      hi[q][2 * y + 1] = h[q][y].y;
+    }
+}
+
+// A face's sum t (one component) as its four corners f[2 dy + dz].
+template <int FORM>
+__device__ __forceinline__ void face_corners(const double (&t)[4], int, double (&f)[4]) {
+  const double s0 = t[0] + t[1], d0 = t[0] - t[1], s1 = t[2] + t[3], d1 = t[2] - t[3];
+  f[0] = s0 + s1;
+  f[1] = d0 + d1;
+  f[2] = s0 - s1;
+  f[3] = d0 - d1;
+}
+template <int FORM>
+__device__ __forceinline__ void face_corners(const float (&t)[4], int q, float (&f)[4]) {
+  float2 a = make_float2(t[0], t[1]), b = make_float2(t[2], t[3]);
+  if (FORM == kFaces) {
+    if (q == 2) {
+      a = swap2(a);
+      b = swap2(b);
+    }
+    const float2 e = zbutterfly(a), o = zbutterfly(b);
+    a = add2(e, o);
+    b = sub2(e, o);
+  }
+  f[0] = a.x;
+  f[1] = a.y;
+  f[2] = b.x;
+  f[3] = b.y;
+}
+
+// Vectors an epilogue reads per DOF besides the operator's own output and input.
+template <int EPI>
+constexpr int epi_operands() {
+  return EPI == EPI_APPLY ? 0 : (EPI == EPI_RESID ? 1 : (EPI == EPI_CHEB ? 3 : 2));
+}
+
+// The epilogues of one node: operands o[0..2] = b, o[3..5] = dinv, o[6..8] = d,
+// staged by the thread itself; evaluates epilogue()'s expressions.  off: first DOF
+// of the node, fr its free bits.
+template <typename T, int EPI>
+__device__ __forceinline__ void node_epilogue(const EpiArgs& ea, int64_t off, unsigned fr, const T* o, const T (&ku)[3],
+                                              const T (&x)[3]) {
+  T* py = (EPI == EPI_APPLY || EPI == EPI_RESID ? (T*)ea.y : (T*)ea.xo) + off;
+  T* pd = (T*)ea.d + off;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const bool f = (fr >> c) & 1;
+    T r = T(0), d = T(0);
+    if (EPI == EPI_APPLY) {
+      r = ku[c];
+    } else if (EPI == EPI_RESID) {
+      r = sub_rn(o[c], ku[c]);
+    } else if (EPI == EPI_CHEB1) {
+      d = mul_rn(o[3 + c], sub_rn(o[c], ku[c]));
+      r = add_rn(x[c], mul_rn((T)ea.s1, d));
+    } else if (EPI == EPI_CHEB) {
+      const T z = mul_rn(o[3 + c], sub_rn(o[c], ku[c]));
+      d = mul_rn((T)ea.s1, add_rn(z, mul_rn((T)ea.s2, o[6 + c])));
+      r = add_rn(x[c], d);
+    } else {
+      r = add_rn(x[c], mul_rn(mul_rn((T)ea.s1, o[3 + c]), sub_rn(o[c], ku[c])));
+    }
+    py[c] = f ? r : T(0);
+    if (EPI == EPI_CHEB1 || EPI == EPI_CHEB) pd[c] = f ? d : T(0);
+  }
+}
+
+constexpr int kSweepThreads = 128;  // of a block at most
+constexpr int kPlaneBufs = 4;       // node-plane tiles: one being read, two in flight, one just read
+constexpr int kTileLoads = 8;       // values of a plane tile staged per thread at most; launch checks
+
+// Blocks of 128 threads resident per SM, as the registers allow without spills:
+// three in FP64 (168 registers), four in FP32 (at most 128; five at 96 spilled up to 56
+// bytes: 31.7 us for the operator of 1M elements, four 28.3).
+template <typename T, bool DENSE>
+constexpr int sweep_resident() { return sizeof(T) == 8 ? (DENSE ? 2 : 3) : 4; }
+
+// Each block stages its (bj+1) x (bk+1) node tile of one x-plane in shared memory
+// with asynchronous copies, one value each, consecutive threads on consecutive
+// values of a tile row; values outside the mesh are zeroed once (their set is the
+// same for every plane).  The epilogue's operands of a plane come the same way, one
+// plane ahead, into slots of the thread's own: read by plain loads they cost an L2
+// round trip per plane between the barrier and the update.  Element plane ie couples
+// node planes ie and ie + 1; of those only ie + 1 is read (plane ie is still in registers, transformed).  One
+// barrier per plane: it makes plane ie + 2 visible (every thread waits for its own
+// copies first), frees the buffer of plane ie - 1 and publishes the face sums,
+// which alternate between two buffers.
+//
+// The kernel is bound by the issue of its ~300 instructions per warp and plane and
+// by the latency between them, not by memory: the products and transforms are 190
+// of them, and addresses are running pointers and immediate offsets (the face sums
+// are stored nine to an element for that reason: 9 words apart is also free of bank
+// conflicts in both types).
+//
+// Operator of 1M elements: FP64 87 us before (42 now; its 58 MB at 6.6 TB/s take
+// 9), FP32 45 (28); 512k: FP64 50 (31), FP32 24 (20); 2M in FP32 101 (50).
+//
+// FORM: how an element's product is evaluated.  kFaces transforms a face once for
+// two elements, as above.  The FP32 smoothing steps and residuals of the cycle keep
+// the element-by-element evaluation instead: on states with many void elements a
+// solve carries FP32 rounding differences of the cycle to 1e-7 of the displacement's
+// largest entries, and its answers are to stay the same to the last bit.  Two such
+// forms exist, by grid size (launch_sweep): the compiler's contraction of the plain
+// expressions up to kFusedElements, every operation rounded by itself beyond.  They
+// take about 1.4 times the arithmetic of kFaces.
+//
+// COMPACT: u and y are the free-DOF vectors of the C interface, so neither an
+// expanded copy of u nor a full result is written.  pinfo[plane] is the free index
+// of the first DOF of a node plane that is wholly free -- its values then lie as in
+// the full layout --, -1 otherwise; on those planes (supports) ninfo[node] gives 8 *
+// (free index of the node's first free DOF) + its three free bits.
+constexpr int64_t kFusedElements = 250000;
+
+template <typename T, int EPI, bool DENSE, bool BF, bool COMPACT, int FORM>
+__global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE>())
+    sweep_kernel(Grid g, SweepShape sh, const T* __restrict__ E, const uint8_t* __restrict__ nmask,
+                 const T* __restrict__ u, const int32_t* __restrict__ ninfo,
+                 const int32_t* __restrict__ pinfo, EpiArgs ea) {
   if (guard_off(ea.guard)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NT = sh.bj * sh.bk;
-  const int W = 3 * (sh.bk + 1);   // values per tile row
-  const int PV = (sh.bj + 1) * W;  // values per plane tile
-  T* F = reinterpret_cast<T*>(smem_raw);  // face sums [2][12][NT]
-  T* P = F + 24 * NT;                     // node-plane tiles [kPlaneBufs][PV]
+  const int W = 3 * (sh.bk + 1);           // values per tile row
+  const int PV = (sh.bj + 1) * W;          // one plane tile
+  constexpr int NO = 3 * epi_operands<EPI>();
+  T* F = reinterpret_cast<T*>(smem_raw);   // face sums [2][NT][9]
+  T* P = F + 18 * NT;                      // plane tiles [kPlaneBufs][PV]
+  T* O = P + kPlaneBufs * PV;              // epilogue operands [2][NT][NO]
   const int t = threadIdx.x;
   const int tj = t / sh.bk, tk = t - tj * sh.bk;
   const int nbk = (g.nz + sh.bk - 1) / (sh.bk - 1);  // ceil((nz+1)/(bk-1))
@@ -169,445 +489,252 @@ __global__ void __launch_bounds__(MAXT) fine_sweep_kernel(Grid g, SweepShape sh,
   const int jb = bjI * (sh.bj - 1) - 1;  // first tile node row = first element row (a halo)
   const int kb = bkI * (sh.bk - 1) - 1;
   const int je = jb + tj, ke = kb + tk;
-  const int i0 = blockIdx.y * sh.cx;
-  const int i1 = min(i0 + sh.cx, g.nx + 1);
+  const int i0 = blockIdx.y * sh.cx, i1 = min(i0 + sh.cx, g.nx + 1);
   const bool colv = je >= 0 && je < g.ny && ke >= 0 && ke < g.nz;
-  const bool own = tj >= 1 && tk >= 1 && je <= g.ny && ke <= g.nz;
-  const int64_t NZ1 = g.nz + 1;
-  const int64_t plane_vals = 3 * (int64_t)(g.ny + 1) * NZ1;
+  const bool own_node = tj >= 1 && tk >= 1 && je <= g.ny && ke <= g.nz;
+  const int NZ1 = g.nz + 1, plane_nodes = (g.ny + 1) * NZ1;
+  const int last = min(i1, g.nx);  // last node plane read
 
+  // tile values t, t + NT, ...: DOF offset in a plane, the same for every plane
   int rel[kTileLoads];
-  bool okq[kTileLoads];
+  unsigned okm = 0;
 #pragma unroll
   for (int q = 0; q < kTileLoads; ++q) {
+    rel[q] = 0;
     const int v = t + q * NT;
-    const int row = v / W, col = v - row * W;
-    const int j = jb + row, k = kb + col / 3;
-    okq[q] = v < PV && j >= 0 && j <= g.ny && k >= 0 && k <= g.nz;
-    rel[q] = okq[q] ? (int)(3 * ((int64_t)j * NZ1 + kb) + col) : 0;
-  }
-  // node plane p (zeros outside the mesh) into tile buffer p mod kPlaneBufs,
-  // asynchronously; every call commits one copy group
-  auto issue_plane = [&](int p) {
-    const bool pv = p >= 0 && p <= g.nx;
-    const int64_t base = pv ? (int64_t)p * plane_vals : 0;
-    T* dst = P + (p & (kPlaneBufs - 1)) * PV;
-#pragma unroll
-    for (int q = 0; q < kTileLoads; ++q) {
-      const int v = t + q * NT;
-      if (q * NT < PV && v < PV) {
-        const bool ok = pv && okq[q];
-        cp_async_elem(dst + v, ok ? u + base + rel[q] : u, ok);
-      }
-    }
-    cp_async_commit();
-  };
-  auto read_face = [&](int buf, T (&uu)[4][3]) {
-    const T* src = P + buf * PV;
-#pragma unroll
-    for (int q2 = 0; q2 < 4; ++q2) {
-      const int idx = (tj + (q2 >> 1)) * W + (tk + (q2 & 1)) * 3;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) uu[q2][c] = src[idx + c];
-    }
-  };
-  auto e_index = [&](int ie) { return ((int64_t)ie * g.ny + je) * g.nz + ke; };
-
-  // prologue: planes i0-1 and i0 in the tile buffers, plane i0+1 in flight
-  issue_plane(i0 - 1);
-  issue_plane(i0);
-  if (i0 + 1 <= i1) issue_plane(i0 + 1);
-  else cp_async_commit();
-  cp_async_wait_all_but_one();
-  T Enext = (colv && i0 - 1 >= 0 && i0 - 1 < g.nx) ? E[e_index(i0 - 1)] : T(0);
-  T carry[4][3];
-#pragma unroll
-  for (int q2 = 0; q2 < 4; ++q2)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) carry[q2][c] = T(0);
-  __syncthreads();
-
-  // Element plane ie couples node planes ie and ie + 1, both read from the
-  // rotating tile buffers (plane q in buffer q mod 4).  One barrier per plane:
-  // the copy of plane ie + 3 is issued at the top (its buffer held plane ie - 1,
-  // last read before the previous barrier), and before the barrier every thread
-  // waits for its copies of plane ie + 2, so after it the next iteration's two
-  // planes are complete and visible; the face sums alternate between two buffers.
-  for (int ie = i0 - 1; ie < i1; ++ie) {
-    if (ie + 3 <= i1) issue_plane(ie + 3);
-    else cp_async_commit();
-    const T Ee = Enext;
-    Enext = (colv && ie + 1 < g.nx) ? E[e_index(ie + 1)] : T(0);
-    const bool do_epi = own && ie >= i0;
-    int64_t node = 0;
-    if (do_epi) node = ((int64_t)ie * (g.ny + 1) + je) * NZ1 + ke;
-    EpiOperands<T, EPI> eo;
-    if (do_epi) eo.load(ea, 3 * node, mask);
-    const int blo = ie & (kPlaneBufs - 1), bhi = (ie + 1) & (kPlaneBufs - 1);
-    // the node's own value, read before the barrier: after it the next
-    // iteration may overwrite this plane's buffer
-    T xv[3];
-    if (do_epi) {
-      const T* xs = P + blo * PV + tj * W + tk * 3;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) xv[c] = xs[c];
-    }
-    T f[8][3];
-    if (colv && ie >= 0 && ie < g.nx) {
-      T ue[8][3];
-      read_face(blo, reinterpret_cast<T(&)[4][3]>(ue[0]));
-      read_face(bhi, reinterpret_cast<T(&)[4][3]>(ue[4]));
-      if (KMODE == 0) {
-        elem_wht<T>(ue, Ee, f);
+    if (v < PV) {
+      const int row = v / W, col = v - row * W;
+      const int j = jb + row, k = kb + col / 3;
+      if (j >= 0 && j <= g.ny && k >= 0 && k <= g.nz) {
+        okm |= 1u << q;
+        rel[q] = 3 * (j * NZ1 + kb) + col;
       } else {
-        elem_bf16(reinterpret_cast<const float(&)[8][3]>(ue), (float)Ee, reinterpret_cast<float(&)[8][3]>(f));
+#pragma unroll
+        for (int p = 0; p < kPlaneBufs; ++p) P[p * PV + v] = T(0);
       }
+    }
+  }
+  // node plane p into its tile buffer; first: pinfo[p] (COMPACT)
+  auto issue_plane = [&](int p, int first) {
+    T* dst = P + (p & (kPlaneBufs - 1)) * PV + t;
+    if (COMPACT && first < 0) {
+      const int32_t* info = ninfo + (int64_t)p * plane_nodes;
+#pragma unroll
+      for (int q = 0; q < kTileLoads; ++q)
+        if ((okm >> q) & 1) {
+          const int nd = rel[q] / 3, c = rel[q] - 3 * nd, ni = info[nd];
+          const bool free_dof = ((ni >> c) & 1) != 0;
+          cp_async_elem(dst + q * NT, free_dof ? u + (ni >> 3) + __popc(ni & ((1 << c) - 1)) : u, free_dof);
+        }
+    } else {
+      const T* src = COMPACT ? u + first : u + (int64_t)p * 3 * plane_nodes;
+#pragma unroll
+      for (int q = 0; q < kTileLoads; ++q)
+        if ((okm >> q) & 1) cp_async_elem(dst + q * NT, src + rel[q], true);
+    }
+  };
+  auto plane_first = [&](int p) { return COMPACT && p <= last ? pinfo[p] : 0; };
+  // epilogue operands of the thread's node in plane ie (first DOF off)
+  auto issue_operands = [&](int ie, int64_t off) {
+    if constexpr (NO > 0) {
+      if (own_node) {
+        T* dst = O + ((ie & 1) * NT + t) * NO;
+        const T* src[3] = {(const T*)ea.b + off, (const T*)ea.dinv + off, (const T*)ea.d + off};
+#pragma unroll
+        for (int k = 0; k < NO; ++k) cp_async_elem(dst + k, src[k / 3] + k % 3, true);
+      }
+    }
+  };
+
+  const int is = max(i0 - 1, 0);  // first element plane (the halo plane below i0, if there is one)
+  int64_t node = (int64_t)i0 * plane_nodes + je * NZ1 + ke;
+  issue_plane(is, plane_first(is));
+  issue_operands(i0, 3 * node);
+  cp_async_commit();
+#pragma unroll
+  for (int d = 1; d <= 2; ++d) {
+    if (is + d <= last) issue_plane(is + d, plane_first(is + d));
+    cp_async_commit();
+  }
+  int first_next = plane_first(is + 3);  // of the plane issued next
+  const int64_t eplane = (int64_t)g.ny * g.nz;
+  const T* Ep = E + (is * eplane + (int64_t)je * g.nz + ke);  // dereferenced only for columns of the mesh
+  T En = colv && is < g.nx ? *Ep : T(0);
+  // free bits of the thread's next node (COMPACT: pinfo of its plane)
+  auto node_bits = [&](int ie, int64_t nd) -> int { return COMPACT ? pinfo[ie] : (own_node ? (int)nmask[nd] : 0); };
+  int bits_next = node_bits(i0, node);
+  cp_async_wait_all_but_one();
+  __syncthreads();
+  const int at = tj * W + 3 * tk;
+  T p[3][4], carry[3][4], own[3];
+  {
+    const T* r = P + (is & (kPlaneBufs - 1)) * PV + at;
+    face_values<BF, FORM>(r, r + W, p, own);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) carry[q][s] = T(0);
+
+  for (int ie = is; ie < i1; ++ie) {
+    const bool sum = ie >= i0;
+    const bool epi = own_node && sum;
+    if (ie + 3 <= last) issue_plane(ie + 3, first_next);
+    if (COMPACT) first_next = plane_first(ie + 4);
+    if (sum && ie + 1 < i1) issue_operands(ie + 1, 3 * (node + plane_nodes));
+    cp_async_commit();
+    const int bits = bits_next;
+    if (sum && ie + 1 < i1) bits_next = node_bits(ie + 1, node + plane_nodes);
+    const T Ee = En;
+    Ep += eplane;
+    En = colv && ie + 1 < g.nx ? *Ep : T(0);
+    T tot[3][4], xv[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) xv[q] = own[q];
+    if (ie < g.nx) {
+      T c[3][4], lo[3][4], hi[3][4];
+      const T* r = P + ((ie + 1) & (kPlaneBufs - 1)) * PV + at;
+      face_values<BF, FORM>(r, r + W, c, own);
+      element_faces<DENSE, BF, FORM>(p, c, Ee, lo, hi);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          tot[q][s] = add_rn(carry[q][s], lo[q][s]);
+          carry[q][s] = hi[q][s];
+          p[q][s] = c[q][s];
+        }
     } else {
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+      for (int q = 0; q < 3; ++q)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) f[q][c] = T(0);
+        for (int s = 0; s < 4; ++s) tot[q][s] = carry[q][s];
     }
-    T* buf = F + (ie & 1) * 12 * NT;
-    if (ie >= i0) {
+    T* buf = F + ((ie & 1) * NT + t) * 9;
+    T f0[3];
+    if (sum) {
 #pragma unroll
-      for (int q2 = 0; q2 < 4; ++q2)
+      for (int q = 0; q < 3; ++q) {
+        T f[4];
+        face_corners<FORM>(tot[q], q, f);
+        f0[q] = f[0];  // corner (0, 0) is the thread's own node
 #pragma unroll
-        for (int c = 0; c < 3; ++c) buf[(q2 * 3 + c) * NT + t] = carry[q2][c] + f[q2][c];
+        for (int s = 1; s < 4; ++s) buf[3 * (s - 1) + q] = f[s];
+      }
     }
     cp_async_wait_all_but_one();
     __syncthreads();
-    if (do_epi) {
+    if (epi) {
+      const T* bz = buf - 9;
+      const T* by = buf - 9 * sh.bk;
+      T ku[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const T ku = ((buf[(0 * 3 + c) * NT + t] + buf[(2 * 3 + c) * NT + t - sh.bk]) +
-                      buf[(1 * 3 + c) * NT + t - 1]) +
-                     buf[(3 * 3 + c) * NT + t - sh.bk - 1];
-        eo.apply(ea, 3 * node + c, c, ku, xv[c]);
+      for (int q = 0; q < 3; ++q) ku[q] = add_rn(add_rn(add_rn(f0[q], by[3 + q]), bz[q]), by[6 + q - 9]);
+      if constexpr (COMPACT) {
+        if (bits >= 0) {
+          T* py = (T*)ea.y + bits + 3 * (je * NZ1 + ke);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) py[q] = ku[q];
+        } else {
+          const int ni = ninfo[node];
+          T* py = (T*)ea.y + (ni >> 3);
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            if ((ni >> q) & 1) py[__popc(ni & ((1 << q) - 1))] = ku[q];
+        }
+      } else {
+        T o[9];
+        const T* src = O + ((ie & 1) * NT + t) * NO;
+#pragma unroll
+        for (int k = 0; k < NO; ++k) o[k] = src[k];
+        node_epilogue<T, EPI>(ea, 3 * node, bits, o, ku, xv);
       }
     }
-#pragma unroll
-    for (int q2 = 0; q2 < 4; ++q2)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) carry[q2][c] = f[4 + q2][c];
+    if (sum) node += plane_nodes;
   }
 }
 
 template <typename T>
-static size_t sweep_smem(const SweepShape& sh) {
-  const size_t NT = (size_t)sh.bj * sh.bk;
-  const size_t PV = (size_t)(sh.bj + 1) * 3 * (sh.bk + 1);
-  return (24 * NT + kPlaneBufs * PV) * sizeof(T);
+static size_t sweep_smem(const SweepShape& sh, int operands) {
+  const size_t NT = (size_t)sh.bj * sh.bk, PV = (size_t)(sh.bj + 1) * 3 * (sh.bk + 1);
+  return sizeof(T) * ((18 + 6 * operands) * NT + kPlaneBufs * PV);
 }
 
-template <typename T, int EPI, int KMODE, int MAXT>
-static cudaError_t launch_sweep(const Grid& g, const SweepShape& sh, const T* E, const uint8_t* mask,
-                                const T* u, const EpiArgs& ea, cudaStream_t s) {
+bool fine_shape_ok(DType t, const Grid& g, const SweepShape& sh) {
   const int NT = sh.bj * sh.bk;
-  if (NT > MAXT || sh.bj < 2 || sh.bk < 2 || sh.cx < 1) return cudaErrorInvalidConfiguration;
-  if ((int64_t)(sh.bj + 1) * 3 * (sh.bk + 1) > (int64_t)kTileLoads * NT) return cudaErrorInvalidConfiguration;
-  const size_t smem = sweep_smem<T>(sh);
+  return sh.bk >= 2 && sh.bj >= 2 && sh.cx >= 1 && NT <= kSweepThreads &&
+         (sh.bj + 1) * 3 * (sh.bk + 1) <= kTileLoads * NT &&
+         4 * (int64_t)(g.ny + 1) * (g.nz + 1) < (int64_t(1) << 31) &&
+         (t == F64 ? sweep_smem<double>(sh, 3) : sweep_smem<float>(sh, 3)) <= 200 * 1024;
+}
+
+template <typename T, int EPI, bool DENSE, bool BF, bool COMPACT, int FORM>
+static cudaError_t launch_sweep_as(const Grid& g, const SweepShape& sh, const T* E, const uint8_t* nmask, const T* u,
+                                   const int32_t* ninfo, const int32_t* pinfo, const EpiArgs& ea, cudaStream_t s) {
+  if (!fine_shape_ok(sizeof(T) == 8 ? F64 : F32, g, sh)) return cudaErrorInvalidConfiguration;
+  auto kernel = sweep_kernel<T, EPI, DENSE, BF, COMPACT, FORM>;
   static std::atomic<uint64_t> attr_done;
-  const cudaError_t ea0 = once_per_device(attr_done, [] {
-    return cudaFuncSetAttribute(fine_sweep_kernel<T, EPI, KMODE, MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                200 * 1024);
+  const cudaError_t ea0 = once_per_device(attr_done, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   });
   if (ea0 != cudaSuccess) return ea0;
   const int nbj = (g.ny + sh.bj - 1) / (sh.bj - 1);
   const int nbk = (g.nz + sh.bk - 1) / (sh.bk - 1);
   dim3 grid(nbj * nbk, div_up(g.nx + 1, sh.cx));
-  fine_sweep_kernel<T, EPI, KMODE, MAXT><<<grid, NT, smem, s>>>(g, sh, E, mask, u, ea);
+  kernel<<<grid, sh.bj * sh.bk, sweep_smem<T>(sh, epi_operands<EPI>()), s>>>(g, sh, E, nmask, u, ninfo, pinfo, ea);
   return sf_launched(1);
 }
 
-// ----------------------------------------------------------------------------
-// FP32 sweep with two elements per thread.  Thread (tj, tp) evaluates the
-// k-adjacent element columns tk = 2tp and 2tp + 1 of the block's tile with the
-// packed FP32 pair instructions of sm_100 (lane x: element 2tp, lane y: element
-// 2tp + 1), which halves the arithmetic instruction count; it owns the nodes at
-// those two positions.  The node tile is stored component-major in shared
-// memory ([c][row][k], rows padded to an even length) so the dk = 0 corner pair
-// of both elements is one aligned 64-bit load.  Elements outside the mesh get
-// E = 0 (their corner values are zero-filled, so they contribute exactly 0)
-// instead of a branch.  Same staging, barrier and summation order as
-// fine_sweep_kernel; 32-bit indexing (the launcher checks ndof < 2^31).
-__device__ __forceinline__ float2 f2sub(float2 a, float2 b) {
-  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);  // a - b, one rounding
-}
-
-__device__ __forceinline__ void wht8x2(float2 (&a)[8]) {
-#pragma unroll
-  for (int m = 4; m >= 1; m >>= 1) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if ((q & m) == 0) {
-        const float2 p = a[q], r = a[q | m];
-        a[q] = __fadd2_rn(p, r);
-        a[q | m] = f2sub(p, r);
-      }
-    }
+template <typename T, int EPI, bool BF>
+static cudaError_t launch_sweep(const Grid& g, const SweepShape& sh, const void* E, const uint8_t* nmask,
+                                const void* u, const EpiArgs& ea, cudaStream_t s) {
+  if constexpr (sizeof(T) == 4 && !BF && EPI != EPI_APPLY) {
+    return g.ne() <= kFusedElements
+               ? launch_sweep_as<T, EPI, true, false, false, kElement>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
+                                                                       nullptr, ea, s)
+               : launch_sweep_as<T, EPI, true, false, false, kElementRn>(g, sh, (const T*)E, nmask, (const T*)u,
+                                                                         nullptr, nullptr, ea, s);
+  } else if constexpr (sizeof(T) == 4) {
+    return launch_sweep_as<T, EPI, true, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr, nullptr,
+                                                            ea, s);
+  } else {
+    return pattern_on_device()
+               ? launch_sweep_as<T, EPI, false, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
+                                                                   nullptr, ea, s)
+               : launch_sweep_as<T, EPI, true, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
+                                                                  nullptr, ea, s);
   }
 }
 
-__device__ __forceinline__ void elem_wht_x2(const float2 (&u)[8][3], float2 E, float2 (&f)[8][3]) {
-  float2 w[3][8];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) w[c][q] = u[q][c];
-    wht8x2(w[c]);
+template <typename T, bool BF>
+static cudaError_t launch_sweep_epi(Epi epi, const Grid& g, const SweepShape& sh, const void* E, const uint8_t* nmask,
+                                    const void* u, const EpiArgs& ea, cudaStream_t s) {
+  switch (epi) {
+    case EPI_APPLY: return launch_sweep<T, EPI_APPLY, BF>(g, sh, E, nmask, u, ea, s);
+    case EPI_RESID: return launch_sweep<T, EPI_RESID, BF>(g, sh, E, nmask, u, ea, s);
+    case EPI_CHEB1: return launch_sweep<T, EPI_CHEB1, BF>(g, sh, E, nmask, u, ea, s);
+    case EPI_CHEB: return launch_sweep<T, EPI_CHEB, BF>(g, sh, E, nmask, u, ea, s);
+    case EPI_JAC: return launch_sweep<T, EPI_JAC, BF>(g, sh, E, nmask, u, ea, s);
   }
-  float2 v[3][8];
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const float2 in0 = w[0][b ^ 4], in1 = w[1][b ^ 2], in2 = w[2][b ^ 1];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      float2 s = __fmul2_rn(c_wht32x2[b][3 * r], in0);
-      s = __ffma2_rn(c_wht32x2[b][3 * r + 1], in1, s);
-      s = __ffma2_rn(c_wht32x2[b][3 * r + 2], in2, s);
-      v[r][b ^ (4 >> r)] = __fmul2_rn(E, s);
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    wht8x2(v[c]);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) f[q][c] = v[c][q];
-  }
+  return cudaErrorInvalidValue;
 }
-
-constexpr int kX2Threads = 256;
-constexpr int kX2NodeLoads = 3;  // tile nodes per thread; launch checks
-
-template <int EPI, int MINB>
-__global__ void __launch_bounds__(kX2Threads, MINB) fine_sweep_x2_kernel(Grid g, SweepShape sh,
-                                                                   const float* __restrict__ E,
-                                                                   const uint8_t* __restrict__ mask,
-                                                                   const float* __restrict__ u, EpiArgs ea) {
-  if (guard_off(ea.guard)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int HK = sh.bk >> 1, NT = sh.bj * HK, NE = sh.bj * sh.bk;
-  const int NK1 = sh.bk + 1, NKP = sh.bk + 2;
-  const int RP = (sh.bj + 1) * NKP;  // one component of one plane tile
-  const int PV = 3 * RP;
-  const int NN = (sh.bj + 1) * NK1;  // tile nodes
-  float* F = reinterpret_cast<float*>(smem_raw);  // face sums [3][12][NE], plane q in q mod 3
-  float* P = F + 36 * NE;                         // plane tiles [3][3][bj+1][NKP]
-  const int t = threadIdx.x;
-  const int tj = t / HK, tp = t - tj * HK, tk0 = 2 * tp;
-  const int nbk = (g.nz + sh.bk - 1) / (sh.bk - 1);
-  const int bjI = blockIdx.x / nbk, bkI = blockIdx.x - bjI * nbk;
-  const int jb = bjI * (sh.bj - 1) - 1, kb = bkI * (sh.bk - 1) - 1;
-  const int je = jb + tj, ke0 = kb + tk0, ke1 = ke0 + 1;
-  const int i0 = blockIdx.y * sh.cx;
-  const int i1 = min(i0 + sh.cx, g.nx + 1);
-  const bool rowv = je >= 0 && je < g.ny;
-  const bool colv0 = rowv && ke0 >= 0 && ke0 < g.nz, colv1 = rowv && ke1 >= 0 && ke1 < g.nz;
-  const bool ownr = tj >= 1 && je <= g.ny;
-  const bool own0 = ownr && tk0 >= 1 && ke0 <= g.nz, own1 = ownr && ke1 <= g.nz;
-  const int NZ1 = g.nz + 1;
-  const int64_t plane_vals = 3 * (int64_t)(g.ny + 1) * NZ1;
-
-  int rel[kX2NodeLoads], sidx[kX2NodeLoads];
-  bool okn[kX2NodeLoads];
-#pragma unroll
-  for (int s = 0; s < kX2NodeLoads; ++s) {
-    const int n = t + s * NT;
-    const int row = n / NK1, kk = n - row * NK1;
-    const int j = jb + row, k = kb + kk;
-    okn[s] = n < NN && j >= 0 && j <= g.ny && k >= 0 && k <= g.nz;
-    rel[s] = okn[s] ? 3 * (j * NZ1 + k) : 0;
-    sidx[s] = n < NN ? row * NKP + kk : -1;
-  }
-  // (the packed sweep stages its planes through registers: with cp.async it
-  // needed 214 registers for the Jacobi epilogue and ran slower)
-  auto load_plane = [&](int p, float (&r)[3 * kX2NodeLoads]) {
-    const bool pv = p >= 0 && p <= g.nx;
-    const float* base = u + (pv ? (int64_t)p * plane_vals : 0);
-#pragma unroll
-    for (int s = 0; s < kX2NodeLoads; ++s)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) r[3 * s + c] = (pv && okn[s]) ? base[rel[s] + c] : 0.f;
-  };
-  auto store_plane = [&](int buf, const float (&r)[3 * kX2NodeLoads]) {
-    float* dst = P + buf * PV;
-#pragma unroll
-    for (int s = 0; s < kX2NodeLoads; ++s)
-      if (sidx[s] >= 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) dst[c * RP + sidx[s]] = r[3 * s + c];
-      }
-  };
-  auto read_face2 = [&](int buf, float2 (&uu)[8][3], int q0) {
-    const float* src = P + buf * PV;
-#pragma unroll
-    for (int q2 = 0; q2 < 4; ++q2) {
-      const int base = (tj + (q2 >> 1)) * NKP + tk0 + (q2 & 1);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float* a = src + c * RP + base;
-        uu[q0 + q2][c] = (q2 & 1) ? make_float2(a[0], a[1]) : *reinterpret_cast<const float2*>(a);
-      }
-    }
-  };
-  auto e_pair = [&](int ie) {
-    const bool pv = ie >= 0 && ie < g.nx;
-    const int idx = (ie * g.ny + je) * g.nz + ke0;
-    return make_float2((pv && colv0) ? E[idx] : 0.f, (pv && colv1) ? E[idx + 1] : 0.f);
-  };
-
-  float pre[3 * kX2NodeLoads];
-  load_plane(i0 - 1, pre);
-  store_plane((i0 + 2) % 3, pre);
-  load_plane(i0, pre);
-  store_plane(i0 % 3, pre);
-  if (i0 + 1 <= i1) load_plane(i0 + 1, pre);
-  float2 En = e_pair(i0 - 1);
-  __syncthreads();
-
-  const int e0 = tj * sh.bk + tk0;
-  const int em1 = tp == 0 ? e0 : e0 - 1;  // node 2tp is a halo when tp == 0
-  for (int ie = i0 - 1; ie < i1; ++ie) {
-    if (ie + 2 <= i1) store_plane((ie + 2) % 3, pre);
-    if (ie + 3 <= i1) load_plane(ie + 3, pre);
-    const float2 Ee = En;
-    En = e_pair(ie + 1);
-    const bool epi0 = own0 && ie >= i0, epi1 = own1 && ie >= i0;
-    const int node0 = (ie * (g.ny + 1) + je) * NZ1 + ke0;
-    const int blo = (ie + 3) % 3, bhi = (ie + 1) % 3;
-    float2 f[8][3];
-    {
-      float2 ue[8][3];
-      read_face2(blo, ue, 0);
-      read_face2(bhi, ue, 4);
-      elem_wht_x2(ue, Ee, f);
-    }
-    // epilogue operands after the element arithmetic (not live across its
-    // register peak); the face-sum stores and the barrier cover their latency
-    EpiOperands<float, EPI> eo0, eo1;
-    if (epi0) eo0.load(ea, 3 * (int64_t)node0, mask);
-    if (epi1) eo1.load(ea, 3 * (int64_t)node0 + 3, mask);
-    float2 xv[3];
-    if (epi0 || epi1) {
-      const float* xs = P + blo * PV + tj * NKP + tk0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) xv[c] = *reinterpret_cast<const float2*>(xs + c * RP);
-    }
-    // face sums of node plane ie: this element plane's -x face added to the
-    // +x face of element plane ie - 1, which this thread parked in the same
-    // slots one iteration earlier; the +x face goes to plane ie + 1's buffer
-    // (last read before the previous barrier)
-    float* Fb = F + ((ie + 3) % 3) * 12 * NE;
-    float* Fn = F + ((ie + 1) % 3) * 12 * NE;
-#pragma unroll
-    for (int q2 = 0; q2 < 4; ++q2)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        float2* slot = reinterpret_cast<float2*>(Fb + (q2 * 3 + c) * NE + e0);
-        if (ie >= i0) *slot = __fadd2_rn(*slot, f[q2][c]);
-        *reinterpret_cast<float2*>(Fn + (q2 * 3 + c) * NE + e0) = f[4 + q2][c];
-      }
-    __syncthreads();
-    if (epi0 || epi1) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float2 a = *reinterpret_cast<const float2*>(Fb + (0 * 3 + c) * NE + e0);
-        const float2 b = *reinterpret_cast<const float2*>(Fb + (2 * 3 + c) * NE + e0 - sh.bk);
-        const float* p1 = Fb + (1 * 3 + c) * NE;
-        const float* p3 = Fb + (3 * 3 + c) * NE - sh.bk;
-        const float2 x1 = make_float2(p1[em1], p1[e0]);
-        const float2 x3 = make_float2(p3[em1], p3[e0]);
-        const float2 ku = __fadd2_rn(__fadd2_rn(__fadd2_rn(a, b), x1), x3);
-        if (epi0) eo0.apply(ea, 3 * (int64_t)node0 + c, c, ku.x, xv[c].x);
-        if (epi1) eo1.apply(ea, 3 * (int64_t)node0 + 3 + c, c, ku.y, xv[c].y);
-      }
-    }
-  }
-}
-
-static bool x2_shape_ok(const Grid& g, const SweepShape& sh) {
-  const int NT = sh.bj * sh.bk / 2;
-  return sh.bk % 2 == 0 && sh.bk >= 4 && sh.bj >= 3 && sh.cx >= 1 && NT <= kX2Threads &&
-         (sh.bj + 1) * (sh.bk + 1) <= kX2NodeLoads * NT && g.ndof < (int64_t(1) << 31);
-}
-
-template <int EPI>
-static cudaError_t launch_sweep_f32(const Grid& g, const SweepShape& sh, const float* E, const uint8_t* mask,
-                                    const float* u, const EpiArgs& ea, cudaStream_t s) {
-  if (sh.variant == 1 || !x2_shape_ok(g, sh)) return launch_sweep<float, EPI, 0, 512>(g, sh, E, mask, u, ea, s);
-  const int NT = sh.bj * sh.bk / 2, NE = sh.bj * sh.bk;
-  const size_t smem = sizeof(float) * (36 * (size_t)NE + 9 * (size_t)(sh.bj + 1) * (sh.bk + 2));
-  static std::atomic<uint64_t> attr_done[2];
-  const int capped = sh.variant == 2 ? 1 : 0;
-  const cudaError_t ea0 = once_per_device(attr_done[capped], [&] {
-    return capped ? cudaFuncSetAttribute(fine_sweep_x2_kernel<EPI, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024)
-                  : cudaFuncSetAttribute(fine_sweep_x2_kernel<EPI, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024);
-  });
-  if (ea0 != cudaSuccess) return ea0;
-  const int nbj = (g.ny + sh.bj - 1) / (sh.bj - 1);
-  const int nbk = (g.nz + sh.bk - 1) / (sh.bk - 1);
-  dim3 grid(nbj * nbk, div_up(g.nx + 1, sh.cx));
-  if (capped)
-    fine_sweep_x2_kernel<EPI, 2><<<grid, NT, smem, s>>>(g, sh, E, mask, u, ea);
-  else
-    fine_sweep_x2_kernel<EPI, 1><<<grid, NT, smem, s>>>(g, sh, E, mask, u, ea);
-  return sf_launched(1);
-}
-
-constexpr int kMaxThreadsF64 = 256;
-constexpr int kMaxThreadsF32 = 512;
 
 cudaError_t launch_fine(DType t, Epi epi, const Grid& g, const SweepShape& sh, const void* E,
-                        const uint8_t* mask, const void* u, const EpiArgs& ea, cudaStream_t s) {
-#define SF_FINE_CASE(T, MAXT, E_)                                                              \
-  case E_:                                                                                     \
-    return launch_sweep<T, E_, 0, MAXT>(g, sh, (const T*)E, mask, (const T*)u, ea, s);
-  if (t == F64) {
-    switch (epi) {
-      SF_FINE_CASE(double, kMaxThreadsF64, EPI_APPLY)
-      SF_FINE_CASE(double, kMaxThreadsF64, EPI_RESID)
-      SF_FINE_CASE(double, kMaxThreadsF64, EPI_CHEB1)
-      SF_FINE_CASE(double, kMaxThreadsF64, EPI_CHEB)
-      SF_FINE_CASE(double, kMaxThreadsF64, EPI_JAC)
-    }
-  } else if (t == F32) {
-    switch (epi) {
-      case EPI_APPLY:
-        return launch_sweep_f32<EPI_APPLY>(g, sh, (const float*)E, mask, (const float*)u, ea, s);
-      case EPI_RESID:
-        return launch_sweep_f32<EPI_RESID>(g, sh, (const float*)E, mask, (const float*)u, ea, s);
-      case EPI_CHEB1:
-        return launch_sweep_f32<EPI_CHEB1>(g, sh, (const float*)E, mask, (const float*)u, ea, s);
-      case EPI_CHEB:
-        return launch_sweep_f32<EPI_CHEB>(g, sh, (const float*)E, mask, (const float*)u, ea, s);
-      case EPI_JAC:
-        return launch_sweep_f32<EPI_JAC>(g, sh, (const float*)E, mask, (const float*)u, ea, s);
-    }
-  } else if (t == BF16) {
-    // BF16 operands (u and KE rounded to bf16), FP32 accumulation and FP32 vectors.
-    switch (epi) {
-      case EPI_APPLY:
-        return launch_sweep<float, EPI_APPLY, 1, kMaxThreadsF32>(g, sh, (const float*)E, mask,
-                                                                 (const float*)u, ea, s);
-      case EPI_RESID:
-        return launch_sweep<float, EPI_RESID, 1, kMaxThreadsF32>(g, sh, (const float*)E, mask,
-                                                                 (const float*)u, ea, s);
-      case EPI_CHEB1:
-        return launch_sweep<float, EPI_CHEB1, 1, kMaxThreadsF32>(g, sh, (const float*)E, mask,
-                                                                 (const float*)u, ea, s);
-      case EPI_CHEB:
-        return launch_sweep<float, EPI_CHEB, 1, kMaxThreadsF32>(g, sh, (const float*)E, mask,
-                                                                (const float*)u, ea, s);
-      case EPI_JAC:
-        return launch_sweep<float, EPI_JAC, 1, kMaxThreadsF32>(g, sh, (const float*)E, mask,
-                                                               (const float*)u, ea, s);
-    }
-  }
-#undef SF_FINE_CASE
+                        const uint8_t* nmask, const void* u, const EpiArgs& ea, cudaStream_t s) {
+  if (t == F64) return launch_sweep_epi<double, false>(epi, g, sh, E, nmask, u, ea, s);
+  if (t == F32) return launch_sweep_epi<float, false>(epi, g, sh, E, nmask, u, ea, s);
+  // BF16 operands (u and KE rounded to bf16), FP32 accumulation and FP32 vectors
+  if (t == BF16) return launch_sweep_epi<float, true>(epi, g, sh, E, nmask, u, ea, s);
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_fine_compact(const Grid& g, const SweepShape& sh, const double* E, const int32_t* ninfo,
+                                const int32_t* pinfo, const double* u_free, double* y_free, cudaStream_t s) {
+  EpiArgs ea;
+  ea.y = y_free;
+  return pattern_on_device()
+             ? launch_sweep_as<double, EPI_APPLY, false, false, true, kFaces>(g, sh, E, nullptr, u_free, ninfo, pinfo, ea, s)
+             : launch_sweep_as<double, EPI_APPLY, true, false, true, kFaces>(g, sh, E, nullptr, u_free, ninfo, pinfo, ea, s);
 }
 
 // ----------------------------------------------------------------------------
@@ -743,7 +870,7 @@ __global__ void element_energy_kernel(Grid g, const double* __restrict__ u, doub
     for (int c = 0; c < 3; ++c) ue[q][c] = u[3 * node + c];
   }
   double f[8][3];
-  elem_wht<double>(ue, 1.0, f);
+  elem_wht(ue, f);
   double acc = 0.0;
 #pragma unroll
   for (int q = 0; q < 8; ++q)

@@ -195,23 +195,81 @@ static std::vector<double> make_w1(int nf, int nc) {
 
 // ----------------------------------------------------------------------------
 
-SweepShape default_shape(const Grid& g, int maxt) {
-  SweepShape s;
-  const int full_k = g.nz + 2;
-  if (full_k <= 64 && full_k * 2 <= maxt) {
-    s.bk = full_k;
-  } else {
-    s.bk = 32;
+static int64_t div_up64(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Time model of a tile (microseconds): the blocks of an SM run in rounds of as many
+// as registers and shared memory hold; a round walks cx node planes after about two
+// of start-up, and a plane takes the larger of one warp's latency and the issue of
+// all resident warps.  Coefficients fitted to the times of 500 candidate tiles on six
+// grids between 24 x 12 x 6 and 252 x 126 x 63 (7 % root mean square in FP32, 8 % in
+// FP64; its first choice was up to 17 % slower than the best tile, the best of its
+// first 32 never: hence the tuner's shortlist).
+static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
+  const double latency = t == F64 ? 0.638 : 0.740, issue = t == F64 ? 0.0968 : 0.0877;
+  const double startup = t == F64 ? 2.03 : 1.85, launch = 4.5;
+  const int64_t es = t == F64 ? 8 : 4, regs = t == F64 ? 168 : 120;
+  const int64_t nt = (int64_t)sh.bj * sh.bk, warps = div_up64(nt, 32);
+  const int64_t smem = es * (18 * nt + 4 * 3 * (sh.bj + 1) * (sh.bk + 1)) + 1024;
+  const int64_t resident =
+      std::max<int64_t>(1, std::min({65536 / (regs * 32 * warps), 233472 / smem, int64_t(32), 64 / warps}));
+  const int64_t blocks =
+      div_up64(g.ny + 1, sh.bj - 1) * div_up64(g.nz + 1, sh.bk - 1) * div_up64(g.nx + 1, sh.cx);
+  const int64_t per_sm = div_up64(blocks, grid_sm_count()), full = per_sm / resident, rest = per_sm % resident;
+  const double planes = sh.cx + startup;
+  double us = launch + full * planes * std::max(latency, issue * resident * warps);
+  if (rest) us += planes * std::max(latency, issue * rest * warps);
+  return us;
+}
+
+// Candidate tiles of a grid: the z extent in one to four equal parts, blocks of up to
+// 256, 128 or 64 threads filled with equal parts of the y extent, cx node planes a
+// block (the halo column and the halo plane make each part one element larger).
+static std::vector<SweepShape> sweep_candidates(DType t, const Grid& g) {
+  std::vector<SweepShape> out;
+  for (int parts = 1; parts <= 4; ++parts) {
+    SweepShape sh;
+    sh.bk = (int)div_up64(g.nz + 1, parts) + 1;
+    sh.bk = std::max(2, sh.bk);
+    if (sh.bk > 130) continue;
+    for (int nt : {128, 96, 64}) {
+      const int most = nt / sh.bk;
+      if (most < 2) continue;
+      const int nb = (int)div_up64(g.ny + 1, most - 1);
+      sh.bj = (int)div_up64(g.ny + 1, nb) + 1;
+      for (int cx : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {
+        sh.cx = cx;
+        if (cx > 1 && cx >= 2 * (g.nx + 1)) continue;
+        if (!fine_shape_ok(t, g, sh)) continue;
+        bool seen = false;
+        for (const SweepShape& o : out) seen = seen || (o.bj == sh.bj && o.bk == sh.bk && o.cx == sh.cx);
+        if (!seen) out.push_back(sh);
+      }
+    }
   }
-  s.bj = std::max(2, std::min(maxt / s.bk, g.ny + 2));
-  s.cx = 8;
-  return s;
+  return out;
+}
+
+// The tile of a mesh that was not tuned.
+SweepShape default_shape(DType t, const Grid& g) {
+  SweepShape best;
+  best.bj = 2;
+  best.bk = 4;
+  best.cx = 1;
+  double best_cost = 1e300;
+  for (const SweepShape& sh : sweep_candidates(t, g)) {
+    const double cost = sweep_cost(t, g, sh);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = sh;
+    }
+  }
+  return best;
 }
 
 void fine_apply(Mesh& m, DType t, Epi epi, const void* E, const void* u, const EpiArgs& ea,
                        cudaStream_t s) {
   const SweepShape& sh = m.sh[t == F64 ? 0 : 1];
-  SF_CUDA(launch_fine(t, epi, m.g, sh, E, m.mask.as<uint8_t>(), u, ea, s));
+  SF_CUDA(launch_fine(t, epi, m.g, sh, E, m.nmask.as<uint8_t>(), u, ea, s));
 }
 
 // Tuner: time candidate sweep shapes on this mesh and keep the fastest.  The
@@ -232,7 +290,6 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
     m.tuned[idx] = true;
     return;
   }
-  const int maxt = t == F64 ? 256 : 512;
   const size_t es = dsize(t == BF16 ? F32 : t);
   DevBuf E, u, y;
   E.alloc(es * std::max<int64_t>(1, m.g.ne()));
@@ -240,59 +297,42 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
   y.alloc(es * m.g.ndof);
   SF_CUDA(launch_fill_hash(t == F64 ? F64 : F32, m.g.ndof, 7u, u.p, s));
   SF_CUDA(launch_fill(t == F64 ? F64 : F32, m.g.ne(), 1.0, E.p, nullptr, s));
-  std::vector<SweepShape> cands;
-  std::vector<int> bks;
-  if (m.g.nz + 2 <= 64) bks.push_back(m.g.nz + 2);
-  for (int bk : {16, 32, 64})
-    if (bk < m.g.nz + 2) bks.push_back(bk);
-  for (int bk : bks)
-    for (int nt : {128, 256, maxt}) {
-      const int bj = nt / bk;
-      if (bj < 2 || bj * bk > maxt) continue;
-      for (int cx : {4, 6, 8, 10, 12, 14, 16, 20}) {  // fine steps: the wave count depends on it
-        SweepShape sh;
-        sh.bj = bj;
-        sh.bk = bk;
-        sh.cx = cx;
-        cands.push_back(sh);
-        // FP32: also the one-element-per-thread sweep (twice the threads of the packed
-        // sweep for the same tile) and the packed sweep with a register cap (more
-        // resident blocks); on grids too small to fill the GPU either can hide more
-        // latency than the packed sweep
-        if (t == F32) {
-          for (int v : {1, 2}) {
-            sh.variant = v;
-            cands.push_back(sh);
-          }
-        }
-      }
-    }
+  // the candidates of the lowest modelled time
+  std::vector<SweepShape> cands = sweep_candidates(t, m.g);
+  std::stable_sort(cands.begin(), cands.end(), [&](const SweepShape& a, const SweepShape& b) {
+    return sweep_cost(t, m.g, a) < sweep_cost(t, m.g, b);
+  });
+  if (cands.size() > 32) cands.resize(32);
+  constexpr int kTuneReps = 8;
   cudaEvent_t e0, e1;
   SF_CUDA(cudaEventCreate(&e0));
   SF_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
-  SweepShape best_sh = default_shape(m.g, maxt);
+  SweepShape best_sh = default_shape(t, m.g);
   // SIMPFEM_TUNE_VERBOSE=1 prints every candidate's time (stderr)
   const char* vb = getenv("SIMPFEM_TUNE_VERBOSE");
   const bool verbose = vb != nullptr && vb[0] != '\0' && vb[0] != '0';
+  // timed as the residual: in FP32 the form the cycle's smoothing steps run
   EpiArgs ea;
   ea.y = y.p;
+  ea.b = u.p;
   for (const SweepShape& sh : cands) {
-    cudaError_t err = launch_fine(t, EPI_APPLY, m.g, sh, E.p, m.mask.as<uint8_t>(), u.p, ea, s);
+    cudaError_t err = launch_fine(t, EPI_RESID, m.g, sh, E.p, m.nmask.as<uint8_t>(), u.p, ea, s);
     if (err != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
     SF_CUDA(cudaEventRecord(e0, s));
-    for (int r = 0; r < 3; ++r)
-      SF_CUDA(launch_fine(t, EPI_APPLY, m.g, sh, E.p, m.mask.as<uint8_t>(), u.p, ea, s));
+    for (int r = 0; r < kTuneReps; ++r)
+      SF_CUDA(launch_fine(t, EPI_RESID, m.g, sh, E.p, m.nmask.as<uint8_t>(), u.p, ea, s));
     SF_CUDA(cudaEventRecord(e1, s));
     SF_CUDA(cudaEventSynchronize(e1));
     float ms = 0.f;
     SF_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     if (verbose)
-      fprintf(stderr, "[simpfem tune] %s %dx%dx%d bj=%d bk=%d cx=%d variant=%d: %.1f us\n",
-              t == F64 ? "f64" : "f32", m.g.nx, m.g.ny, m.g.nz, sh.bj, sh.bk, sh.cx, sh.variant, ms * 1000.f / 3.f);
+      fprintf(stderr, "[simpfem tune] %s %dx%dx%d bj=%d bk=%d cx=%d: %.1f us (model %.1f)\n",
+              t == F64 ? "f64" : "f32", m.g.nx, m.g.ny, m.g.nz, sh.bj, sh.bk, sh.cx, ms * 1000.f / kTuneReps,
+              sweep_cost(t, m.g, sh));
     if (ms < best) {
       best = ms;
       best_sh = sh;

@@ -78,6 +78,9 @@ struct Mesh {
   std::vector<int32_t> free_h;
   std::vector<uint8_t> mask_h;
   DevBuf free_idx, mask;
+  DevBuf nmask;  // the three free bits of every node
+  // tables of the compact operator (launch_fine_compact), empty beyond 2^28 free DOFs
+  DevBuf ninfo, pinfo;
   double ke[576];
   WhtBlocks wb;
   std::vector<double> Q;
@@ -249,7 +252,7 @@ using PrecFn = std::function<void(const double* in, double* out, const int* guar
 
 WhtBlocks make_wht_blocks(const double* ke, double* max_off);
 std::vector<double> make_level1_Q(const double* ke);
-SweepShape default_shape(const Grid& g, int maxt);
+SweepShape default_shape(DType t, const Grid& g);
 void fine_apply(Mesh& m, DType t, Epi epi, const void* E, const void* u, const EpiArgs& ea, cudaStream_t s);
 void tune_mesh(Mesh& m, DType t, cudaStream_t s);
 Gmg* gmg_create(Mesh* m, const simpfem_gmg_opts& o);

@@ -59,11 +59,8 @@ struct Grid {
 // Tile shape of the fine-operator sweep kernel (chosen by the tuner).
 struct SweepShape {
   int bj = 8;   // element columns along y per block (one of them is a halo column)
-  int bk = 32;  // element columns along z per block (one halo column)
+  int bk = 16;  // element columns along z per block (one halo column)
   int cx = 8;   // node planes along x per block
-  int variant = 0;  // FP32 kernel, picked by the tuner like the tile: 0 = two elements per
-                    // thread (packed FP32 pairs), 1 = one element per thread, 2 = two per
-                    // thread compiled for two resident 256-thread blocks (a 128-register cap)
 };
 
 struct WhtBlocks {
@@ -116,8 +113,15 @@ enum ScalarOp { OP_LS1 = 0, OP_LS2 = 1, OP_RLF = 2, OP_RLL = 3 };
 
 // ---------------------------------------------------------------- fine.cu
 void set_fine_constants(const double* ke576, const WhtBlocks& wb);
+// nmask: the three free bits of every node, one byte a node
 cudaError_t launch_fine(DType t, Epi epi, const Grid& g, const SweepShape& sh, const void* E,
-                        const uint8_t* mask, const void* u, const EpiArgs& ea, cudaStream_t s);
+                        const uint8_t* nmask, const void* u, const EpiArgs& ea, cudaStream_t s);
+bool fine_shape_ok(DType t, const Grid& g, const SweepShape& sh);
+// y_free = K_ff u_free on compact free-DOF vectors (FP64); ninfo[node] = 8 * (free
+// index of the node's first free DOF) + its three free bits, pinfo[x plane] = the
+// free index of its first DOF when all its DOFs are free, else -1
+cudaError_t launch_fine_compact(const Grid& g, const SweepShape& sh, const double* E, const int32_t* ninfo,
+                                const int32_t* pinfo, const double* u_free, double* y_free, cudaStream_t s);
 cudaError_t launch_fine_diag(const Grid& g, const double* E, const uint8_t* mask, double kd,
                              double* diag, cudaStream_t s);
 cudaError_t launch_node_blocks(const Grid& g, const double* E, const uint8_t* mask,

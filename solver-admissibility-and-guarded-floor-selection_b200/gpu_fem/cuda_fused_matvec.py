@@ -32,7 +32,7 @@ class FusedMatvec:
     BLOCK_X = BLOCK_X_FP32
 
     def __init__(self, edof_gpu, KE_unit_gpu, ndof: int):
-        torch = _lib.require_cuda()
+        _lib.require_cuda()
         shape = tuple(edof_gpu.shape)
         if len(shape) != 2 or shape[1] != self.KE_SIZE:
             raise ValueError(f"FusedMatvec currently supports ke_size=24 only, got {shape[-1]}")
@@ -45,7 +45,6 @@ class FusedMatvec:
         if self._mesh.ndof != self._ndof:
             raise ValueError("ndof does not match the mesh of the edof table")
         self._bf16_available = True
-        self._y_full = torch.zeros(self._ndof, dtype=torch.float32, device="cuda")
 
     def _launch(self, dtype: str, u_full, y_full, E_f32) -> None:
         if dtype == "fp32":
@@ -64,7 +63,7 @@ class FusedMatvec:
         u_full = torch.zeros(self._ndof, dtype=torch.float32, device="cuda")
         u_full[free] = _lib.as_cuda(u_free, torch.float32)
         E = _lib.as_cuda(E_e, torch.float32)
-        y_full = self._y_full
+        y_full = torch.empty_like(u_full)
         self._launch(dtype, u_full, y_full, E)
         return y_full[free]
 
@@ -75,6 +74,6 @@ class FusedMatvec:
         if u_full.numel() != self._ndof:
             raise ValueError("u_full must have ndof entries")
         E = _lib.as_cuda(E_e, torch.float32)
-        y_full = self._y_full
+        y_full = torch.empty(self._ndof, dtype=torch.float32, device="cuda")
         self._launch(dtype, u_full, y_full, E)
-        return y_full.clone()
+        return y_full
