@@ -218,6 +218,68 @@ __device__ __forceinline__ void element_product2(const float2 (&ulo)[3][2], cons
   }
 }
 
+// The same in FP64; faces are node values [component][2 dy + dz].  All entries are
+// taken: those outside the pattern can hold roundings of the transform.  They come
+// from shared memory (cw: ten values a block): constants are hoisted out of the
+// plane loop into registers, 144 of them (512k elements: 47 us at two blocks per SM,
+// 37 so at three).
+constexpr int kBlockCoefs = 10;
+__device__ __forceinline__ void element_product(const double (&ulo)[3][4], const double (&uhi)[3][4], double E,
+                                                const double* cw, double (&flo)[3][4], double (&fhi)[3][4]) {
+  double w[3][8], v[3][8];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      w[q][s] = ulo[q][s];
+      w[q][4 + s] = uhi[q][s];
+    }
+    wht8(w[q]);
+  }
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const double in[3] = {w[0][b ^ 4], w[1][b ^ 2], w[2][b ^ 1]};
+    double co[kBlockCoefs];
+#pragma unroll
+    for (int k = 0; k < kBlockCoefs; k += 2) {
+      const double2 c = *reinterpret_cast<const double2*>(cw + b * kBlockCoefs + k);
+      co[k] = c.x;
+      co[k + 1] = c.y;
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      double acc = mul_rn(co[3 * r + 1], in[1]);
+      acc = fma(co[3 * r], in[0], acc);
+      acc = fma(co[3 * r + 2], in[2], acc);
+      v[r][b ^ (4 >> r)] = acc;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    double f[8];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const double r = mul_rn(E, v[q][4 + s]);
+      f[s] = fma(E, v[q][s], r);
+      f[4 + s] = fma(E, v[q][s], -r);
+    }
+#pragma unroll
+    for (int m = 2; m >= 1; m >>= 1)
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if ((s & m) == 0) {
+          const double a = f[s], b = f[s | m];
+          f[s] = a + b;
+          f[s | m] = a - b;
+        }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      flo[q][s] = f[s];
+      fhi[q][s] = f[4 + s];
+    }
+  }
+}
+
 // One value copied global -> shared asynchronously (cp.async; zero-filled when ok
 // is false, reading nothing from src, which is then any valid address).
 template <typename T>
@@ -242,6 +304,13 @@ __device__ __forceinline__ void face_values(const double* r0, const double* r1, 
   for (int q = 0; q < 3; ++q) {
     own[q] = r0[q];
     const double n00 = own[q], n01 = r0[3 + q], n10 = r1[q], n11 = r1[3 + q];
+    if (FORM != kFaces) {
+      v[q][0] = n00;
+      v[q][1] = n01;
+      v[q][2] = n10;
+      v[q][3] = n11;
+      continue;
+    }
     const double s0 = n00 + n01, d0 = n00 - n01, s1 = n10 + n11, d1 = n10 - n11;
     v[q][0] = s0 + s1;
     v[q][1] = d0 + d1;
@@ -280,43 +349,47 @@ __device__ __forceinline__ void face_values(const float* r0, const float* r1, fl
 // them, in the faces' representation, scaled by the modulus E.
 template <bool DENSE, bool BF, int FORM>
 __device__ __forceinline__ void element_faces(const double (&p)[3][4], const double (&c)[3][4], double E,
-                                              double (&lo)[3][4], double (&hi)[3][4]) {
-  double w[3][8], v[3][8];
+                                              const double* cw, double (&lo)[3][4], double (&hi)[3][4]) {
+  if constexpr (FORM != kFaces) {
+    element_product(p, c, E, cw, lo, hi);
+  } else {
+    double w[3][8], v[3][8];
 #pragma unroll
-  for (int q = 0; q < 3; ++q)
+    for (int q = 0; q < 3; ++q)
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      w[q][s] = p[q][s] + c[q][s];
-      w[q][4 + s] = p[q][s] - c[q][s];
-    }
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const double in[3] = {w[0][b ^ 4], w[1][b ^ 2], w[2][b ^ 1]};
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      double acc = 0.0;
-      bool first = true;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        if (!DENSE && !block_entry(b, r, k)) continue;
-        const double co = c_wht64[b][3 * r + k];
-        acc = first ? co * in[k] : fma(co, in[k], acc);
-        first = false;
+      for (int s = 0; s < 4; ++s) {
+        w[q][s] = p[q][s] + c[q][s];
+        w[q][4 + s] = p[q][s] - c[q][s];
       }
-      v[r][b ^ (4 >> r)] = E * acc;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const double in[3] = {w[0][b ^ 4], w[1][b ^ 2], w[2][b ^ 1]};
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        double acc = 0.0;
+        bool first = true;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (!DENSE && !block_entry(b, r, k)) continue;
+          const double co = c_wht64[b][3 * r + k];
+          acc = first ? co * in[k] : fma(co, in[k], acc);
+          first = false;
+        }
+        v[r][b ^ (4 >> r)] = E * acc;
+      }
     }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        lo[q][s] = v[q][s] + v[q][4 + s];
+        hi[q][s] = v[q][s] - v[q][4 + s];
+      }
   }
-#pragma unroll
-  for (int q = 0; q < 3; ++q)
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      lo[q][s] = v[q][s] + v[q][4 + s];
-      hi[q][s] = v[q][s] - v[q][4 + s];
-    }
 }
 template <bool DENSE, bool BF, int FORM>
 __device__ __forceinline__ void element_faces(const float (&p)[3][4], const float (&c)[3][4], float E,
-                                              float (&lo)[3][4], float (&hi)[3][4]) {
+                                              const double*, float (&lo)[3][4], float (&hi)[3][4]) {
   float2 a[3][2], b[3][2], l[3][2], h[3][2];
 #pragma unroll
   for (int q = 0; q < 3; ++q)
@@ -361,6 +434,11 @@ __device__ __forceinline__ void element_faces(const float (&p)[3][4], const floa
 // A face's sum t (one component) as its four corners f[2 dy + dz].
 template <int FORM>
 __device__ __forceinline__ void face_corners(const double (&t)[4], int, double (&f)[4]) {
+  if (FORM != kFaces) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) f[s] = t[s];
+    return;
+  }
   const double s0 = t[0] + t[1], d0 = t[0] - t[1], s1 = t[2] + t[3], d1 = t[2] - t[3];
   f[0] = s0 + s1;
   f[1] = d0 + d1;
@@ -429,8 +507,8 @@ constexpr int kTileLoads = 8;       // values of a plane tile staged per thread 
 // Blocks of 128 threads resident per SM, as the registers allow without spills:
 // three in FP64 (168 registers), four in FP32 (at most 128; five at 96 spilled up to 56
 // bytes: 31.7 us for the operator of 1M elements, four 28.3).
-template <typename T, bool DENSE>
-constexpr int sweep_resident() { return sizeof(T) == 8 ? (DENSE ? 2 : 3) : 4; }
+template <typename T, bool DENSE, int FORM>
+constexpr int sweep_resident() { return sizeof(T) == 8 ? (FORM == kFaces && DENSE ? 2 : 3) : 4; }
 
 // Each block stages its (bj+1) x (bk+1) node tile of one x-plane in shared memory
 // with asynchronous copies, one value each, consecutive threads on consecutive
@@ -453,13 +531,14 @@ constexpr int sweep_resident() { return sizeof(T) == 8 ? (DENSE ? 2 : 3) : 4; }
 // 9), FP32 45 (28); 512k: FP64 50 (31), FP32 24 (20); 2M in FP32 101 (50).
 //
 // FORM: how an element's product is evaluated.  kFaces transforms a face once for
-// two elements, as above.  The FP32 smoothing steps and residuals of the cycle keep
-// the element-by-element evaluation instead: on states with many void elements a
-// solve carries FP32 rounding differences of the cycle to 1e-7 of the displacement's
-// largest entries, and its answers are to stay the same to the last bit.  Two such
-// forms exist, by grid size (launch_sweep): the compiler's contraction of the plain
-// expressions up to kFusedElements, every operation rounded by itself beyond.  They
-// take about 1.4 times the arithmetic of kFaces.
+// two elements, as above.  The products inside a solve -- smoothing steps, residuals
+// and the hierarchy's own FP64 operator -- keep the element-by-element evaluation
+// instead: FP32 cycles turn a difference of 1e-16 in a Krylov vector into 1e-8 of the
+// displacement of nodes that hang in void alone, the nested Krylov solves of the FP64
+// stacks into 1e-9 of all of it, and their answers are to stay the same to the last
+// bit.  FP32 has two such forms, by grid size (launch_sweep): the compiler's
+// contraction of the plain expressions up to kFusedElements, every operation rounded
+// by itself beyond.  They take about 1.4 times the arithmetic of kFaces.
 //
 // COMPACT: u and y are the free-DOF vectors of the C interface, so neither an
 // expanded copy of u nor a full result is written.  pinfo[plane] is the free index
@@ -469,7 +548,7 @@ constexpr int sweep_resident() { return sizeof(T) == 8 ? (DENSE ? 2 : 3) : 4; }
 constexpr int64_t kFusedElements = 250000;
 
 template <typename T, int EPI, bool DENSE, bool BF, bool COMPACT, int FORM>
-__global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE>())
+__global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE, FORM>())
     sweep_kernel(Grid g, SweepShape sh, const T* __restrict__ E, const uint8_t* __restrict__ nmask,
                  const T* __restrict__ u, const int32_t* __restrict__ ninfo,
                  const int32_t* __restrict__ pinfo, EpiArgs ea) {
@@ -483,6 +562,10 @@ __global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE>())
   T* P = F + 18 * NT;                      // plane tiles [kPlaneBufs][PV]
   T* O = P + kPlaneBufs * PV;              // epilogue operands [2][NT][NO]
   const int t = threadIdx.x;
+  __shared__ __align__(16) double cw[sizeof(T) == 8 && FORM != kFaces ? 8 * kBlockCoefs : 2];
+  if (sizeof(T) == 8 && FORM != kFaces)
+    for (int k = t; k < 8 * kBlockCoefs; k += NT)
+      cw[k] = k % kBlockCoefs < 9 ? c_wht64[k / kBlockCoefs][k % kBlockCoefs] : 0.0;
   const int tj = t / sh.bk, tk = t - tj * sh.bk;
   const int nbk = (g.nz + sh.bk - 1) / (sh.bk - 1);  // ceil((nz+1)/(bk-1))
   const int bjI = blockIdx.x / nbk, bkI = blockIdx.x - bjI * nbk;
@@ -595,7 +678,7 @@ __global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE>())
       T c[3][4], lo[3][4], hi[3][4];
       const T* r = P + ((ie + 1) & (kPlaneBufs - 1)) * PV + at;
       face_values<BF, FORM>(r, r + W, c, own);
-      element_faces<DENSE, BF, FORM>(p, c, Ee, lo, hi);
+      element_faces<DENSE, BF, FORM>(p, c, Ee, cw, lo, hi);
 #pragma unroll
       for (int q = 0; q < 3; ++q)
 #pragma unroll
@@ -688,6 +771,11 @@ static cudaError_t launch_sweep_as(const Grid& g, const SweepShape& sh, const T*
 template <typename T, int EPI, bool BF>
 static cudaError_t launch_sweep(const Grid& g, const SweepShape& sh, const void* E, const uint8_t* nmask,
                                 const void* u, const EpiArgs& ea, cudaStream_t s) {
+  if constexpr (sizeof(T) == 8) {
+    if ((EPI != EPI_APPLY && EPI != EPI_RESID) || ea.by_element)
+      return launch_sweep_as<T, EPI, true, false, false, kElement>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
+                                                                   nullptr, ea, s);
+  }
   if constexpr (sizeof(T) == 4 && !BF && EPI != EPI_APPLY) {
     return g.ne() <= kFusedElements
                ? launch_sweep_as<T, EPI, true, false, false, kElement>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
@@ -697,13 +785,14 @@ static cudaError_t launch_sweep(const Grid& g, const SweepShape& sh, const void*
   } else if constexpr (sizeof(T) == 4) {
     return launch_sweep_as<T, EPI, true, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr, nullptr,
                                                             ea, s);
-  } else {
+  } else if constexpr (EPI == EPI_APPLY || EPI == EPI_RESID) {
     return pattern_on_device()
                ? launch_sweep_as<T, EPI, false, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
                                                                    nullptr, ea, s)
                : launch_sweep_as<T, EPI, true, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
                                                                   nullptr, ea, s);
   }
+  return cudaErrorInvalidValue;
 }
 
 template <typename T, bool BF>

@@ -203,7 +203,7 @@ static int64_t div_up64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // all resident warps.  Coefficients fitted to the times of 500 candidate tiles on six
 // grids between 24 x 12 x 6 and 252 x 126 x 63 (7 % root mean square in FP32, 8 % in
 // FP64; its first choice was up to 17 % slower than the best tile, the best of its
-// first 32 never: hence the tuner's shortlist).
+// first 48 never: hence the tuner's shortlist).
 static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
   const double latency = t == F64 ? 0.638 : 0.740, issue = t == F64 ? 0.0968 : 0.0877;
   const double startup = t == F64 ? 2.03 : 1.85, launch = 4.5;
@@ -267,9 +267,15 @@ SweepShape default_shape(DType t, const Grid& g) {
 }
 
 void fine_apply(Mesh& m, DType t, Epi epi, const void* E, const void* u, const EpiArgs& ea,
-                       cudaStream_t s) {
+                cudaStream_t s) {
   const SweepShape& sh = m.sh[t == F64 ? 0 : 1];
   SF_CUDA(launch_fine(t, epi, m.g, sh, E, m.nmask.as<uint8_t>(), u, ea, s));
+}
+
+// The hierarchy's own FP64 product, element by element (SweepForm).
+void fine_apply64(Gmg& G, Epi epi, const void* u, EpiArgs ea, cudaStream_t s) {
+  ea.by_element = true;
+  fine_apply(*G.m, F64, epi, G.E64.p, u, ea, s);
 }
 
 // Tuner: time candidate sweep shapes on this mesh and keep the fastest.  The
@@ -302,7 +308,7 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
   std::stable_sort(cands.begin(), cands.end(), [&](const SweepShape& a, const SweepShape& b) {
     return sweep_cost(t, m.g, a) < sweep_cost(t, m.g, b);
   });
-  if (cands.size() > 32) cands.resize(32);
+  if (cands.size() > 48) cands.resize(48);
   constexpr int kTuneReps = 8;
   cudaEvent_t e0, e1;
   SF_CUDA(cudaEventCreate(&e0));
@@ -312,8 +318,9 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
   // SIMPFEM_TUNE_VERBOSE=1 prints every candidate's time (stderr)
   const char* vb = getenv("SIMPFEM_TUNE_VERBOSE");
   const bool verbose = vb != nullptr && vb[0] != '\0' && vb[0] != '0';
-  // timed as the residual: in FP32 the form the cycle's smoothing steps run
+  // timed as the residual of a solve: the form its smoothing steps run
   EpiArgs ea;
+  ea.by_element = t == F64;
   ea.y = y.p;
   ea.b = u.p;
   for (const SweepShape& sh : cands) {
@@ -504,6 +511,7 @@ void level_op(Gmg& G, int l, DType vt, int precsel, Epi epi, const void* u, EpiA
   if (l == 0) {
     DType ft = vt;
     if (vt == F32 && precsel == BF16) ft = BF16;
+    ea.by_element = vt == F64;
     fine_apply(*G.m, ft, epi, fine_E(G, vt), u, ea, G.st);
     return;
   }
@@ -971,14 +979,14 @@ static void fgmres(Gmg& G, KrylovWs& K, const double* b, double* x, bool x0_zero
     EpiArgs ea;
     ea.y = y;
     ea.guard = guard;
-    fine_apply(m, F64, EPI_APPLY, G.E64.p, u, ea, G.st);
+    fine_apply64(G, EPI_APPLY, u, ea, G.st);
   };
   E.R = [&G, &m](const double* u, const double* rhs, double* r, const int* guard) {
     EpiArgs ea;
     ea.y = r;
     ea.b = rhs;
     ea.guard = guard;
-    fine_apply(m, F64, EPI_RESID, G.E64.p, u, ea, G.st);
+    fine_apply64(G, EPI_RESID, u, ea, G.st);
   };
   // the preconditioner may move the hierarchy's skip flag; the operator's
   // launches after it take theirs explicitly
@@ -1004,7 +1012,7 @@ void root_local(Gmg& G, const double* rhs, double* x) {
     ea.y = residual;
     ea.b = rhs;
     ea.guard = G.guard;
-    fine_apply(m, F64, EPI_RESID, G.E64.p, x, ea, G.st);
+    fine_apply64(G, EPI_RESID, x, ea, G.st);
   }
   if (G.o.root_local_correction_mode == 2) {
     const int steps = G.o.root_local_correction_inner_steps;
@@ -1022,7 +1030,7 @@ void root_local(Gmg& G, const double* rhs, double* x) {
     EpiArgs ea;
     ea.y = Ac;
     ea.guard = G.guard;
-    fine_apply(m, F64, EPI_APPLY, G.E64.p, corr, ea, G.st);
+    fine_apply64(G, EPI_APPLY, corr, ea, G.st);
     SF_CUDA(launch_trial_residual(F64, n, residual, Ac, sc, 1, nullptr, m.rw, G.guard, G.st));
     SF_CUDA(launch_scalar_op(OP_RLF, sc, 0.0, 0.0, G.guard, G.st));
     SF_CUDA(launch_select_axpy(F64, n, x, corr, sc, 1, G.guard, G.st));
@@ -1036,7 +1044,7 @@ void root_local(Gmg& G, const double* rhs, double* x) {
     EpiArgs ea;
     ea.y = Ac;
     ea.guard = G.guard;
-    fine_apply(m, F64, EPI_APPLY, G.E64.p, corr, ea, G.st);
+    fine_apply64(G, EPI_APPLY, corr, ea, G.st);
     DotSet d2;
     d2.a[0] = Ac; d2.b[0] = Ac;
     d2.a[1] = residual; d2.b[1] = Ac;
@@ -1175,7 +1183,7 @@ static double fine_lambda(Gmg& G) {
   for (int it = 0; it < 20; ++it) {
     EpiArgs ea;
     ea.y = Kv;
-    fine_apply(m, F64, EPI_APPLY, G.E64.p, v, ea, G.st);
+    fine_apply64(G, EPI_APPLY, v, ea, G.st);
     DotSet d2;
     d2.a[0] = v; d2.b[0] = v; d2.c[0] = d; d2.mode[0] = 1;
     d2.a[1] = v; d2.b[1] = Kv;
@@ -1440,7 +1448,6 @@ float time_smoother_step(Gmg& G, int l, int reps) {
   void* xo = vt == t ? L.x[1].p : L.xs[1].p;
   void* rhs = vt == t ? L.rhs.p : L.rhss.p;
   void* d = vt == t ? L.d.p : L.ds.p;
-  const size_t es = vt == F64 ? 8 : 4;
   // non-constant inputs, so the timed step moves data like a real cycle does
   SF_CUDA(launch_fill_hash(vt, L.g.ndof, 11u, x, G.st));
   SF_CUDA(launch_fill_hash(vt, L.g.ndof, 12u, rhs, G.st));
@@ -1525,14 +1532,14 @@ void run_pcg(Gmg& G, const double* b, double* x, double tol, int maxiter, std::v
     EpiArgs ea;
     ea.y = y;
     ea.guard = guard;
-    fine_apply(m, F64, EPI_APPLY, G.E64.p, u, ea, G.st);
+    fine_apply64(G, EPI_APPLY, u, ea, G.st);
   };
   E.R = [&G, &m](const double* u, const double* rhs, double* r, const int* guard) {
     EpiArgs ea;
     ea.y = r;
     ea.b = rhs;
     ea.guard = guard;
-    fine_apply(m, F64, EPI_RESID, G.E64.p, u, ea, G.st);
+    fine_apply64(G, EPI_RESID, u, ea, G.st);
   };
   PrecFn M = [&G](const double* in, double* out, const int*) { apply_full(G, in, out, nullptr); };
   pcg_core(E, M, b, x, tol, maxiter, rb.as<double>(), zb.as<double>(), pb.as<double>(), apb.as<double>(),

@@ -106,6 +106,8 @@ struct KrylovWs {
   int restart = 0;
   int64_t n = 0;
   DevBuf V, Z, w, r, H, cs, sn, g, y, sc, Zptr;
+  DevBuf comm;      // exchange slots of the one-launch Arnoldi column
+  ColumnPlan plan;
   DevBuf flags_dev;     // device-side control flags (read by every guarded kernel)
   PinnedBuf flags_pin;  // host mirror, refreshed by sync_flags()
   KrylovDev kd;
@@ -125,6 +127,11 @@ struct KrylovWs {
     g.alloc(sizeof(double) * (restart + 1));
     y.alloc(sizeof(double) * restart);
     sc.alloc(sizeof(double) * 16);
+    plan = arnoldi_plan(n, cooperative_available());
+    if (plan.per > 0 && !comm.p) {
+      comm.alloc(arnoldi_comm_bytes());
+      SF_CUDA(cudaMemset(comm.p, 0, arnoldi_comm_bytes()));
+    }
     flags_dev.alloc(sizeof(int) * NFLAGS);
     SF_CUDA(cudaMemset(flags_dev.p, 0, sizeof(int) * NFLAGS));
     flags_pin.alloc(sizeof(int) * NFLAGS);
@@ -254,6 +261,7 @@ WhtBlocks make_wht_blocks(const double* ke, double* max_off);
 std::vector<double> make_level1_Q(const double* ke);
 SweepShape default_shape(DType t, const Grid& g);
 void fine_apply(Mesh& m, DType t, Epi epi, const void* E, const void* u, const EpiArgs& ea, cudaStream_t s);
+void fine_apply64(Gmg& G, Epi epi, const void* u, EpiArgs ea, cudaStream_t s);
 void tune_mesh(Mesh& m, DType t, cudaStream_t s);
 Gmg* gmg_create(Mesh* m, const simpfem_gmg_opts& o);
 void gmg_setup(Gmg& G, const double* E, const double* fine_diag_free);

@@ -97,6 +97,44 @@ __device__ __forceinline__ bool grid_allreduce_warp(ulonglong2* slots, unsigned 
   return all;
 }
 
+// Sum of nparts numbered parts, added one by one in their order, as a kernel with one
+// part a block and one thread for the sum adds them.  The caller has put its parts
+// into half + number; every lane holds the sum on return.  stage: shared memory of
+// kGridParts doubles.
+constexpr int kGridParts = 2 * kGridMaxBlocks;
+static_assert(kGridParts + kGridCopies <= kGridMaxVals * kGridSlots, "slots");
+
+__device__ __forceinline__ bool grid_sum_parts_warp(ulonglong2* half, unsigned epoch, int nparts, double* stage,
+                                                    double& v) {
+  const int lane = threadIdx.x & 31, nb = (int)gridDim.x;
+  bool all = false;
+  if (nb <= kGridFlat || blockIdx.x == 0) {
+    constexpr int PER = kGridParts / 32;
+    for (int tries = 0; tries < kGridPolls && !all; ++tries) {
+      bool ok = true;
+#pragma unroll
+      for (int p = 0; p < PER; ++p) {
+        const int b = lane + 32 * p;
+        double got = 0.0;
+        if (b < nparts) ok = grid_get(half + b, got, epoch) && ok;
+        stage[b] = got;
+      }
+      all = __all_sync(0xffffffffu, ok);
+    }
+    __syncwarp();
+    double s = 0.0;
+#pragma unroll 8
+    for (int b = 0; b < nparts; ++b) s += stage[b];
+    __syncwarp();
+    v = s;
+    if (all && nb > kGridFlat && lane < kGridCopies) grid_put(half + kGridParts + lane, s, epoch);
+  } else {
+    for (int tries = 0; tries < kGridPolls && !all; ++tries)
+      all = __all_sync(0xffffffffu, grid_get(half + kGridParts + blockIdx.x % kGridCopies, v, epoch));
+  }
+  return all;
+}
+
 // SMs of the current device (blocks of a cooperative grid at one block per SM).
 int grid_sm_count();
 

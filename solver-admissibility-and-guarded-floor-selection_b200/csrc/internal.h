@@ -37,6 +37,7 @@ struct EpiArgs {
   void* d = nullptr;
   void* xo = nullptr;
   double s1 = 0.0, s2 = 0.0;
+  bool by_element = false;  // FP64 apply and residual: the element-by-element form
   const int* guard = nullptr;  // kernel body runs only when guard is null or *guard != 0
 };
 
@@ -242,6 +243,18 @@ cudaError_t launch_krylov_restart(KrylovDev k, double tol, double* hist_host, in
                                   cudaStream_t s);
 cudaError_t launch_givens(KrylovDev k, int j, double tol, double* hist_host, int hist_cap,
                           cudaStream_t s);
+// One Arnoldi column (Gram-Schmidt, Givens, V_{j+1}) in one cooperative launch.
+struct ColumnPlan {
+  int per = 0;  // elements a thread; 0: not available
+  int parts = 0;  // partial sums of a dot product
+  int blocks = 0;
+  bool wsmem = false;  // w in shared memory instead of registers
+};
+size_t arnoldi_comm_bytes();
+ColumnPlan arnoldi_plan(int64_t n, bool cooperative);
+// comm: arnoldi_comm_bytes() bytes zeroed once, serving one stream at a time
+cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
+                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm, cudaStream_t s);
 cudaError_t launch_scale_vec(int64_t n, const double* src, const double* denom_dev, double* dst,
                              const int* guard, cudaStream_t s);
 cudaError_t launch_backsolve(KrylovDev k, cudaStream_t s);

@@ -72,15 +72,20 @@ void fgmres_core(const KrylovEnv& E, KrylovWs& K, const double* b, double* x, bo
     for (int j = 0; j < inner; ++j) {
       M(K.Vj(j), K.Zj(j), cyc);
       E.A(K.Zj(j), K.w.as<double>(), cyc);
-      double* Hc = kd.H + (size_t)j * ld;
-      SF_CUDA(launch_mgs_first(n, K.Vj(0), K.w.as<double>(), E.rw, Hc, cyc, st));
-      for (int i = 0; i <= j; ++i) {
-        const bool last = (i == j);
-        SF_CUDA(launch_mgs_step(n, K.Vj(i), last ? nullptr : K.Vj(i + 1), K.w.as<double>(), Hc + i, E.rw,
-                                last ? kd.sc + SC_HSQ : Hc + i + 1, cyc, st));
+      if (K.plan.per > 0) {
+        SF_CUDA(launch_arnoldi(n, kd, j, K.Vj(0), K.w.as<double>(), K.Vj(j + 1), tol, hist_dev, hist_cap, K.plan,
+                               K.comm.p, st));
+      } else {
+        double* Hc = kd.H + (size_t)j * ld;
+        SF_CUDA(launch_mgs_first(n, K.Vj(0), K.w.as<double>(), E.rw, Hc, cyc, st));
+        for (int i = 0; i <= j; ++i) {
+          const bool last = (i == j);
+          SF_CUDA(launch_mgs_step(n, K.Vj(i), last ? nullptr : K.Vj(i + 1), K.w.as<double>(), Hc + i, E.rw,
+                                  last ? kd.sc + SC_HSQ : Hc + i + 1, cyc, st));
+        }
+        SF_CUDA(launch_givens(kd, j, tol, hist_dev, hist_cap, st));
+        SF_CUDA(launch_scale_vec(n, K.w.as<double>(), kd.sc + SC_HNORM, K.Vj(j + 1), cyc, st));
       }
-      SF_CUDA(launch_givens(kd, j, tol, hist_dev, hist_cap, st));
-      SF_CUDA(launch_scale_vec(n, K.w.as<double>(), kd.sc + SC_HNORM, K.Vj(j + 1), cyc, st));
       if (host_control) {
         K.sync_flags(st);
         if (!K.hflags()[F_CYC]) break;

@@ -5,6 +5,8 @@
 // so every dot product is bitwise reproducible run to run.
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "gridcomm.cuh"
 
@@ -699,22 +701,21 @@ __global__ void krylov_restart_kernel(KrylovDev k, double tol, double* hist_host
   k.g[0] = beta;
 }
 
-// Givens update of column j (the reference's host-side loop, done on the device).
-__global__ void givens_kernel(KrylovDev k, int j, double tol, double* hist_host, int hist_cap) {
+// Givens update of column j (the reference's host-side loop, done on the device);
+// H[0..j] holds the column's projections.
+__device__ __forceinline__ void givens_update(const KrylovDev& k, int j, double h_norm, double tol, double* hist,
+                                              int hist_cap) {
   int* f = k.flags;
-  if (!f[F_CYC]) return;
   const int ld = k.restart + 1;
   double* H = k.H + (int64_t)j * ld;  // column j
-  const double h_norm = sqrt(k.sc[SC_HSQ]);
-  H[j + 1] = h_norm;
   k.sc[SC_HNORM] = h_norm;
+  double cur = H[0];  // the rotated entry carried along the column
   for (int i = 0; i < j; ++i) {
-    const double a = H[i], b = H[i + 1];
-    const double tmp = __dadd_rn(__dmul_rn(k.cs[i], a), __dmul_rn(k.sn[i], b));
-    H[i + 1] = __dadd_rn(__dmul_rn(-k.sn[i], a), __dmul_rn(k.cs[i], b));
-    H[i] = tmp;
+    const double nxt = H[i + 1], c = k.cs[i], s = k.sn[i];
+    H[i] = __dadd_rn(__dmul_rn(c, cur), __dmul_rn(s, nxt));
+    cur = __dadd_rn(__dmul_rn(-s, cur), __dmul_rn(c, nxt));
   }
-  const double hjj = H[j], hj1 = H[j + 1];
+  const double hjj = cur, hj1 = h_norm;
   const double denom = sqrt(__dadd_rn(__dmul_rn(hjj, hjj), __dmul_rn(hj1, hj1)));
   double c, sn;
   if (denom < 1e-300) {
@@ -734,7 +735,7 @@ __global__ void givens_kernel(KrylovDev k, int j, double tol, double* hist_host,
   f[F_TOTAL] += 1;
   f[F_JF] = j + 1;
   const double rel = fabs(k.g[j + 1]) / k.sc[SC_BNORM];
-  if (hist_host != nullptr && f[F_HISTN] < hist_cap) hist_host[f[F_HISTN]] = rel;
+  if (hist != nullptr && f[F_HISTN] < hist_cap) hist[f[F_HISTN]] = rel;
   f[F_HISTN] += 1;
   if (rel <= tol) {
     f[F_CONV] = 1;
@@ -749,6 +750,255 @@ __global__ void givens_kernel(KrylovDev k, int j, double tol, double* hist_host,
     f[F_BREAK] = 1;
     f[F_CYC] = 0;
   }
+}
+
+__global__ void givens_kernel(KrylovDev k, int j, double tol, double* hist, int hist_cap) {
+  if (!k.flags[F_CYC]) return;
+  givens_update(k, j, sqrt(k.sc[SC_HSQ]), tol, hist, hist_cap);
+}
+
+// One Arnoldi column in one cooperative launch: modified Gram-Schmidt of w against
+// V_0 .. V_j, the Givens update and V_{j+1} = w / |w|.
+//
+// Launched step by step a projection cost 6.6 us at 0.2 M and 14 us at 1.6 M
+// unknowns: w, v_i and v_{i+1} read and w written again for each (51 MB at 1.6 M),
+// one thread adding 296 partial sums, a launch.  Here w stays in registers (MP * PER
+// values a thread; WSMEM: in shared memory), every v_i is read once, by
+// asynchronous copies into slots of the thread's own that fly during the grid
+// exchange of the step before (WSMEM: twice, through L2), and the step is that one
+// exchange.  The block that gathers the exchanges is the one that rotates.
+//
+// The sums are the launched kernels' to the last bit (nested solves and FP32 cycles
+// amplify a difference of 1e-16 beyond 1e-9 of the solution): the vectors are split
+// into the same parts, part p owning the elements p * kRedThreads + t, + parts *
+// kRedThreads, ..., and one chain adds the parts in order (1.2 us of an exchange's
+// 3).  A block holds 2 * MP parts; MP is chosen for about eight elements a thread,
+// because fewer blocks exchange faster and leave SMs to other streams (45 x 30 x 30,
+// eight solves at a time: with two parts in every block 148 blocks of each solve
+// queued for all SMs at once and the batch took 36.9 ms against 33.3 launched).
+constexpr int kColThreads = 2 * kRedThreads;
+
+template <int MP, int PER, bool WSMEM>
+__global__ void __launch_bounds__(kColThreads, 1)
+    arnoldi_kernel(int64_t n, KrylovDev k, int j, const double* __restrict__ V, const double* __restrict__ w,
+                   double* __restrict__ vnew, double tol, double* hist, int hist_cap, int per, int parts,
+                   ulonglong2* slots, unsigned* last) {
+  if (!k.flags[F_CYC]) return;
+  extern __shared__ __align__(16) double csm[];  // WSMEM: w [per][threads]; else two vectors [2][MP * PER][threads]
+  __shared__ double red[MP * kColThreads / 32], stage[kGridParts];
+  __shared__ double total;
+  __shared__ int good;
+  constexpr int NE = MP * PER;  // elements a thread
+  static_assert(!WSMEM || (MP == 1 && PER == 1), "one part per thread there");
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int len = (int)n;  // the plan bounds it
+  const int part0 = (int)blockIdx.x * 2 * MP;
+  const int first = part0 * kRedThreads + tid, stride = parts * kRedThreads;
+  // element q of the thread's m-th part (number part0 + 2 m, + 1 in the upper half);
+  // len: none.  A part beyond the last would alias elements of the others.
+  auto element = [&](int m, int q) -> int {
+    const int base = first + m * kColThreads;
+    const int e = base + q * stride;
+    return base < stride && e < len ? e : len;
+  };
+  unsigned epoch = *(volatile unsigned*)last;
+  double wr[NE];
+  auto fetch = [&](int i) {  // V_i into slot i & 1
+    const double* src = V + (int64_t)i * n;
+    double* dst = csm + (size_t)(i & 1) * NE * kColThreads + tid;
+#pragma unroll
+    for (int m = 0; m < MP; ++m)
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+        const int e = element(m, q);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(dst + (m * PER + q) * kColThreads)),
+                     "l"(e < len ? src + e : V), "r"(e < len ? 8 : 0));
+      }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  // the grid's sum of the parts v[m]; false when the exchange ran out of its wait
+  auto grid_sum = [&](const double (&v)[MP], double& out) -> bool {
+#pragma unroll
+    for (int m = 0; m < MP; ++m) {
+      double s = v[m];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) red[m * (kColThreads / 32) + wid] = s;
+    }
+    __syncthreads();
+    ++epoch;
+    if (wid == 0) {
+      ulonglong2* half = slots + (size_t)(epoch & 1) * kGridMaxVals * kGridSlots;
+#pragma unroll
+      for (int z = 0; z < (MP + 1) / 2; ++z) {  // eight warps a part, four parts a round
+        const int r = z * 32 + lane;
+        double s = r < MP * kColThreads / 32 ? red[r] : 0.0;
+#pragma unroll
+        for (int o = kRedThreads / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const int mine = r / 8;
+        if (r % 8 == 0 && mine < 2 * MP && part0 + mine < parts) grid_put(half + part0 + mine, s, epoch);
+      }
+      double s = 0.0;
+      const bool all = grid_sum_parts_warp(half, epoch, parts, stage, s);
+      if (lane == 0) {
+        total = s;
+        good = all ? 1 : 0;
+      }
+    }
+    __syncthreads();
+    out = total;
+    return good != 0;
+  };
+  const int ld = k.restart + 1;
+  double* H = k.H + (int64_t)j * ld;
+  double h = 0.0, part[MP];
+#pragma unroll
+  for (int m = 0; m < MP; ++m) part[m] = 0.0;
+  if constexpr (WSMEM) {
+    for (int q = 0; q < per; ++q) {
+      const int e = element(0, q);
+      const double x = e < len ? w[e] : 0.0;
+      csm[q * kColThreads + tid] = x;
+      if (e < len) part[0] = fma(V[e], x, part[0]);
+    }
+  } else {
+    fetch(0);
+    if (j > 0) fetch(1);
+#pragma unroll
+    for (int m = 0; m < MP; ++m)
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+        const int e = element(m, q);
+        wr[m * PER + q] = e < len ? w[e] : 0.0;
+      }
+    if (j > 0) asm volatile("cp.async.wait_group 1;\n" ::);
+    else asm volatile("cp.async.wait_group 0;\n" ::);
+#pragma unroll
+    for (int m = 0; m < MP; ++m)
+#pragma unroll
+      for (int q = 0; q < PER; ++q) part[m] = fma(csm[(m * PER + q) * kColThreads + tid], wr[m * PER + q], part[m]);
+  }
+  bool ok = grid_sum(part, h);
+  for (int i = 0; ok && i <= j; ++i) {
+    if (blockIdx.x == 0 && tid == 0) H[i] = h;
+#pragma unroll
+    for (int m = 0; m < MP; ++m) part[m] = 0.0;
+    if constexpr (WSMEM) {
+      const double* vi = V + (int64_t)i * n;
+      const double* vn = i < j ? vi + n : nullptr;
+#pragma unroll 8
+      for (int q = 0; q < per; ++q) {
+        const int e = element(0, q);
+        if (e < len) {
+          const double x = sub_rn(csm[q * kColThreads + tid], mul_rn(h, vi[e]));
+          csm[q * kColThreads + tid] = x;
+          part[0] = fma(vn ? vn[e] : x, x, part[0]);
+        }
+      }
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::);
+      const double* vi = csm + (size_t)(i & 1) * NE * kColThreads + tid;
+      const double* vn = csm + (size_t)((i + 1) & 1) * NE * kColThreads + tid;
+#pragma unroll
+      for (int m = 0; m < MP; ++m)
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+          const int r = m * PER + q;
+          wr[r] = sub_rn(wr[r], mul_rn(h, vi[r * kColThreads]));
+          part[m] = fma(i < j ? vn[r * kColThreads] : wr[r], wr[r], part[m]);
+        }
+      if (i + 2 <= j) fetch(i + 2);  // into the slot just read, by this thread alone
+    }
+    ok = grid_sum(part, h);
+  }
+  const double hn = sqrt(h);  // h = <w, w>
+  if (ok) {
+    if constexpr (WSMEM) {
+      for (int q = 0; q < per; ++q) {
+        const int e = element(0, q);
+        if (e < len) vnew[e] = csm[q * kColThreads + tid] / hn;
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < MP; ++m)
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+          const int e = element(m, q);
+          if (e < len) vnew[e] = wr[m * PER + q] / hn;
+        }
+    }
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    if (ok) {
+      givens_update(k, j, hn, tol, hist, hist_cap);
+    } else {  // the solve ends unconverged; its caller's recomputed residual refuses the iterate
+      k.flags[F_DONE] = 1;
+      k.flags[F_NOTDONE] = 0;
+      k.flags[F_CYC] = 0;
+    }
+    *last = epoch;
+  }
+}
+
+size_t arnoldi_comm_bytes() { return kGridCommBytes + 16; }
+
+// The variant of the one-launch column; per = 0: the vectors are too long (or the
+// device cannot), the launched form runs.
+ColumnPlan arnoldi_plan(int64_t n, bool cooperative) {
+  ColumnPlan p;
+  if (!cooperative || n < 1) return p;
+  const int parts = red_blocks(n);
+  const int64_t per = div_up(n, (int64_t)parts * kRedThreads);
+  if (per * kColThreads * 8 > 216 * 1024) return p;
+  const int mp = per == 1 ? 8 : (per == 2 ? 4 : (per <= 4 ? 2 : 1));
+  const int blocks = (parts + 2 * mp - 1) / (2 * mp);
+  if (blocks > grid_sm_count()) return p;
+  p.per = (int)per;
+  p.parts = parts;
+  p.blocks = blocks;
+  p.wsmem = per > 24;
+  return p;
+}
+
+struct ColumnKernel {
+  const void* fn;
+  int elements;  // a thread
+};
+// by plan: MP * PER elements a thread
+static ColumnKernel column_kernel(const ColumnPlan& p) {
+  if (p.wsmem) return {(const void*)arnoldi_kernel<1, 1, true>, 0};
+  if (p.per == 1) return {(const void*)arnoldi_kernel<8, 1, false>, 8};
+  if (p.per == 2) return {(const void*)arnoldi_kernel<4, 2, false>, 8};
+  if (p.per <= 4) return {(const void*)arnoldi_kernel<2, 4, false>, 8};
+  if (p.per <= 8) return {(const void*)arnoldi_kernel<1, 8, false>, 8};
+  if (p.per <= 12) return {(const void*)arnoldi_kernel<1, 12, false>, 12};
+  return {(const void*)arnoldi_kernel<1, 24, false>, 24};
+}
+
+cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
+                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm, cudaStream_t s) {
+  static std::atomic<uint64_t> attr_done;
+  cudaError_t e = once_per_device(attr_done, [] {
+    for (const void* f : {(const void*)arnoldi_kernel<1, 1, true>, (const void*)arnoldi_kernel<8, 1, false>,
+                          (const void*)arnoldi_kernel<4, 2, false>, (const void*)arnoldi_kernel<2, 4, false>,
+                          (const void*)arnoldi_kernel<1, 8, false>, (const void*)arnoldi_kernel<1, 12, false>,
+                          (const void*)arnoldi_kernel<1, 24, false>}) {
+      const cudaError_t e2 = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+      if (e2 != cudaSuccess) return e2;
+    }
+    return cudaSuccess;
+  });
+  if (e != cudaSuccess) return e;
+  const ColumnKernel c = column_kernel(p);
+  const size_t smem = (size_t)(p.wsmem ? p.per : 2 * c.elements) * kColThreads * sizeof(double);
+  ulonglong2* slots = (ulonglong2*)comm;
+  unsigned* last = (unsigned*)((char*)comm + kGridCommBytes);
+  KrylovDev kd = k;
+  int per = p.per, parts = p.parts;
+  void* args[] = {&n, &kd, &j, (void*)&V, (void*)&w, &vnew, &tol, &hist, &hist_cap, &per, &parts, &slots, &last};
+  e = cudaLaunchCooperativeKernel(c.fn, dim3(p.blocks), dim3(kColThreads), args, smem, s);
+  return e != cudaSuccess ? e : sf_launched(1);
 }
 
 // dst = src / (*denom)   (V[j+1] = w / h_norm ; V[0] = r / beta)

@@ -116,7 +116,7 @@ Attempt attempt(Worker& W, const simpfem_policy_opts& o, const double* density, 
   EpiArgs ea;
   ea.y = G.tmp64a.p;
   ea.b = b;
-  fine_apply(m, F64, EPI_RESID, G.E64.p, x, ea, W.st);
+  fine_apply64(G, EPI_RESID, x, ea, W.st);
   DotSet ds;
   ds.a[0] = G.tmp64a.p;
   ds.b[0] = G.tmp64a.p;

@@ -216,7 +216,6 @@ void* trace_level(Tracer& T, int l, const void* rhs) {
 
 void trace_cycle(Gmg& G, const double* rhs_full, int cycle_type, std::vector<double>* visits, double* summary) {
   G.guard = nullptr;
-  Mesh& m = *G.m;
   const int64_t n = G.nfull();
   Tracer T{G, cycle_type, visits};
   T.dd.alloc(8 * sizeof(double));
@@ -238,7 +237,7 @@ void trace_cycle(Gmg& G, const double* rhs_full, int cycle_type, std::vector<dou
     EpiArgs ea;
     ea.y = res;
     ea.b = rhs_full;
-    fine_apply(m, F64, EPI_RESID, G.E64.p, x, ea, G.st);
+    fine_apply64(G, EPI_RESID, x, ea, G.st);
   };
   auto norm64 = [&](const double* v) { return sqrt(std::max(T.dot(F64, n, v, v), 0.0)); };
   residual();
