@@ -1409,18 +1409,19 @@ void gmg_setup(Gmg& G, const double* E, const double* fine_diag_free) {
     if (reest || std::isnan(L.lam)) L.lam = sparse_lambda(G, l);
     pt.mark("lambda coarse");
     const int p = G.prec[l];
-    const bool need32 = (p == F32) || (G.cyc == F32);
+    // an FP32 copy where the level is applied in FP32; the mixed cycle's BF16 levels
+    // read the BF16 copy alone
+    const bool need32 = p == F32 || (G.cyc == F32 && p != BF16);
     if (need32) {
       L.K32.alloc(4 * 243 * L.g.nn);
       SF_CUDA(launch_convert(F64, F32, L.K64.p, L.K32.p, 243 * L.g.nn, nullptr, G.st));
+    }
+    if (need32 || G.cyc == F32) {
       L.dinv32.alloc(4 * L.g.ndof);
       SF_CUDA(launch_convert(F64, F32, L.dinv64.p, L.dinv32.p, L.g.ndof, nullptr, G.st));
-      if (G.cyc == F32 && L.xs[0].p == nullptr) {
-        // nothing: mixed mode uses the cycle buffers directly
-      }
     }
     if (G.cyc == F32 && p == BF16) {
-      L.K16.alloc(2 * 288 * L.g.nn);  // node-major by neighbour column, 288 entries per node
+      L.K16.alloc(stencil_colmajor_bytes(L.g.nn));
       SF_CUDA(launch_stencil_colmajor_bf16(L.g.nn, L.K64.as<double>(), L.K16.as<__nv_bfloat16>(), G.st));
     }
   }

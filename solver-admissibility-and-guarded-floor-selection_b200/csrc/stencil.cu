@@ -35,53 +35,124 @@ __device__ __forceinline__ float coef_to<float, __nv_bfloat16>(__nv_bfloat16 c) 
   return __bfloat162float(c);
 }
 
-// One thread per (node, output component r): 81 coefficient loads (coalesced
-// across the warp's consecutive nodes) and 81 gathered vector loads.  A
-// neighbour outside the grid has zero coefficients (the assembly writes them),
-// so its offset is clamped to 0 instead of branching and every load of the
-// thread can be in flight at once.  32-bit node indices (levels >= 1 have at
-// most 1/8 of the fine nodes; the launcher checks 3 * nn < 2^31).
-template <typename VT, typename CT, int EPI>
-__global__ void __launch_bounds__(256) stencil_kernel(Grid g, const CT* __restrict__ coef,
-                                                      const uint8_t* __restrict__ mask, const VT* __restrict__ u,
-                                                      EpiArgs ea) {
-  if (guard_off(ea.guard)) return;
-  const int nn = (int)g.nn;
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y;
-  if (n >= nn) return;
-  const int NZ1 = g.nz + 1, NY1 = g.ny + 1;
-  const int k = n % NZ1, jq = n / NZ1;
-  const int j = jq % NY1, i = jq / NY1;
-  const int sx[3] = {i > 0 ? -NY1 * NZ1 : 0, 0, i < g.nx ? NY1 * NZ1 : 0};
-  const int sy[3] = {j > 0 ? -NZ1 : 0, 0, j < g.ny ? NZ1 : 0};
-  const int sz[3] = {k > 0 ? -1 : 0, 0, k < g.nz ? 1 : 0};
-  const CT* cp = coef + (int64_t)(r * 3) * nn + n;
-  VT acc = VT(0);
-#pragma unroll
-  for (int o = 0; o < 27; ++o) {
-    const VT* um = u + 3 * (n + sx[o / 9] + sy[(o / 3) % 3] + sz[o % 3]);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) acc += coef_to<VT, CT>(cp[(int64_t)(o * 9 + q) * nn]) * um[q];
+// Unsigned division by an invariant d >= 1 for dividends below 2^31: one multiply
+// instead of the twenty instructions of an integer division.
+struct FastDiv {
+  unsigned d = 1, mul = 0, shift = 0;
+  static FastDiv make(unsigned d) {
+    FastDiv f;
+    f.d = d;
+    unsigned l = 0;
+    while ((1u << l) < d && l < 31) ++l;  // 2^l >= d
+    f.shift = l;
+    f.mul = (unsigned)((((uint64_t)1 << 32) * (((uint64_t)1 << l) - d)) / d + 1);
+    return f;
   }
-  const int dof = 3 * n + r;
-  epilogue<VT, EPI>(ea, dof, mask[dof] != 0, acc, u[dof]);
+  __device__ __forceinline__ unsigned div(unsigned n) const {
+    return (unsigned)(((uint64_t)__umulhi(n, mul) + n) >> shift);
+  }
+};
+
+// 32 nodes a block, nine warps: warp col = 3 ox + oy loads what couples its 32 nodes'
+// rows to their three z-neighbours in column (ox, oy) -- 27 coefficients and nine
+// vector entries a lane, coalesced over the nodes and all in flight together -- and
+// the warps then take up the rows' sums one after the other, column by column, so
+// a row is one chain of 81 multiply-adds in the operator's order (nested Krylov
+// solves hang on its last bit); 96 threads apply the epilogue with operands they read
+// up front.  (A thread per row had 6 warps on an SM for its 81 loads: 8.0 us on the
+// 9,471 + 1,386 nodes of the two coarse levels of 80 x 40 x 20, now 3.9; reading the
+// operator from L2 takes 2.  69,741 nodes are bound by their 136 MB of coefficients
+// either way.)  A neighbour outside the grid has zero coefficients (the
+// assembly writes them), so its offset is clamped to 0 instead of branching.  32-bit
+// node indices (levels >= 1 have at most 1/8 of the fine nodes; the launcher checks
+// 3 * nn < 2^31).
+constexpr int kStencilNodes = 32, kStencilThreads = 9 * 32;
+
+template <typename VT, typename CT, int EPI>
+__global__ void __launch_bounds__(kStencilThreads) stencil_kernel(Grid g, FastDiv dz, FastDiv dy,
+                                                                  const CT* __restrict__ coef,
+                                                                  const uint8_t* __restrict__ mask,
+                                                                  const VT* __restrict__ u, EpiArgs ea) {
+  if (guard_off(ea.guard)) return;
+  __shared__ VT part[kStencilNodes * 3];
+  const int nn = (int)g.nn, tid = threadIdx.x, col = tid >> 5, nl = tid & 31;
+  const int n0 = blockIdx.x * kStencilNodes, n = min(n0 + nl, nn - 1);
+  const int dof = 3 * n0 + tid;
+  const bool row = tid < 3 * kStencilNodes && dof < 3 * nn;
+  VT ob = VT(0), od = VT(0), oi = VT(0), ox_ = VT(0);
+  uint8_t fr = 0;
+  if (row) {
+    fr = mask[dof];
+    if (EPI != EPI_APPLY) ob = ((const VT*)ea.b)[dof];
+    if (EPI == EPI_CHEB1 || EPI == EPI_CHEB || EPI == EPI_JAC) oi = ((const VT*)ea.dinv)[dof];
+    if (EPI == EPI_CHEB) od = ((const VT*)ea.d)[dof];
+    if (EPI == EPI_CHEB1 || EPI == EPI_CHEB || EPI == EPI_JAC) ox_ = u[dof];
+  }
+  const int NZ1 = g.nz + 1, NY1 = g.ny + 1;
+  const int jq = (int)dz.div(n), k = n - jq * NZ1, i = (int)dy.div(jq), j = jq - i * NY1;
+  const int ox = col / 3, oy = col - 3 * ox;
+  const int sx = ox == 0 ? (i > 0 ? -NY1 * NZ1 : 0) : (ox == 2 ? (i < g.nx ? NY1 * NZ1 : 0) : 0);
+  const int sy = oy == 0 ? (j > 0 ? -NZ1 : 0) : (oy == 2 ? (j < g.ny ? NZ1 : 0) : 0);
+  const CT* cp = coef + (int64_t)(col * 27) * nn + n;
+  CT cf[27];
+#pragma unroll
+  for (int e = 0; e < 27; ++e) cf[e] = cp[(int64_t)e * nn];
+  VT uv[9];
+#pragma unroll
+  for (int oz = 0; oz < 3; ++oz) {
+    const int sz = oz == 0 ? (k > 0 ? -1 : 0) : (oz == 2 ? (k < g.nz ? 1 : 0) : 0);
+    const VT* um = u + 3 * (n + sx + sy + sz);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) uv[3 * oz + q] = um[q];
+  }
+  for (int c = 0; c < 9; ++c) {
+    if (col == c) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        VT acc = c > 0 ? part[3 * nl + r] : VT(0);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) acc = fma(coef_to<VT, CT>(cf[e / 3 * 9 + r * 3 + e % 3]), uv[e], acc);
+        part[3 * nl + r] = acc;
+      }
+    }
+    __syncthreads();
+  }
+  if (!row) return;
+  const VT ku = part[tid];
+  const bool f = fr != 0;
+  VT* py = (EPI == EPI_APPLY || EPI == EPI_RESID ? (VT*)ea.y : (VT*)ea.xo) + dof;
+  VT res = VT(0), dn = VT(0);
+  if (EPI == EPI_APPLY) {
+    res = ku;
+  } else if (EPI == EPI_RESID) {
+    res = sub_rn(ob, ku);
+  } else if (EPI == EPI_CHEB1) {
+    dn = mul_rn(oi, sub_rn(ob, ku));
+    res = add_rn(ox_, mul_rn((VT)ea.s1, dn));
+  } else if (EPI == EPI_CHEB) {
+    dn = mul_rn((VT)ea.s1, add_rn(mul_rn(oi, sub_rn(ob, ku)), mul_rn((VT)ea.s2, od)));
+    res = add_rn(ox_, dn);
+  } else {
+    res = add_rn(ox_, mul_rn(mul_rn((VT)ea.s1, oi), sub_rn(ob, ku)));
+  }
+  *py = f ? res : VT(0);
+  if (EPI == EPI_CHEB1 || EPI == EPI_CHEB) ((VT*)ea.d)[dof] = f ? dn : VT(0);
 }
 
 template <typename VT, typename CT>
 static cudaError_t stencil_dispatch(Epi epi, const Grid& g, const void* coef, const uint8_t* mask,
                                     const void* u, const EpiArgs& ea, cudaStream_t s) {
   if (3 * g.nn >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
-  const int bs = 256;
-  const dim3 nb(div_up(g.nn, bs), 3);
+  const int bs = kStencilThreads, nb = div_up(g.nn, kStencilNodes);
+  const FastDiv dz = FastDiv::make(g.nz + 1), dy = FastDiv::make(g.ny + 1);
   const CT* c = (const CT*)coef;
   const VT* uu = (const VT*)u;
   switch (epi) {
-    case EPI_APPLY: stencil_kernel<VT, CT, EPI_APPLY><<<nb, bs, 0, s>>>(g, c, mask, uu, ea); break;
-    case EPI_RESID: stencil_kernel<VT, CT, EPI_RESID><<<nb, bs, 0, s>>>(g, c, mask, uu, ea); break;
-    case EPI_CHEB1: stencil_kernel<VT, CT, EPI_CHEB1><<<nb, bs, 0, s>>>(g, c, mask, uu, ea); break;
-    case EPI_CHEB: stencil_kernel<VT, CT, EPI_CHEB><<<nb, bs, 0, s>>>(g, c, mask, uu, ea); break;
-    case EPI_JAC: stencil_kernel<VT, CT, EPI_JAC><<<nb, bs, 0, s>>>(g, c, mask, uu, ea); break;
+    case EPI_APPLY: stencil_kernel<VT, CT, EPI_APPLY><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_RESID: stencil_kernel<VT, CT, EPI_RESID><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_CHEB1: stencil_kernel<VT, CT, EPI_CHEB1><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_CHEB: stencil_kernel<VT, CT, EPI_CHEB><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_JAC: stencil_kernel<VT, CT, EPI_JAC><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
     default: return cudaErrorInvalidValue;
   }
   return sf_launched(1);
@@ -98,48 +169,61 @@ cudaError_t launch_stencil(DType vt, DType ct, Epi epi, const Grid& g, const voi
 }
 
 // ----------------------------------------------------------------------------
-// BF16 stencils of the mixed-precision cycle, node-major by neighbour column:
-// coefC[n * 288 + col * 32 + oz * 9 + r * 3 + q] with col = ox * 3 + oy, i.e.
-// the 27 coefficients coupling node n to its three z-neighbours in column
-// (ox, oy) in one 64-byte slot (entries 27..31 zero).  Made from the FP64
-// structure-of-arrays operator once per setup.
+// BF16 stencils of the mixed-precision cycle, by node and neighbour column.  The 27
+// coefficients coupling node n to its three z-neighbours in column (ox, oy) are 32
+// entries [oz * 9 + r * 3 + q] (27..31 zero), i.e. four 16-byte quarters; quarter q of
+// the nine columns of three consecutive nodes is contiguous:
+// coefC[((n / 3 * 4 + q) * 27 + n % 3 * 9 + col) * 8 + entry % 8], col = ox * 3 + oy.
+// Made from the FP64 structure-of-arrays operator once per setup.
 //
-// Nine lanes per node, three nodes per warp: lane (t, col) loads its slot with
-// four 16-byte loads and the 9 vector entries of its z-neighbours, forms its
-// part of the node's three row sums, and the node's first lane adds the nine
-// parts (in column order, through shared memory) and applies the epilogue with
-// operands it read up front.  The row-per-thread kernel above chains 81 loads
-// per thread (latency-bound on the small coarse levels) and a warp per node
-// spends its issue slots on per-node index and reduction work; this split keeps
-// both small.
-constexpr int kColSlot = 32, kNodeStrideC = 9 * kColSlot;
+// Nine lanes per node, three nodes per warp: lane (t, col) loads its four quarters
+// (a warp's 27 quarters are one run of 432 bytes) and the 9 vector entries of its
+// z-neighbours and forms its part of the node's three row sums; nine lanes then add
+// a row's nine parts each, in column order, and apply its epilogue.  The kernel is
+// bound by its instructions (8.4 M at 69,741 nodes before, 361 a warp): the node's
+// position comes from multiplications instead of divisions, and nine lanes instead of
+// three share the sums (160 x 80 x 40, mean of its two smoothed levels: 9.0 us before,
+// 6.1; 200 x 100 x 50: 15.4, 10.7; reading the larger level takes 6.1 and 12).
+constexpr int kColSlot = 32, kNodeStrideC = 9 * kColSlot, kPackNodes = 30;
 
-// 32 nodes per block: coalesced reads along n of the FP64 operator, the tile
-// transposed through shared memory, coalesced node-major BF16 writes
+__device__ __forceinline__ int64_t col_slot(int n, int col, int quarter) {
+  return ((int64_t)(n / 3 * 4 + quarter) * 27 + n % 3 * 9 + col) * 8;
+}
+
+// 30 nodes per block: coalesced reads along n of the FP64 operator, rounded into
+// shared memory, 16-byte writes of the quarters
 __global__ void __launch_bounds__(256) stencil_colmajor_bf16_kernel(int nn, const double* __restrict__ K64,
                                                                      __nv_bfloat16* __restrict__ out) {
-  __shared__ __nv_bfloat16 tile[32 * kNodeStrideC];
-  const int n0 = blockIdx.x * 32;
+  __shared__ __align__(16) __nv_bfloat16 tile[kPackNodes * kNodeStrideC];
+  const int n0 = blockIdx.x * kPackNodes;
   const int nl = threadIdx.x & 31, c0 = threadIdx.x >> 5;
-  const int cnt = min(32, nn - n0);
-  for (int c = c0; c < kNodeStrideC; c += 8) {
-    const int col = c / kColSlot, w = c % kColSlot;
-    float v = 0.f;
-    if (nl < cnt && w < 27) {
-      const int o = col * 3 + w / 9;  // o = ox * 9 + oy * 3 + oz
-      v = (float)K64[(int64_t)(o * 9 + w % 9) * nn + n0 + nl];
+  const int cnt = min(kPackNodes, nn - n0);
+  if (nl < kPackNodes)
+    for (int c = c0; c < kNodeStrideC; c += 8) {
+      const int col = c / kColSlot, w = c % kColSlot;
+      float v = 0.f;
+      if (nl < cnt && w < 27) {
+        const int o = col * 3 + w / 9;  // o = ox * 9 + oy * 3 + oz
+        v = (float)K64[(int64_t)(o * 9 + w % 9) * nn + n0 + nl];
+      }
+      tile[nl * kNodeStrideC + c] = __float2bfloat16_rn(v);
     }
-    tile[nl * kNodeStrideC + c] = __float2bfloat16_rn(v);
-  }
   __syncthreads();
-  __nv_bfloat16* dst = out + (int64_t)n0 * kNodeStrideC;
-  for (int e = threadIdx.x; e < cnt * kNodeStrideC; e += blockDim.x) dst[e] = tile[e];
+  // nodes beyond the last fill its group of three with zeros
+  const int groups = (cnt + 2) / 3;
+  for (int e = threadIdx.x; e < groups * 3 * 36; e += blockDim.x) {
+    const int nd = e / 36, qc = e % 36, col = qc >> 2, q = qc & 3;
+    *reinterpret_cast<uint4*>(out + col_slot(n0 + nd, col, q)) =
+        *reinterpret_cast<const uint4*>(tile + nd * kNodeStrideC + col * kColSlot + q * 8);
+  }
 }
+
+size_t stencil_colmajor_bytes(int64_t nn) { return (size_t)((nn + 2) / 3 * 3) * kNodeStrideC * 2; }
 
 cudaError_t launch_stencil_colmajor_bf16(int64_t nn, const double* K64, __nv_bfloat16* out, cudaStream_t s) {
   if (nn <= 0) return cudaSuccess;
   if (nn * kNodeStrideC >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
-  stencil_colmajor_bf16_kernel<<<div_up(nn, 32), 256, 0, s>>>((int)nn, K64, out);
+  stencil_colmajor_bf16_kernel<<<div_up(nn, kPackNodes), 256, 0, s>>>((int)nn, K64, out);
   return sf_launched(1);
 }
 
@@ -147,38 +231,39 @@ __device__ __forceinline__ float bf16_lo(unsigned w) { return __uint_as_float(w 
 __device__ __forceinline__ float bf16_hi(unsigned w) { return __uint_as_float(w & 0xffff0000u); }
 
 template <int EPI>
-__global__ void __launch_bounds__(256) stencil_col_bf16_kernel(Grid g, const __nv_bfloat16* __restrict__ coefC,
+__global__ void __launch_bounds__(256) stencil_col_bf16_kernel(Grid g, FastDiv dz, FastDiv dy,
+                                                               const __nv_bfloat16* __restrict__ coefC,
                                                                const uint8_t* __restrict__ mask,
                                                                const float* __restrict__ u, EpiArgs ea) {
-  __shared__ float part[8][27][3];
+  __shared__ float part[8][9][9];  // [warp][column][3 nodes x 3 rows]
   if (guard_off(ea.guard)) return;
   const int nn = (int)g.nn;
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp * 3 >= nn) return;  // whole warps leave together
-  const int t = lane / 9, col = lane - 9 * t;
-  const int64_t n64 = warp * 3 + t;
-  const bool act = lane < 27 && n64 < nn;
-  const int n = act ? (int)n64 : 0;
-  EpiOperands<float, EPI> eo;
-  float xv[3];
-  if (act && col == 0) {
-    eo.load(ea, 3 * (int64_t)n, mask);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) xv[c] = u[3 * n + c];
+  const int group = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);  // three nodes
+  if (group * 3 >= nn) return;  // whole warps leave together
+  // the row of this lane's sums
+  const int dof = 9 * group + lane;
+  const bool row = lane < 9 && dof < 3 * nn;
+  float ob = 0.f, oi = 0.f, od = 0.f, xv = 0.f;
+  uint8_t fr = 0;
+  if (row) {
+    fr = mask[dof];
+    if (EPI != EPI_APPLY) ob = ((const float*)ea.b)[dof];
+    if (EPI == EPI_CHEB1 || EPI == EPI_CHEB || EPI == EPI_JAC) oi = ((const float*)ea.dinv)[dof];
+    if (EPI == EPI_CHEB) od = ((const float*)ea.d)[dof];
+    if (EPI == EPI_CHEB1 || EPI == EPI_CHEB || EPI == EPI_JAC) xv = u[dof];
   }
-  float p0 = 0.f, p1 = 0.f, p2 = 0.f;
-  if (act) {
+  const int t = lane / 9, col = lane - 9 * t, n = group * 3 + t;
+  if (lane < 27 && n < nn) {
+    const uint4* cp = reinterpret_cast<const uint4*>(coefC) + (int64_t)group * 108 + lane;
+    const uint4 q0 = cp[0], q1 = cp[27], q2 = cp[54], q3 = cp[81];
     const int NZ1 = g.nz + 1, NY1 = g.ny + 1;
-    const int k = n % NZ1, jq = n / NZ1;
-    const int j = jq % NY1, i = jq / NY1;
-    const int ox = col / 3, oy = col % 3;
+    const int jq = (int)dz.div(n), k = n - jq * NZ1, i = (int)dy.div(jq), j = jq - i * NY1;
+    const int ox = col / 3, oy = col - 3 * ox;
     // a neighbour outside the grid has zero coefficients: clamp it to the node itself
     const int dx = (ox == 0) ? (i > 0 ? -NY1 * NZ1 : 0) : (ox == 2 ? (i < g.nx ? NY1 * NZ1 : 0) : 0);
-    const int dy = (oy == 0) ? (j > 0 ? -NZ1 : 0) : (oy == 2 ? (j < g.ny ? NZ1 : 0) : 0);
-    const int base = n + dx + dy;
-    const uint4* cp = reinterpret_cast<const uint4*>(coefC + (int64_t)n * kNodeStrideC + col * kColSlot);
-    const uint4 q0 = cp[0], q1 = cp[1], q2 = cp[2], q3 = cp[3];
+    const int dyo = (oy == 0) ? (j > 0 ? -NZ1 : 0) : (oy == 2 ? (j < g.ny ? NZ1 : 0) : 0);
+    const int base = n + dx + dyo;
     const unsigned wv[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
                              q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
     float cf[28];
@@ -187,47 +272,57 @@ __global__ void __launch_bounds__(256) stencil_col_bf16_kernel(Grid g, const __n
       cf[2 * e] = bf16_lo(wv[e]);
       cf[2 * e + 1] = bf16_hi(wv[e]);
     }
+    float p0 = 0.f, p1 = 0.f, p2 = 0.f;
 #pragma unroll
     for (int oz = 0; oz < 3; ++oz) {
-      const int dz = (oz == 0) ? (k > 0 ? -1 : 0) : (oz == 2 ? (k < g.nz ? 1 : 0) : 0);
-      const float* um = u + 3 * (base + dz);
+      const int dzo = (oz == 0) ? (k > 0 ? -1 : 0) : (oz == 2 ? (k < g.nz ? 1 : 0) : 0);
+      const float* um = u + 3 * (base + dzo);
       const float u0 = um[0], u1 = um[1], u2 = um[2];
       const float* c = cf + oz * 9;
       p0 = fmaf(c[0], u0, fmaf(c[1], u1, fmaf(c[2], u2, p0)));
       p1 = fmaf(c[3], u0, fmaf(c[4], u1, fmaf(c[5], u2, p1)));
       p2 = fmaf(c[6], u0, fmaf(c[7], u1, fmaf(c[8], u2, p2)));
     }
-  }
-  if (lane < 27) {
-    part[wib][lane][0] = p0;
-    part[wib][lane][1] = p1;
-    part[wib][lane][2] = p2;
+    part[wib][col][3 * t] = p0;
+    part[wib][col][3 * t + 1] = p1;
+    part[wib][col][3 * t + 2] = p2;
   }
   __syncwarp();
-  if (act && col == 0) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+  if (!row) return;
+  float ku = 0.f;
 #pragma unroll
-    for (int cc = 0; cc < 9; ++cc) {
-      a0 += part[wib][lane + cc][0];
-      a1 += part[wib][lane + cc][1];
-      a2 += part[wib][lane + cc][2];
-    }
-    eo.apply(ea, 3 * (int64_t)n, 0, a0, xv[0]);
-    eo.apply(ea, 3 * (int64_t)n + 1, 1, a1, xv[1]);
-    eo.apply(ea, 3 * (int64_t)n + 2, 2, a2, xv[2]);
+  for (int cc = 0; cc < 9; ++cc) ku += part[wib][cc][lane];
+  const bool f = fr != 0;
+  float* py = (EPI == EPI_APPLY || EPI == EPI_RESID ? (float*)ea.y : (float*)ea.xo) + dof;
+  float res = 0.f, dn = 0.f;
+  if (EPI == EPI_APPLY) {
+    res = ku;
+  } else if (EPI == EPI_RESID) {
+    res = sub_rn(ob, ku);
+  } else if (EPI == EPI_CHEB1) {
+    dn = mul_rn(oi, sub_rn(ob, ku));
+    res = add_rn(xv, mul_rn((float)ea.s1, dn));
+  } else if (EPI == EPI_CHEB) {
+    dn = mul_rn((float)ea.s1, add_rn(mul_rn(oi, sub_rn(ob, ku)), mul_rn((float)ea.s2, od)));
+    res = add_rn(xv, dn);
+  } else {
+    res = add_rn(xv, mul_rn(mul_rn((float)ea.s1, oi), sub_rn(ob, ku)));
   }
+  *py = f ? res : 0.f;
+  if (EPI == EPI_CHEB1 || EPI == EPI_CHEB) ((float*)ea.d)[dof] = f ? dn : 0.f;
 }
 
 cudaError_t launch_stencil_col_bf16(Epi epi, const Grid& g, const __nv_bfloat16* coefC, const uint8_t* mask,
                                     const float* u, const EpiArgs& ea, cudaStream_t s) {
   if (3 * g.nn >= (int64_t(1) << 31) || g.nn * kNodeStrideC >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
   const int nb = div_up(div_up(g.nn, 3), 8);
+  const FastDiv dz = FastDiv::make(g.nz + 1), dy = FastDiv::make(g.ny + 1);
   switch (epi) {
-    case EPI_APPLY: stencil_col_bf16_kernel<EPI_APPLY><<<nb, 256, 0, s>>>(g, coefC, mask, u, ea); break;
-    case EPI_RESID: stencil_col_bf16_kernel<EPI_RESID><<<nb, 256, 0, s>>>(g, coefC, mask, u, ea); break;
-    case EPI_CHEB1: stencil_col_bf16_kernel<EPI_CHEB1><<<nb, 256, 0, s>>>(g, coefC, mask, u, ea); break;
-    case EPI_CHEB: stencil_col_bf16_kernel<EPI_CHEB><<<nb, 256, 0, s>>>(g, coefC, mask, u, ea); break;
-    case EPI_JAC: stencil_col_bf16_kernel<EPI_JAC><<<nb, 256, 0, s>>>(g, coefC, mask, u, ea); break;
+    case EPI_APPLY: stencil_col_bf16_kernel<EPI_APPLY><<<nb, 256, 0, s>>>(g, dz, dy, coefC, mask, u, ea); break;
+    case EPI_RESID: stencil_col_bf16_kernel<EPI_RESID><<<nb, 256, 0, s>>>(g, dz, dy, coefC, mask, u, ea); break;
+    case EPI_CHEB1: stencil_col_bf16_kernel<EPI_CHEB1><<<nb, 256, 0, s>>>(g, dz, dy, coefC, mask, u, ea); break;
+    case EPI_CHEB: stencil_col_bf16_kernel<EPI_CHEB><<<nb, 256, 0, s>>>(g, dz, dy, coefC, mask, u, ea); break;
+    case EPI_JAC: stencil_col_bf16_kernel<EPI_JAC><<<nb, 256, 0, s>>>(g, dz, dy, coefC, mask, u, ea); break;
     default: return cudaErrorInvalidValue;
   }
   return sf_launched(1);
