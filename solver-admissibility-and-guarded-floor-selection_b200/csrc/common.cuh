@@ -130,6 +130,19 @@ struct EpiOperands {
   }
 };
 
+// First smoothing step from a zero start on entry i with right-hand side r
+// (run_smoother's step 0: x = (s dinv) r, or d = dinv r and x = s d).
+template <typename T>
+__device__ __forceinline__ void zero_start(const ZeroStart& z, int64_t i, T r) {
+  if (z.mode == 1) {
+    ((T*)z.x)[i] = mul_rn(mul_rn((T)z.s, ((const T*)z.dinv)[i]), r);
+  } else if (z.mode == 2) {
+    const T d = mul_rn(((const T*)z.dinv)[i], r);
+    ((T*)z.d)[i] = d;
+    ((T*)z.x)[i] = mul_rn((T)z.s, d);
+  }
+}
+
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 }  // namespace simpfem

@@ -586,8 +586,9 @@ static ChebCoefs cheb_coefs(double lm, double lf, int degree, bool f32) {
 
 // Runs `steps` smoothing steps of the level-l operator in dtype t.  x0 null =>
 // zero initial guess.  xa / xb are the ping-pong buffers; returns the result buffer.
+// started: step 0 of a zero initial guess is in xa (and d) already.
 static void* run_smoother(Gmg& G, int l, DType t, int precsel, const void* rhs, const void* x0, void* xa,
-                          void* xb, void* d, const void* dinv, double lm, double lf, int steps) {
+                          void* xb, void* d, const void* dinv, double lm, double lf, int steps, bool started = false) {
   const int64_t n = G.lv[l].g.ndof;
   const bool f32 = (t == F32);
   void* cur = nullptr;
@@ -600,7 +601,9 @@ static void* run_smoother(Gmg& G, int l, DType t, int precsel, const void* rhs, 
       ea.dinv = dinv;
       ea.d = d;
       if (k == 0) {
-        if (x0 == nullptr) {
+        if (started) {
+          // nothing to do
+        } else if (x0 == nullptr) {
           SF_CUDA(launch_cheb_zero(t, n, cc.alpha0, dinv, rhs, d, nxt, G.guard, G.st));
         } else {
           ea.xo = nxt;
@@ -620,7 +623,9 @@ static void* run_smoother(Gmg& G, int l, DType t, int precsel, const void* rhs, 
     // damped Jacobi: x <- x + (omega * dinv) * (rhs - A x)
     const double om = f32 ? (double)(float)G.omega_used : G.omega_used;
     for (int k = 0; k < steps; ++k) {
-      if (k == 0 && x0 == nullptr) {
+      if (k == 0 && started) {
+        // nothing to do
+      } else if (k == 0 && x0 == nullptr) {
         SF_CUDA(launch_jac_zero(t, n, om, dinv, rhs, nxt, G.guard, G.st));
       } else {
         EpiArgs ea;
@@ -637,31 +642,67 @@ static void* run_smoother(Gmg& G, int l, DType t, int precsel, const void* rhs, 
   return cur;
 }
 
-// smooth at level l; x_in null => zero initial guess; result in one of lv[l].x
-void* smooth(Gmg& G, int l, const void* rhs, const void* x_in) {
+// lambda_max, lower fraction and step count of a smoothing run at level l
+struct SmoothSpec {
+  double lm, lf;
+  int steps;
+};
+static SmoothSpec smooth_spec(const Gmg& G, int l) {
+  SmoothSpec sp;
+  sp.lf = G.o.cheb_lower_frac;
+  if (G.high) sp.lf = std::min(G.o.cheb_lower_frac, 1.0 / 100.0);
+  if (l == 0) {
+    sp.lm = G.lv[0].lam;
+    sp.steps = G.fine_deg;
+  } else {
+    sp.lm = std::isfinite(G.lv[l].lam) ? G.lv[l].lam : 1.0;
+    sp.steps = G.coarse_iters;
+  }
+  return sp;
+}
+// whether the reference mode smooths level l in FP32 on cast copies
+static bool smooths_low(const Gmg& G, int l) {
+  const int p = G.prec[l];
+  return G.cyc == F64 && (l == 0 ? (p == F32 || p == BF16) : (p == F32 && G.lv[l].K32.p != nullptr));
+}
+// The zero start of level l's pre-smoothing for the kernel that writes its right-hand
+// side (none at the coarsest level or where the smoother works on cast copies).
+static ZeroStart zero_start_of(Gmg& G, int l) {
+  ZeroStart z;
+  const SmoothSpec sp = smooth_spec(G, l);
+  if (l == G.L - 1 || sp.steps < 1 || smooths_low(G, l)) return z;
+  const bool f32 = G.cyc == F32;
+  z.x = G.lv[l].x[0].p;
+  z.d = G.lv[l].d.p;
+  z.dinv = level_dinv(G, l, G.cyc);
+  if (G.o.smoother_type == 0) {
+    z.mode = 2;
+    z.s = cheb_coefs(sp.lm, sp.lf, sp.steps, f32).alpha0;
+  } else {
+    z.mode = 1;
+    z.s = f32 ? (double)(float)G.omega_used : G.omega_used;
+  }
+  return z;
+}
+
+// smooth at level l; x_in null => zero initial guess, whose first step is in lv[l].x[0]
+// already when started; result in one of lv[l].x
+static void* smooth_from(Gmg& G, int l, const void* rhs, const void* x_in, bool started) {
   Level& L = G.lv[l];
   const int64_t n = L.g.ndof;
-  double lm, lf = G.o.cheb_lower_frac;
-  if (G.high) lf = std::min(G.o.cheb_lower_frac, 1.0 / 100.0);
-  int steps;
-  if (l == 0) {
-    lm = G.lv[0].lam;
-    steps = G.fine_deg;
-  } else {
-    lm = std::isfinite(L.lam) ? L.lam : 1.0;
-    steps = G.coarse_iters;
-  }
+  const SmoothSpec sp = smooth_spec(G, l);
+  const double lm = sp.lm, lf = sp.lf;
+  const int steps = sp.steps;
   const int p = G.prec[l];
   // output buffer that is not x_in
   void* xa = (x_in == L.x[0].p) ? L.x[1].p : L.x[0].p;
   void* xb = (x_in == L.x[0].p) ? L.x[0].p : L.x[1].p;
   if (G.cyc == F32) {
-    return run_smoother(G, l, F32, p, rhs, x_in, xa, xb, L.d.p, level_dinv(G, l, F32), lm, lf, steps);
+    return run_smoother(G, l, F32, p, rhs, x_in, xa, xb, L.d.p, level_dinv(G, l, F32), lm, lf, steps, started);
   }
   // reference mode: FP64 vectors; FP32 / BF16 smoothing on cast copies
-  const bool low = (l == 0) ? (p == F32 || p == BF16) : (p == F32 && L.K32.p != nullptr);
-  if (!low) {
-    return run_smoother(G, l, F64, F64, rhs, x_in, xa, xb, L.d.p, level_dinv(G, l, F64), lm, lf, steps);
+  if (!smooths_low(G, l)) {
+    return run_smoother(G, l, F64, F64, rhs, x_in, xa, xb, L.d.p, level_dinv(G, l, F64), lm, lf, steps, started);
   }
   SF_CUDA(launch_convert(F64, F32, rhs, L.rhss.p, n, G.guard, G.st));
   const void* x0 = nullptr;
@@ -674,6 +715,8 @@ void* smooth(Gmg& G, int l, const void* rhs, const void* x_in) {
   SF_CUDA(launch_convert(F32, F64, r, xa, n, G.guard, G.st));
   return xa;
 }
+
+void* smooth(Gmg& G, int l, const void* rhs, const void* x_in) { return smooth_from(G, l, rhs, x_in, false); }
 
 // ----------------------------------------------------------------------------
 // Coarsest solve (dense via explicit Cholesky inverse factor, or fixed Jacobi-PCG)
@@ -694,6 +737,17 @@ void solve_coarsest(Gmg& G, const void* rhs, void* x) {
                             G.pz.as<double>(), coarse_pcg_count(G), G.pcomm.p, G.guard, G.st));
     return;
   }
+  if (G.coarse_mode == 1) {
+    SF_CUDA(launch_gather_idx(G.cyc, G.nc, G.c_idx.as<int32_t>(), rhs, G.cb.as<double>(), G.guard, G.st));
+    if (G.cyc == F32 && G.LinvF.p)
+      SF_CUDA(launch_coarsest_solve_f32(G.LinvF.as<float>(), G.LinvTF.as<float>(), G.nc, G.cb.as<double>(),
+                                        G.ctmp.as<double>(), G.cx.as<double>(), G.guard, G.st));
+    else
+      SF_CUDA(launch_coarsest_solve(G.Linv.as<double>(), G.LinvT.as<double>(), G.nc, G.cb.as<double>(),
+                                    G.ctmp.as<double>(), G.cx.as<double>(), G.guard, G.st));
+    SF_CUDA(launch_place_idx(G.cyc, n, G.c_didx.as<int32_t>(), G.cx.as<double>(), x, G.guard, G.st));
+    return;
+  }
   const double* b64 = (const double*)rhs;
   double* x64 = (double*)x;
   if (G.cyc == F32) {
@@ -701,19 +755,7 @@ void solve_coarsest(Gmg& G, const void* rhs, void* x) {
     b64 = G.tmp64a.as<double>();
     x64 = G.tmp64b.as<double>();
   }
-  if (G.coarse_mode == 1) {
-    SF_CUDA(launch_gather_idx(G.nc, G.c_idx.as<int32_t>(), b64, G.cb.as<double>(), G.guard, G.st));
-    if (G.cyc == F32 && G.LinvF.p)
-      SF_CUDA(launch_coarsest_solve_f32(G.LinvF.as<float>(), G.LinvTF.as<float>(), G.nc, G.cb.as<double>(),
-                                        G.ctmp.as<double>(), G.cx.as<double>(), G.guard, G.st));
-    else
-      SF_CUDA(launch_coarsest_solve(G.Linv.as<double>(), G.LinvT.as<double>(), G.nc, G.cb.as<double>(),
-                                    G.ctmp.as<double>(), G.cx.as<double>(), G.guard, G.st));
-    SF_CUDA(launch_fill(F64, n, 0.0, x64, G.guard, G.st));
-    SF_CUDA(launch_scatter_idx(G.nc, G.c_idx.as<int32_t>(), G.cx.as<double>(), x64, G.guard, G.st));
-  } else {
-    fixed_pcg_coarse(G, l, b64, x64);
-  }
+  fixed_pcg_coarse(G, l, b64, x64);
   if (G.cyc == F32) SF_CUDA(launch_convert(F64, F32, x64, x, n, G.guard, G.st));
 }
 
@@ -775,7 +817,7 @@ void enrichment_rhs(Gmg& G, const void* residual, void* rc_out) {
     SF_CUDA(launch_restrict(F64, L0.g, L1.g, L0.wx.as<double>(), L0.wy.as<double>(), L0.wz.as<double>(),
                             L1.mask.as<uint8_t>(), r64, G.tmp64a.p, G.guard, G.st));
     SF_CUDA(launch_prolong(F64, L0.g, L1.g, L0.wx.as<double>(), L0.wy.as<double>(), L0.wz.as<double>(),
-                           L0.mask.as<uint8_t>(), G.tmp64a.p, G.tmp64b.p, G.guard, G.st));
+                           L0.mask.as<uint8_t>(), G.tmp64a.p, G.tmp64b.p, false, G.guard, G.st));
     proj = G.tmp64b.as<double>();
   }
   SF_CUDA(launch_enrich_rhs(n, kmode, G.wenrich.as<double>(), G.o.root_enrichment_weight_floor, r64, proj,
@@ -790,65 +832,79 @@ void enrichment_rhs(Gmg& G, const void* residual, void* rc_out) {
   }
 }
 
-static void* cycle(Gmg& G, int l, const void* rhs);
+static void* cycle(Gmg& G, int l, const void* rhs, bool started);
 
-// one coarse visit: restrict `res`, recurse, prolong into lv[l].c
-static void coarse_visit(Gmg& G, int l, const void* res, bool restrict_given) {
+// one coarse visit: restrict `res`, recurse, prolong into lv[l].c, or with add_to
+// non-null into add_to += P e
+static void coarse_visit(Gmg& G, int l, const void* res, bool restrict_given, void* add_to = nullptr) {
   Level& L = G.lv[l];
   Level& C = G.lv[l + 1];
   const DType t = G.cyc;
-  if (!restrict_given)
+  bool started = false;
+  if (!restrict_given) {
+    const ZeroStart zs = zero_start_of(G, l + 1);
+    started = zs.mode != 0;
     SF_CUDA(launch_restrict(t, L.g, C.g, L.wx.as<double>(), L.wy.as<double>(), L.wz.as<double>(),
-                            C.mask.as<uint8_t>(), res, C.rhs.p, G.guard, G.st));
-  void* e = cycle(G, l + 1, C.rhs.p);
+                            C.mask.as<uint8_t>(), res, C.rhs.p, G.guard, G.st, zs));
+  }
+  void* e = cycle(G, l + 1, C.rhs.p, started);
   SF_CUDA(launch_prolong(t, L.g, C.g, L.wx.as<double>(), L.wy.as<double>(), L.wz.as<double>(),
-                         L.mask.as<uint8_t>(), e, L.c.p, G.guard, G.st));
+                         L.mask.as<uint8_t>(), e, add_to ? add_to : L.c.p, add_to != nullptr, G.guard, G.st));
 }
 
 // V-cycle (cycle_type 0) or W-cycle (1) at level l; returns the buffer with x.
-static void* cycle(Gmg& G, int l, const void* rhs) {
+// started: the first pre-smoothing step from zero is done (zero_start_of).
+static void* cycle(Gmg& G, int l, const void* rhs, bool started) {
   Level& L = G.lv[l];
-  const int64_t n = L.g.ndof;
   const DType t = G.cyc;
   if (l == G.L - 1) {
     solve_coarsest(G, rhs, L.x[0].p);
     return L.x[0].p;
   }
   const int rsel = (t == F32) ? G.prec[l] : F64;  // residual operator precision
-  void* x = smooth(G, l, rhs, nullptr);
+  void* x = smooth_from(G, l, rhs, nullptr, started);
   {
     EpiArgs ea;
     ea.y = L.res.p;
     ea.b = rhs;
     level_op(G, l, t, rsel, EPI_RESID, x, ea);
   }
+  // without a line search the correction goes straight into x
+  const bool plain = G.o.coarse_correction_policy == 0;
   const bool enrich = (l == 0 && G.o.root_enrichment_mode != 0 && G.L > 1);
   if (G.o.cycle_type == 0) {
-    coarse_visit(G, l, L.res.p, false);
-    coarse_correction(G, l, x, L.res.p, L.c.p, enrich ? L.res2.p : nullptr);
-    if (enrich) {
-      enrichment_rhs(G, L.res2.p, G.lv[1].rhs.p);
-      coarse_visit(G, l, nullptr, true);
-      coarse_correction(G, l, x, L.res2.p, L.c.p, nullptr);
+    if (plain && !enrich) {
+      coarse_visit(G, l, L.res.p, false, x);
+    } else {
+      coarse_visit(G, l, L.res.p, false);
+      coarse_correction(G, l, x, L.res.p, L.c.p, enrich ? L.res2.p : nullptr);
+      if (enrich) {
+        enrichment_rhs(G, L.res2.p, G.lv[1].rhs.p);
+        coarse_visit(G, l, nullptr, true);
+        coarse_correction(G, l, x, L.res2.p, L.c.p, nullptr);
+      }
     }
   } else {
-    coarse_visit(G, l, L.res.p, false);
-    if (G.o.coarse_correction_policy == 0) {
-      SF_CUDA(launch_axpby(t, n, 1.0, x, 1.0, L.c.p, x, G.guard, G.st));
+    if (plain) {
+      coarse_visit(G, l, L.res.p, false, x);
       EpiArgs ea;
       ea.y = L.res2.p;
       ea.b = rhs;
       level_op(G, l, t, rsel, EPI_RESID, x, ea);
     } else {
+      coarse_visit(G, l, L.res.p, false);
       coarse_correction(G, l, x, L.res.p, L.c.p, L.res2.p);
     }
     if (enrich) {
       enrichment_rhs(G, L.res2.p, G.lv[1].rhs.p);
       coarse_visit(G, l, nullptr, true);
+      coarse_correction(G, l, x, L.res2.p, L.c.p, nullptr);
+    } else if (plain) {
+      coarse_visit(G, l, L.res2.p, false, x);
     } else {
       coarse_visit(G, l, L.res2.p, false);
+      coarse_correction(G, l, x, L.res2.p, L.c.p, nullptr);
     }
-    coarse_correction(G, l, x, L.res2.p, L.c.p, nullptr);
   }
   x = smooth(G, l, rhs, x);
   if (l == 0 && G.high) x = smooth(G, l, rhs, x);
@@ -874,8 +930,8 @@ static int kernel_nodes(cudaGraph_t graph) {
 // FP64 cycle): run directly, or captured once per setup and guard pointer on a
 // private stream and replayed on the hierarchy's stream (Gmg::CycleGraph).
 // Replays run the identical kernels with identical arguments.
-static void* run_cycle(Gmg& G, const void* in) {
-  if (!G.o.use_graphs || G.graphs_off) return cycle(G, 0, in);
+static void* run_cycle(Gmg& G, const void* in, bool started) {
+  if (!G.o.use_graphs || G.graphs_off) return cycle(G, 0, in, started);
   Gmg::CycleGraph* cg = nullptr;
   for (Gmg::CycleGraph& c : G.graphs)
     if (c.guard == G.guard) cg = &c;
@@ -895,7 +951,7 @@ static void* run_cycle(Gmg& G, const void* in) {
     ++G.graph_replays;
     return cg->out;
   }
-  if (cg->direct++ == 0) return cycle(G, 0, in);  // first cycle after a setup: direct
+  if (cg->direct++ == 0) return cycle(G, 0, in, started);  // first cycle after a setup: direct
   if (!G.cap_stream) SF_CUDA(cudaStreamCreateWithFlags(&G.cap_stream, cudaStreamNonBlocking));
   cudaStream_t user = G.st;
   cudaGraph_t graph = nullptr;
@@ -904,7 +960,7 @@ static void* run_cycle(Gmg& G, const void* in) {
   if (ok) {
     G.st = G.cap_stream;
     try {
-      out = cycle(G, 0, in);
+      out = cycle(G, 0, in, started);
     } catch (...) {  // the stream must leave capture mode before anything is reported
       ok = false;
     }
@@ -931,7 +987,7 @@ static void* run_cycle(Gmg& G, const void* in) {
   cudaGetLastError();  // a refused capture leaves its error here; the cycle then runs directly
   if (!ok) {
     G.graphs_off = true;
-    return cycle(G, 0, in);
+    return cycle(G, 0, in, started);
   }
   cg->launches = nk;
   cg->out = out;
@@ -946,16 +1002,17 @@ static void* run_cycle(Gmg& G, const void* in) {
 static void base_cycle(Gmg& G, const double* rhs, double* out) {
   const int64_t n = G.nfull();
   if (G.cyc == F32) {
-    SF_CUDA(launch_convert(F64, F32, rhs, G.cyc_in.p, n, G.guard, G.st));
-    void* r = run_cycle(G, G.cyc_in.p);
+    const ZeroStart zs = zero_start_of(G, 0);
+    SF_CUDA(launch_convert_start(n, rhs, G.cyc_in.as<float>(), zs, G.guard, G.st));
+    void* r = run_cycle(G, G.cyc_in.p, zs.mode != 0);
     SF_CUDA(launch_convert(F32, F64, r, out, n, G.guard, G.st));
   } else if (G.o.use_graphs && !G.graphs_off) {
     // a captured cycle reads a fixed input buffer
     SF_CUDA(launch_copy(F64, n, rhs, G.rhs64.p, G.guard, G.st));
-    void* r = run_cycle(G, G.rhs64.p);
+    void* r = run_cycle(G, G.rhs64.p, false);
     SF_CUDA(launch_copy(F64, n, r, out, G.guard, G.st));
   } else {
-    void* r = cycle(G, 0, rhs);
+    void* r = cycle(G, 0, rhs, false);
     SF_CUDA(launch_copy(F64, n, r, out, G.guard, G.st));
   }
 }

@@ -41,6 +41,16 @@ struct EpiArgs {
   const int* guard = nullptr;  // kernel body runs only when guard is null or *guard != 0
 };
 
+// The first smoothing step of a level from a zero start, formed by the kernel that
+// produces its right-hand side (mode 0: not requested, 1 Jacobi, 2 Chebyshev).
+struct ZeroStart {
+  int mode = 0;
+  double s = 0.0;
+  const void* dinv = nullptr;
+  void* d = nullptr;
+  void* x = nullptr;
+};
+
 struct Grid {
   int nx = 0, ny = 0, nz = 0;  // elements
   int64_t nn = 0;              // nodes
@@ -155,10 +165,15 @@ cudaError_t launch_stencil_diag(const Grid& g, const double* coef, const uint8_t
                                 double* dinv, cudaStream_t s);
 cudaError_t launch_restrict(DType t, const Grid& gf, const Grid& gc, const double* wx,
                             const double* wy, const double* wz, const uint8_t* mask_c,
-                            const void* fine, void* coarse, const int* guard, cudaStream_t s);
+                            const void* fine, void* coarse, const int* guard, cudaStream_t s,
+                            const ZeroStart& zs = ZeroStart());
+// add: fine += P coarse, else fine = P coarse
 cudaError_t launch_prolong(DType t, const Grid& gf, const Grid& gc, const double* wx,
                            const double* wy, const double* wz, const uint8_t* mask_f,
-                           const void* coarse, void* fine, const int* guard, cudaStream_t s);
+                           const void* coarse, void* fine, bool add, const int* guard, cudaStream_t s);
+// dst = (float)src, and the level's zero start on it
+cudaError_t launch_convert_start(int64_t n, const double* src, float* dst, const ZeroStart& zs, const int* guard,
+                                 cudaStream_t s);
 cudaError_t launch_stencil_to_dense(const Grid& g, const double* coef, const int32_t* dense_idx,
                                     int64_t n, double* A, cudaStream_t s);
 cudaError_t launch_convert(DType from, DType to, const void* src, void* dst, int64_t n,
@@ -184,10 +199,12 @@ cudaError_t launch_expand(DType t, int64_t n_free, const int32_t* free_idx, cons
                           void* dst_full, cudaStream_t s);
 cudaError_t launch_compress(DType t, int64_t n_free, const int32_t* free_idx,
                             const void* src_full, void* dst_free, cudaStream_t s);
-cudaError_t launch_gather_idx(int64_t n, const int32_t* idx, const double* src, double* dst,
+// dst[i] = src[idx[i]] (src of type t), and dst[i] = idx[i] >= 0 ? src[idx[i]] : 0
+// (dst of type t)
+cudaError_t launch_gather_idx(DType t, int64_t n, const int32_t* idx, const void* src, double* dst,
                               const int* guard, cudaStream_t s);
-cudaError_t launch_scatter_idx(int64_t n, const int32_t* idx, const double* src, double* dst,
-                               const int* guard, cudaStream_t s);
+cudaError_t launch_place_idx(DType t, int64_t n, const int32_t* idx, const double* src, void* dst,
+                             const int* guard, cudaStream_t s);
 cudaError_t launch_vec_op(int64_t n, int op, const double* a, const double* b, const uint8_t* mask,
                           double s, const double* s_dev, double* out, cudaStream_t st);
 cudaError_t launch_enrich_weights(int64_t n, const double* diag, const uint8_t* mask,

@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kRedThreads) minmax_kernel(int64_t n, const do
   __shared__ double sh[32 * 3];
   double v[3] = {INFINITY, -INFINITY, 0.0};
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const double e = E[i];
     v[0] = fmin(v[0], e);
@@ -188,14 +189,37 @@ __global__ void __launch_bounds__(kRedThreads) minmax_kernel(int64_t n, const do
     is_last = atomicAdd(w.ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (is_last && threadIdx.x == 0) {
-    __threadfence();
+  if (!is_last) return;
+  // the last block: its warps reduce the blocks' partials (counts are whole numbers,
+  // so their order does not matter)
+  __threadfence();
+  volatile double* p = w.partials;
+  v[0] = INFINITY;
+  v[1] = -INFINITY;
+  v[2] = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+    v[0] = fmin(v[0], p[k]);
+    v[1] = fmax(v[1], p[kRedBlocks + k]);
+    v[2] += p[2 * kRedBlocks + k];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v[0] = fmin(v[0], __shfl_down_sync(0xffffffffu, v[0], o));
+    v[1] = fmax(v[1], __shfl_down_sync(0xffffffffu, v[1], o));
+    v[2] += __shfl_down_sync(0xffffffffu, v[2], o);
+  }
+  if (lane == 0) {
+    sh[wid] = v[0];
+    sh[32 + wid] = v[1];
+    sh[64 + wid] = v[2];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
     double a = INFINITY, b = -INFINITY, c = 0.0;
-    volatile double* p = w.partials;
-    for (int k = 0; k < (int)gridDim.x; ++k) {
-      a = fmin(a, p[k]);
-      b = fmax(b, p[kRedBlocks + k]);
-      c += p[2 * kRedBlocks + k];
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+      a = fmin(a, sh[k]);
+      b = fmax(b, sh[32 + k]);
+      c += sh[64 + k];
     }
     out[0] = a;
     out[1] = b;
@@ -364,27 +388,33 @@ cudaError_t launch_compress(DType t, int64_t n_free, const int32_t* free_idx,
   return sf_launched(1);
 }
 
-__global__ void gather_idx_kernel(int64_t n, const int32_t* __restrict__ idx, const double* __restrict__ src,
+template <typename T>
+__global__ void gather_idx_kernel(int64_t n, const int32_t* __restrict__ idx, const T* __restrict__ src,
                                   double* __restrict__ dst, const int* guard) {
   if (guard_off(guard)) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = src[idx[i]];
+  if (i < n) dst[i] = (double)src[idx[i]];
 }
-__global__ void scatter_idx_kernel(int64_t n, const int32_t* __restrict__ idx, const double* __restrict__ src,
-                                   double* __restrict__ dst, const int* guard) {
+template <typename T>
+__global__ void place_idx_kernel(int64_t n, const int32_t* __restrict__ idx, const double* __restrict__ src,
+                                 T* __restrict__ dst, const int* guard) {
   if (guard_off(guard)) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[idx[i]] = src[i];
+  if (i >= n) return;
+  const int32_t k = idx[i];
+  dst[i] = k >= 0 ? (T)src[k] : T(0);
 }
 
-cudaError_t launch_gather_idx(int64_t n, const int32_t* idx, const double* src, double* dst,
+cudaError_t launch_gather_idx(DType t, int64_t n, const int32_t* idx, const void* src, double* dst,
                               const int* guard, cudaStream_t s) {
-  gather_idx_kernel<<<div_up(n, 256), 256, 0, s>>>(n, idx, src, dst, guard);
+  if (t == F64) gather_idx_kernel<double><<<div_up(n, 256), 256, 0, s>>>(n, idx, (const double*)src, dst, guard);
+  else gather_idx_kernel<float><<<div_up(n, 256), 256, 0, s>>>(n, idx, (const float*)src, dst, guard);
   return sf_launched(1);
 }
-cudaError_t launch_scatter_idx(int64_t n, const int32_t* idx, const double* src, double* dst,
-                               const int* guard, cudaStream_t s) {
-  scatter_idx_kernel<<<div_up(n, 256), 256, 0, s>>>(n, idx, src, dst, guard);
+cudaError_t launch_place_idx(DType t, int64_t n, const int32_t* idx, const double* src, void* dst,
+                             const int* guard, cudaStream_t s) {
+  if (t == F64) place_idx_kernel<double><<<div_up(n, 256), 256, 0, s>>>(n, idx, src, (double*)dst, guard);
+  else place_idx_kernel<float><<<div_up(n, 256), 256, 0, s>>>(n, idx, src, (float*)dst, guard);
   return sf_launched(1);
 }
 

@@ -106,7 +106,7 @@ void prolong_to(Gmg& G, int l, const void* coarse, void* fine) {
   Level& L = G.lv[l];
   Level& C = G.lv[l + 1];
   SF_CUDA(launch_prolong(G.cyc, L.g, C.g, L.wx.as<double>(), L.wy.as<double>(), L.wz.as<double>(),
-                         L.mask.as<uint8_t>(), coarse, fine, nullptr, G.st));
+                         L.mask.as<uint8_t>(), coarse, fine, false, nullptr, G.st));
 }
 
 // residual rhs - K_l x into out, with the operator precision of the cycle's residual
