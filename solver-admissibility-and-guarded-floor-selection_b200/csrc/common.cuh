@@ -143,6 +143,25 @@ __device__ __forceinline__ void zero_start(const ZeroStart& z, int64_t i, T r) {
   }
 }
 
+// v[0] + v[1] + ... + v[n - 1] (shared memory, 16-byte aligned, zeros from n to a
+// multiple of sixteen) added one by one; sixteen values are loaded together, so the
+// chain waits for additions only (a zero added at its end changes nothing).
+__device__ __forceinline__ double ordered_sum(const double* v, int n) {
+  double s = 0.0;
+#pragma unroll 1
+  for (int b = 0; b < n; b += 16) {
+    double2 c[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = reinterpret_cast<const double2*>(v + b)[q];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      s += c[q].x;
+      s += c[q].y;
+    }
+  }
+  return s;
+}
+
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 }  // namespace simpfem

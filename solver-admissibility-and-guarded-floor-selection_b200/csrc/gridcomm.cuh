@@ -100,9 +100,9 @@ __device__ __forceinline__ bool grid_allreduce_warp(ulonglong2* slots, unsigned 
 // Sum of nparts numbered parts, added one by one in their order, as a kernel with one
 // part a block and one thread for the sum adds them.  The caller has put its parts
 // into half + number; every lane holds the sum on return.  stage: shared memory of
-// kGridParts doubles.
+// kGridParts doubles, 16-byte aligned.
 constexpr int kGridParts = 2 * kGridMaxBlocks;
-static_assert(kGridParts + kGridCopies <= kGridMaxVals * kGridSlots, "slots");
+static_assert(kGridParts + kGridCopies <= kGridMaxVals * kGridSlots && kGridParts % 16 == 0, "slots");
 
 __device__ __forceinline__ bool grid_sum_parts_warp(ulonglong2* half, unsigned epoch, int nparts, double* stage,
                                                     double& v) {
@@ -122,9 +122,7 @@ __device__ __forceinline__ bool grid_sum_parts_warp(ulonglong2* half, unsigned e
       all = __all_sync(0xffffffffu, ok);
     }
     __syncwarp();
-    double s = 0.0;
-#pragma unroll 8
-    for (int b = 0; b < nparts; ++b) s += stage[b];
+    const double s = ordered_sum(stage, nparts);
     __syncwarp();
     v = s;
     if (all && nb > kGridFlat && lane < kGridCopies) grid_put(half + kGridParts + lane, s, epoch);

@@ -48,7 +48,8 @@ __device__ __forceinline__ void block_sum(double (&v)[ND], double* sh /*32*ND*/)
 template <int ND>
 __device__ __forceinline__ bool last_block_finalize(const double (&v)[ND], RedWork w, double* out) {
   __shared__ bool is_last;
-  __shared__ double stage[4 * kRedBlocks];
+  constexpr int kStage = (kRedBlocks + 15) / 16 * 16;  // partials of a value, zeros behind them
+  __shared__ __align__(16) double stage[ND * kStage];
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < ND; ++k) w.partials[k * kRedBlocks + blockIdx.x] = v[k];
@@ -60,16 +61,14 @@ __device__ __forceinline__ bool last_block_finalize(const double (&v)[ND], RedWo
   if (!is_last) return false;
   __threadfence();
   const int nb = (int)gridDim.x;
-  for (int e = threadIdx.x; e < ND * nb; e += blockDim.x) {
-    const int k = e / nb, b = e - k * nb;
-    stage[k * kRedBlocks + b] = ((volatile double*)w.partials)[k * kRedBlocks + b];
+  for (int e = threadIdx.x; e < ND * kStage; e += blockDim.x) {
+    const int k = e / kStage, b = e - k * kStage;
+    stage[e] = b < nb ? ((volatile double*)w.partials)[k * kRedBlocks + b] : 0.0;
   }
   __syncthreads();
   if (threadIdx.x < ND) {
     const int k = threadIdx.x;
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += stage[k * kRedBlocks + b];
-    out[k] = s;
+    out[k] = ordered_sum(stage + k * kStage, nb);
   }
   if (threadIdx.x == 0) *w.ticket = 0u;
   return true;
@@ -815,7 +814,8 @@ __global__ void __launch_bounds__(kColThreads, 1)
                    ulonglong2* slots, unsigned* last) {
   if (!k.flags[F_CYC]) return;
   extern __shared__ __align__(16) double csm[];  // WSMEM: w [per][threads]; else two vectors [2][MP * PER][threads]
-  __shared__ double red[MP * kColThreads / 32], stage[kGridParts];
+  __shared__ double red[MP * kColThreads / 32];
+  __shared__ __align__(16) double stage[kGridParts];
   __shared__ double total;
   __shared__ int good;
   constexpr int NE = MP * PER;  // elements a thread

@@ -52,6 +52,14 @@ struct FastDiv {
     return (unsigned)(((uint64_t)__umulhi(n, mul) + n) >> shift);
   }
 };
+// node_ijk by multiplications; dz, dy divide by nz + 1 and ny + 1
+__device__ __forceinline__ void node_ijk(const Grid& g, const FastDiv& dz, const FastDiv& dy, int n, int& i, int& j,
+                                         int& k) {
+  const int jq = (int)dz.div(n);
+  k = n - jq * (g.nz + 1);
+  i = (int)dy.div(jq);
+  j = jq - i * (g.ny + 1);
+}
 
 // 32 nodes a block, nine warps: warp col = 3 ox + oy loads what couples its 32 nodes'
 // rows to their three z-neighbours in column (ox, oy) -- 27 coefficients and nine
@@ -334,54 +342,75 @@ cudaError_t launch_stencil_col_bf16(Epi epi, const Grid& g, const __nv_bfloat16*
 // Q_stu = P24(stu)^T KE P24(stu), child clamped to the fine grid exactly as
 // gpu_fem/multigrid_v4.py:285-289 does.  Q is given in corner-major order
 // Q[stu][(a * 3 + r) * 24 + b * 3 + q] with a, b coarse-element corners.
-__global__ void level1_assemble_kernel(Grid gc, Grid gf, const double* __restrict__ E,
-                                       const double* __restrict__ Q, const uint8_t* __restrict__ mask,
-                                       double* __restrict__ coef) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 27 * gc.nn) return;
-  const int o = (int)(idx / gc.nn);
-  const int64_t n = idx - (int64_t)o * gc.nn;
+//
+// A block makes one offset o of 128 coarse nodes.  A thread per (node, offset) with nine
+// loads of Q from L1 for nine products and 64-bit divisions for the node's position took
+// 151 us at 69,741 nodes (their 321 M FP64 products take 17); with the block's part of Q
+// in shared memory and an element's eight moduli in flight together 94 (two nodes a
+// thread, sharing the loads of Q: 108, for the registers).
+constexpr int kL1Threads = 128;
+
+__global__ void __launch_bounds__(kL1Threads) level1_assemble_kernel(Grid gc, Grid gf, FastDiv dz, FastDiv dy,
+                                                                     const double* __restrict__ E,
+                                                                     const double* __restrict__ Q,
+                                                                     const uint8_t* __restrict__ mask,
+                                                                     double* __restrict__ coef) {
+  __shared__ __align__(16) double q[8 * 8 * 10];  // [a][stu][3 x 3, padded], corners a with node + o in the element
+  const int o = blockIdx.y, ox = o / 9 - 1, oy = (o / 3) % 3 - 1, oz = o % 3 - 1;
+  for (int e = threadIdx.x; e < 8 * 8 * 10; e += kL1Threads) {
+    const int a = e / 80, stu = e / 10 % 8, r = e % 10;
+    const int bx = (a >> 2) + ox, by = ((a >> 1) & 1) + oy, bz = (a & 1) + oz;
+    const bool in = r < 9 && bx >= 0 && bx <= 1 && by >= 0 && by <= 1 && bz >= 0 && bz <= 1;
+    q[(a * 8 + stu) * 10 + r] =
+        in ? Q[(int64_t)stu * 576 + (a * 3 + r / 3) * 24 + (bx * 4 + by * 2 + bz) * 3 + r % 3] : 0.0;
+  }
+  __syncthreads();
+  const int64_t n = (int64_t)blockIdx.x * kL1Threads + threadIdx.x;
+  if (n >= gc.nn) return;
   int i, j, k;
-  node_ijk(gc, n, i, j, k);
-  const int ox = o / 9 - 1, oy = (o / 3) % 3 - 1, oz = o % 3 - 1;
+  node_ijk(gc, dz, dy, (int)n, i, j, k);
   const int mi = i + ox, mj = j + oy, mk = k + oz;
+  const bool ok = mi >= 0 && mj >= 0 && mk >= 0 && mi <= gc.nx && mj <= gc.ny && mk <= gc.nz;
   double blk[9];
 #pragma unroll
   for (int r = 0; r < 9; ++r) blk[r] = 0.0;
-  const bool nb_ok = mi >= 0 && mj >= 0 && mk >= 0 && mi <= gc.nx && mj <= gc.ny && mk <= gc.nz;
-  if (nb_ok) {
-    for (int a = 0; a < 8; ++a) {
-      const int ax = a >> 2, ay = (a >> 1) & 1, az = a & 1;
-      const int bx = ax + ox, by = ay + oy, bz = az + oz;
-      if (bx < 0 || bx > 1 || by < 0 || by > 1 || bz < 0 || bz > 1) continue;
-      const int ci = i - ax, cj = j - ay, ck = k - az;
-      if (ci < 0 || cj < 0 || ck < 0 || ci >= gc.nx || cj >= gc.ny || ck >= gc.nz) continue;
-      const int b = bx * 4 + by * 2 + bz;
-      double elem[9];
+  for (int a = 0; a < 8 && ok; ++a) {
+    const int ax = a >> 2, ay = (a >> 1) & 1, az = a & 1;
+    const int bx = ax + ox, by = ay + oy, bz = az + oz;
+    if (bx < 0 || bx > 1 || by < 0 || by > 1 || bz < 0 || bz > 1) continue;
+    const int ci = i - ax, cj = j - ay, ck = k - az;
+    if (ci < 0 || cj < 0 || ck < 0 || ci >= gc.nx || cj >= gc.ny || ck >= gc.nz) continue;
+    double Ee[8], elem[9];
 #pragma unroll
-      for (int r = 0; r < 9; ++r) elem[r] = 0.0;
-      for (int stu = 0; stu < 8; ++stu) {
-        const int s_ = stu >> 2, t_ = (stu >> 1) & 1, u_ = stu & 1;
-        const int fi = min(2 * ci + s_, gf.nx - 1);
-        const int fj = min(2 * cj + t_, gf.ny - 1);
-        const int fk = min(2 * ck + u_, gf.nz - 1);
-        const double Ee = E[((int64_t)fi * gf.ny + fj) * gf.nz + fk];
-        const double* q = Q + (int64_t)stu * 576;
+    for (int stu = 0; stu < 8; ++stu) {
+      const int fi = min(2 * ci + (stu >> 2), gf.nx - 1);
+      const int fj = min(2 * cj + ((stu >> 1) & 1), gf.ny - 1);
+      const int fk = min(2 * ck + (stu & 1), gf.nz - 1);
+      Ee[stu] = E[((int64_t)fi * gf.ny + fj) * gf.nz + fk];
+    }
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 9; ++r) elem[r] = 0.0;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) elem[r * 3 + c] += Ee * q[(a * 3 + r) * 24 + b * 3 + c];
+    for (int stu = 0; stu < 8; ++stu) {
+      double qv[10];
+#pragma unroll
+      for (int r = 0; r < 10; r += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(q + (a * 8 + stu) * 10 + r);
+        qv[r] = v.x;
+        qv[r + 1] = v.y;
       }
 #pragma unroll
-      for (int r = 0; r < 9; ++r) blk[r] += elem[r];
+      for (int r = 0; r < 9; ++r) elem[r] = fma(Ee[stu], qv[r], elem[r]);
     }
+#pragma unroll
+    for (int r = 0; r < 9; ++r) blk[r] += elem[r];
   }
-  const int64_t m = nb_ok ? node_id(gc, mi, mj, mk) : 0;
+  const int64_t m = ok ? node_id(gc, mi, mj, mk) : 0;
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const bool keep = nb_ok && mask[3 * n + r] && mask[3 * m + c];
+      const bool keep = ok && mask[3 * n + r] && mask[3 * m + c];
       coef[((int64_t)o * 9 + r * 3 + c) * gc.nn + n] = keep ? blk[r * 3 + c] : 0.0;
     }
 }
@@ -389,7 +418,10 @@ __global__ void level1_assemble_kernel(Grid gc, Grid gf, const double* __restric
 cudaError_t launch_level1_assemble(const Grid& gc, const Grid& gf, const double* E_fine,
                                    const double* Q, const uint8_t* mask_c, double* coef,
                                    cudaStream_t s) {
-  level1_assemble_kernel<<<div_up(27 * gc.nn, 128), 128, 0, s>>>(gc, gf, E_fine, Q, mask_c, coef);
+  if (gc.nn >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
+  const FastDiv dz = FastDiv::make(gc.nz + 1), dy = FastDiv::make(gc.ny + 1);
+  level1_assemble_kernel<<<dim3(div_up(gc.nn, kL1Threads), 27), kL1Threads, 0, s>>>(gc, gf, dz, dy, E_fine, Q, mask_c,
+                                                                                    coef);
   return sf_launched(1);
 }
 
@@ -404,94 +436,113 @@ __device__ __forceinline__ double w1(const double* w, int f, int c) {
 // K_c = R K_f P on stencils (Galerkin triple product of the reference's RAP loop).
 // Coarse block (n, M = n + o) = sum over fine nodes f in the support of n and
 // fine neighbours g = f + d of f in the support of M of
-// P[f, n] K_f[f, g] P[g, M].  The trilinear weights factor per axis, so each
-// axis contributes a list of at most 7 valid (f, d) pairs with weight
-// w(f, I) w(g, I + m) (m the axis component of o), and the sum runs over the
-// product of the three lists: only non-zero terms, no per-term bounds checks
-// or weight lookups (the thread is otherwise bound by that scan of 27 x 27
-// candidate pairs).
-struct RapAxis {
-  double w[7];
-  int64_t off[7];  // fine-node offset (f - 2I) * node stride + d * stencil-block stride
-  int cnt;
-};
+// P[f, n] K_f[f, g] P[g, M].  The trilinear weights factor per axis: with f = 2 I + a - 1
+// and g = f + d - 1 (a, d = 0..2), g supports I + m where a + d is 0 or 1 for m = -1, 1
+// to 3 for m = 0 and 3 or 4 for m = 1, and the sum runs over the product of the axes'
+// pairs, x outermost, in ascending (a, d).
+//
+// One thread per coarse node, entry r of the 3 x 3 block and (mx, my), all three mz: a
+// warp is 32 nodes along z, the nine warps of a block the nine (mx, my) of one entry,
+// whose fine coefficients (126 KB) its L1 holds.  An x pair's y pairs are straight-line
+// code (MY), nine loads each that the three mz share.  A thread per block with all
+// nine entries chained up to 343 x 9 loads: 140 us each for the 1,386 and the 168
+// coarse nodes of 80 x 40 x 20 (two levels), 241 for the two of 160 x 80 x 40, 341 of
+// 200 x 100 x 50; now 23, 98 and 179.  Two blocks per SM at 96 registers spill 56 bytes
+// and are faster than one at 134 (122 and 228).
+__host__ __device__ constexpr bool rap_pair(int a, int d, int m) {
+  return m < 0 ? a + d <= 1 : (m > 0 ? a + d >= 3 : a + d >= 1 && a + d <= 3);
+}
+// w(f, I) w(g, I + m) of pair (a, d); zero where a node is missing
+__device__ __forceinline__ double rap_weight(const double* __restrict__ w, int I, int m, int nf, int nc, int a, int d) {
+  const int f = 2 * I + a - 1, gg = f + d - 1, c = I + m;
+  if (f < 0 || f > nf || gg < 0 || gg > nf || c < 0 || c > nc) return 0.0;
+  return w[3 * f + a] * w1(w, gg, c);
+}
 
-__device__ __forceinline__ void rap_axis(RapAxis& ax, const double* __restrict__ w, int I, int m, int nf,
-                                         int64_t node_stride, int64_t blk_stride) {
-  ax.cnt = 0;
+// base: entry r of the fine node (2I, 2J, 2K), stencil block of offset (0, 0, 0);
+// block (dx, dy, dz) lies (dx * 9 + dy * 3 + dz) * 9 * nn further
+template <int MY>
+__device__ __forceinline__ void rap_sum(const Grid& gf, const Grid& gc, const double* __restrict__ base,
+                                        const double* __restrict__ wx, const double* __restrict__ wy,
+                                        const double* __restrict__ wz, int I, int J, int K, int mx, double (&acc)[3]) {
+  const int64_t nn = gf.nn, ys = gf.nz + 1, xs = (gf.ny + 1) * ys;
+  double pz[3][3][3], py[3][3];  // [m + 1][a][d], [a][d]; entries outside rap_pair are not used
+  bool fz[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const int f = 2 * I + a - 1;
-    if (f < 0 || f > nf) continue;
-    const double wf = w1(w, f, I);
-    if (wf == 0.0) continue;
+    fz[a] = 2 * K + a - 1 >= 0 && 2 * K + a - 1 <= gf.nz;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const int gg = f + d - 1;
-      if (gg < 0 || gg > nf) continue;
-      const double wg = w1(w, gg, I + m);
-      if (wg == 0.0) continue;
-      ax.w[ax.cnt] = wf * wg;
-      ax.off[ax.cnt] = (int64_t)(a - 1) * node_stride + (int64_t)d * blk_stride;
-      ++ax.cnt;
+      if (rap_pair(a, d, MY)) py[a][d] = rap_weight(wy, J, MY, gf.ny, gc.ny, a, d);
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+        if (rap_pair(a, d, m - 1)) pz[m][a][d] = rap_weight(wz, K, m - 1, gf.nz, gc.nz, a, d);
     }
+  }
+  for (int ex = 0; ex < 9; ++ex) {
+    const int ax = ex / 3, dx = ex % 3;
+    if (!rap_pair(ax, dx, mx)) continue;
+    const double px = rap_weight(wx, I, mx, gf.nx, gc.nx, ax, dx);
+    if (px == 0.0) continue;
+    const double* bx = base + (ax - 1) * xs + dx * 81 * nn;
+#pragma unroll
+    for (int ay = 0; ay < 3; ++ay)
+#pragma unroll
+      for (int dy = 0; dy < 3; ++dy)
+        if (rap_pair(ay, dy, MY)) {
+          const double pxy = px * py[ay][dy];
+          const double* bxy = bx + (ay - 1) * ys + dy * 27 * nn;
+          double v[3][3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) v[a][d] = fz[a] && pxy != 0.0 ? bxy[d * 9 * nn + a - 1] : 0.0;
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const double pv = pxy * v[a][d];  // exact: the weights are powers of two
+#pragma unroll
+              for (int m = 0; m < 3; ++m)
+                if (rap_pair(a, d, m - 1)) acc[m] = fma(pz[m][a][d], pv, acc[m]);
+            }
+        }
   }
 }
 
-__global__ void rap_kernel(Grid gf, Grid gc, const double* __restrict__ cf, const uint8_t* __restrict__ mask_c,
-                           const double* __restrict__ wx, const double* __restrict__ wy,
-                           const double* __restrict__ wz, double* __restrict__ cc) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 27 * gc.nn) return;
-  const int o = (int)(idx / gc.nn);
-  const int64_t n = idx - (int64_t)o * gc.nn;
+__global__ void __launch_bounds__(288, 2) rap_kernel(Grid gf, Grid gc, FastDiv dz, FastDiv dy,
+                                                     const double* __restrict__ cf,
+                                                     const uint8_t* __restrict__ mask_c,
+                                                     const double* __restrict__ wx, const double* __restrict__ wy,
+                                                     const double* __restrict__ wz, double* __restrict__ cc) {
+  const int64_t n = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+  if (n >= gc.nn) return;
+  const int r = blockIdx.y, warp = threadIdx.x >> 5, mx = warp / 3 - 1, my = warp % 3 - 1;
   int I, J, K;
-  node_ijk(gc, n, I, J, K);
-  const int mx = o / 9 - 1, my = (o / 3) % 3 - 1, mz = o % 3 - 1;
-  const int MI = I + mx, MJ = J + my, MK = K + mz;
-  double blk[9];
-#pragma unroll
-  for (int r = 0; r < 9; ++r) blk[r] = 0.0;
-  const bool nb_ok = MI >= 0 && MJ >= 0 && MK >= 0 && MI <= gc.nx && MJ <= gc.ny && MK <= gc.nz;
-  if (nb_ok) {
-    const int64_t nn = gf.nn, NZ1 = gf.nz + 1, NY1 = gf.ny + 1;
-    // stencil block of offset (dx, dy, dz) starts at ((dx * 9 + dy * 3 + dz) * 9) * nn
-    RapAxis ax, ay, az;
-    rap_axis(ax, wx, I, mx, gf.nx, NY1 * NZ1, 81 * nn);
-    rap_axis(ay, wy, J, my, gf.ny, NZ1, 27 * nn);
-    rap_axis(az, wz, K, mz, gf.nz, 1, 9 * nn);
-    // index of the fine node (2I, 2J, 2K); every listed pair adds an offset that
-    // lands on a fine node inside the grid
-    const int64_t base = node_id(gf, 2 * I, 2 * J, 2 * K);
-    for (int ex = 0; ex < ax.cnt; ++ex) {
-      for (int ey = 0; ey < ay.cnt; ++ey) {
-        const double wxy = ax.w[ex] * ay.w[ey];
-        const int64_t bxy = base + ax.off[ex] + ay.off[ey];
-#pragma unroll
-        for (int ez = 0; ez < 7; ++ez) {
-          if (ez >= az.cnt) break;
-          const double pp = wxy * az.w[ez];
-          const double* src = cf + (bxy + az.off[ez]);
-#pragma unroll
-          for (int r = 0; r < 9; ++r) blk[r] += pp * src[(int64_t)r * nn];
-        }
-      }
-    }
+  node_ijk(gc, dz, dy, (int)n, I, J, K);
+  const bool col = I + mx >= 0 && I + mx <= gc.nx && J + my >= 0 && J + my <= gc.ny;
+  double acc[3] = {0.0, 0.0, 0.0};
+  if (col) {
+    const double* base = cf + r * gf.nn + node_id(gf, 2 * I, 2 * J, 2 * K);
+    if (my < 0) rap_sum<-1>(gf, gc, base, wx, wy, wz, I, J, K, mx, acc);
+    else if (my > 0) rap_sum<1>(gf, gc, base, wx, wy, wz, I, J, K, mx, acc);
+    else rap_sum<0>(gf, gc, base, wx, wy, wz, I, J, K, mx, acc);
   }
-  const int64_t m = nb_ok ? node_id(gc, MI, MJ, MK) : 0;
 #pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const bool keep = nb_ok && mask_c[3 * n + r] && mask_c[3 * m + c];
-      cc[((int64_t)o * 9 + r * 3 + c) * gc.nn + n] = keep ? blk[r * 3 + c] : 0.0;
-    }
+  for (int m = 0; m < 3; ++m) {
+    const int MK = K + m - 1;
+    bool keep = col && MK >= 0 && MK <= gc.nz;
+    if (keep) keep = mask_c[3 * n + r / 3] && mask_c[3 * node_id(gc, I + mx, J + my, MK) + r % 3];
+    cc[((int64_t)((mx + 1) * 9 + (my + 1) * 3 + m) * 9 + r) * gc.nn + n] = keep ? acc[m] : 0.0;
+  }
 }
 
 cudaError_t launch_rap(const Grid& gf, const Grid& gc, const double* coef_f, const uint8_t* mask_c,
                        const double* wx, const double* wy, const double* wz, double* coef_c,
                        cudaStream_t s) {
-  rap_kernel<<<div_up(27 * gc.nn, 128), 128, 0, s>>>(gf, gc, coef_f, mask_c, wx, wy, wz, coef_c);
+  if (gc.nn >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
+  const FastDiv dz = FastDiv::make(gc.nz + 1), dy = FastDiv::make(gc.ny + 1);
+  rap_kernel<<<dim3(div_up(gc.nn, 32), 9), 288, 0, s>>>(gf, gc, dz, dy, coef_f, mask_c, wx, wy, wz, coef_c);
   return sf_launched(1);
 }
 
