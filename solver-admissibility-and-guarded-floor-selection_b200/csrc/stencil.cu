@@ -346,7 +346,7 @@ cudaError_t launch_stencil_col_bf16(Epi epi, const Grid& g, const __nv_bfloat16*
 // A block makes one offset o of 128 coarse nodes.  A thread per (node, offset) with nine
 // loads of Q from L1 for nine products and 64-bit divisions for the node's position took
 // 151 us at 69,741 nodes (their 321 M FP64 products take 17); with the block's part of Q
-// in shared memory and an element's eight moduli in flight together 94 (two nodes a
+// in shared memory and an element's eight moduli in flight together 100 (two nodes a
 // thread, sharing the loads of Q: 108, for the registers).
 constexpr int kL1Threads = 128;
 
@@ -379,14 +379,15 @@ __global__ void __launch_bounds__(kL1Threads) level1_assemble_kernel(Grid gc, Gr
     const int bx = ax + ox, by = ay + oy, bz = az + oz;
     if (bx < 0 || bx > 1 || by < 0 || by > 1 || bz < 0 || bz > 1) continue;
     const int ci = i - ax, cj = j - ay, ck = k - az;
-    if (ci < 0 || cj < 0 || ck < 0 || ci >= gc.nx || cj >= gc.ny || ck >= gc.nz) continue;
+    // no branch around the loads: one corner's fly while the last one's products run
+    const bool in = ci >= 0 && cj >= 0 && ck >= 0 && ci < gc.nx && cj < gc.ny && ck < gc.nz;
     double Ee[8], elem[9];
 #pragma unroll
     for (int stu = 0; stu < 8; ++stu) {
       const int fi = min(2 * ci + (stu >> 2), gf.nx - 1);
       const int fj = min(2 * cj + ((stu >> 1) & 1), gf.ny - 1);
       const int fk = min(2 * ck + (stu & 1), gf.nz - 1);
-      Ee[stu] = E[((int64_t)fi * gf.ny + fj) * gf.nz + fk];
+      Ee[stu] = in ? E[((int64_t)fi * gf.ny + fj) * gf.nz + fk] : 0.0;
     }
 #pragma unroll
     for (int r = 0; r < 9; ++r) elem[r] = 0.0;
@@ -402,8 +403,10 @@ __global__ void __launch_bounds__(kL1Threads) level1_assemble_kernel(Grid gc, Gr
 #pragma unroll
       for (int r = 0; r < 9; ++r) elem[r] = fma(Ee[stu], qv[r], elem[r]);
     }
+    if (in) {
 #pragma unroll
-    for (int r = 0; r < 9; ++r) blk[r] += elem[r];
+      for (int r = 0; r < 9; ++r) blk[r] += elem[r];
+    }
   }
   const int64_t m = ok ? node_id(gc, mi, mj, mk) : 0;
 #pragma unroll
