@@ -115,6 +115,10 @@ class FloorProposerNet:
         if f.shape[0] != x.shape[0]:
             raise ValueError("x and feats must hold the same number of samples")
         n = x.shape[0]
+        if 0 < n <= self.max_batch:
+            p = torch.empty((n, 3), dtype=torch.float32, device="cuda")
+            _lib.call("simpfem_cnn_forward", self._h, _lib.ptr(x), _lib.ptr(f), n, _lib.ptr(p), _lib.stream_ptr())
+            return p
         probs = []
         for s in range(0, n, self.max_batch):
             e = min(n, s + self.max_batch)
@@ -133,8 +137,10 @@ class FloorProposerNet:
         y = _lib.as_cuda(labels, torch.int32).contiguous()
         if y.numel() != x.shape[0] or f.shape[0] != x.shape[0]:
             raise ValueError("x, feats and labels must hold the same number of samples")
-        if y.numel() and (int(y.min()) < 0 or int(y.max()) >= len(RUNGS)):
-            raise ValueError("labels must index the rungs 0..2")
+        if y.numel():
+            lo, hi = torch.stack(torch.aminmax(y)).tolist()
+            if lo < 0 or hi >= len(RUNGS):
+                raise ValueError("labels must index the rungs 0..2")
         loss = ctypes.c_float()
         g = np.empty(self.n_params, dtype=np.float32) if want_grad else None
         _lib.call("simpfem_cnn_loss_grad", self._h, _lib.ptr(x), _lib.ptr(f), _lib.ptr(y), int(x.shape[0]),
