@@ -219,6 +219,13 @@ static DType api_dtype(int dt) {
   throw InvalidArg{"unknown dtype"};
 }
 
+// The compact operator reads u and E while it writes y, so a y that shares memory with
+// either keeps the form that finishes reading first (expand, product, compress).
+static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb && y < x + na;
+}
+
 int simpfem_matvec(simpfem_mesh* mh, int dtype, const void* E, const void* u_free, void* y_free,
                    void* stream) {
   SF_API_BEGIN
@@ -227,7 +234,8 @@ int simpfem_matvec(simpfem_mesh* mh, int dtype, const void* E, const void* u_fre
   const DType t = api_dtype(dtype);
   if (t == BF16) throw InvalidArg{"simpfem_matvec: dtype must be F64 or F32"};
   const size_t es = t == F64 ? 8 : 4;
-  if (t == F64 && m.ninfo.p && u_free != y_free) {
+  if (t == F64 && m.ninfo.p && !overlap(y_free, es * m.n_free, u_free, es * m.n_free) &&
+      !overlap(y_free, es * m.n_free, E, es * m.g.ne())) {
     SF_CUDA(launch_fine_compact(m.g, m.sh[0], (const double*)E, m.ninfo.as<int32_t>(), m.pinfo.as<int32_t>(),
                                 (const double*)u_free, (double*)y_free, S(stream)));
     return SIMPFEM_OK;
