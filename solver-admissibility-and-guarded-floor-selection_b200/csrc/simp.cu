@@ -131,7 +131,14 @@ __global__ void __launch_bounds__(kFilterThreads) cone_filter_kernel(int nx, int
 // A tile holds whole rows along z up to 64 elements (else 32, so that the halo
 // stays a small share of a row) and is filled up along y and x to at most
 // kFilterThreads * kFilterPer outputs with y about as long as x: the halo of a
-// cube is the smallest.
+// cube is the smallest.  On a rod, which is filled along x alone, the halo is a
+// multiple of the outputs; there x is shortened until the tile fits.
+constexpr size_t kFilterSmem = 227 * 1024;
+size_t filter_smem(const FilterTile& f) {
+  const size_t nc = (size_t)(f.r + 1) * (f.r + 1), h = 2 * f.r;
+  return sizeof(double) * (nc * nc * nc + (f.tx + h) * (f.ty + h) * (f.tz + h)) + sizeof(int) * kMaxOff;
+}
+
 FilterTile filter_tile(int nx, int ny, int nz, int r) {
   FilterTile f;
   f.r = r;
@@ -141,6 +148,7 @@ FilterTile filter_tile(int nx, int ny, int nz, int r) {
   while ((side + 1) * (side + 1) <= plane) ++side;
   f.ty = std::min(ny, side);
   f.tx = std::min(nx, std::max(1, plane / f.ty));
+  while (f.tx > 1 && filter_smem(f) > kFilterSmem) f.tx = (f.tx + 1) / 2;
   f.bx = div_up(nx, f.tx);
   f.by = div_up(ny, f.ty);
   f.bz = div_up(nz, f.tz);
@@ -151,13 +159,10 @@ cudaError_t launch_filter(int nx, int ny, int nz, double rmin, int transpose, co
                           cudaStream_t s) {
   const int r = (int)floor(rmin);
   const FilterTile f = filter_tile(nx, ny, nz, r);
-  const int NC = (r + 1) * (r + 1);
-  const size_t smem = sizeof(double) * ((size_t)NC * NC * NC +
-                                        (size_t)(f.tx + 2 * r) * (f.ty + 2 * r) * (f.tz + 2 * r)) +
-                      sizeof(int) * kMaxOff;
+  const size_t smem = filter_smem(f);
   static std::atomic<uint64_t> attr_done;
   const cudaError_t e = once_per_device(attr_done, [] {
-    return cudaFuncSetAttribute(cone_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return cudaFuncSetAttribute(cone_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterSmem);
   });
   if (e != cudaSuccess) return e;
   cone_filter_kernel<<<f.bx * f.by * f.bz, kFilterThreads, smem, s>>>(nx, ny, nz, f, transpose, x, y);
