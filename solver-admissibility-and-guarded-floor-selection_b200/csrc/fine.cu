@@ -746,7 +746,7 @@ static size_t sweep_smem(const SweepShape& sh, int operands) {
 bool fine_shape_ok(DType t, const Grid& g, const SweepShape& sh) {
   const int NT = sh.bj * sh.bk;
   return sh.bk >= 2 && sh.bj >= 2 && sh.cx >= 1 && NT <= kSweepThreads &&
-         (sh.bj + 1) * 3 * (sh.bk + 1) <= kTileLoads * NT &&
+         (sh.bj + 1) * 3 * (sh.bk + 1) <= kTileLoads * NT && div_up(g.nx + 1, sh.cx) <= 65535 &&
          4 * (int64_t)(g.ny + 1) * (g.nz + 1) < (int64_t(1) << 31) &&
          (t == F64 ? sweep_smem<double>(sh, 3) : sweep_smem<float>(sh, 3)) <= 200 * 1024;
 }

@@ -226,11 +226,12 @@ static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
 // block (the halo column and the halo plane make each part one element larger).
 static std::vector<SweepShape> sweep_candidates(DType t, const Grid& g) {
   std::vector<SweepShape> out;
-  for (int parts = 1; parts <= 4; ++parts) {
+  // a block takes 63 of the nz + 1 nodes along z at most (two rows of 64 threads)
+  const int fewest = (int)div_up64(g.nz + 1, 63), most_parts = std::max(4, fewest + 1);
+  for (int parts = fewest; parts <= most_parts; ++parts) {
     SweepShape sh;
     sh.bk = (int)div_up64(g.nz + 1, parts) + 1;
     sh.bk = std::max(2, sh.bk);
-    if (sh.bk > 130) continue;
     for (int nt : {128, 96, 64}) {
       const int most = nt / sh.bk;
       if (most < 2) continue;
