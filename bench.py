@@ -572,7 +572,7 @@ def run_native(args):
         },
         "gpu_launches": int(launches),
         "roofline": {
-            "kernel": f"fine_sweep_x2_kernel<EPI_{'JAC' if args.stack == 'plain' else 'CHEB'}> (FP32 fused smoothing step, cold L2)",
+            "kernel": f"sweep_kernel<float, EPI_{'JAC' if args.stack == 'plain' else 'CHEB'}> (FP32 fused smoothing step, cold L2)",
             "bound": "hbm",
             "achieved": round(achieved, 1),
             "peak": hbm_peak,
@@ -584,7 +584,7 @@ def run_native(args):
             "avg_launch_us": round(avg.value * 1e3, 3),
         },
         "roofline_fp64_operator": {
-            "kernel": "fine_sweep_kernel<double, EPI_APPLY> (FP64 operator product, cold L2)",
+            "kernel": "sweep_kernel<double, EPI_APPLY> (FP64 operator product, cold L2)",
             "bound": "hbm",
             "achieved": round(op_bytes / (avg64.value * 1e-3) / 1e9, 1),
             "peak": hbm_peak,
