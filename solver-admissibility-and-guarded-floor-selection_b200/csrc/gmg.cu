@@ -224,7 +224,15 @@ static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
 // Candidate tiles of a grid: the z extent in one to four equal parts, blocks of up to
 // 256, 128 or 64 threads filled with equal parts of the y extent, cx node planes a
 // block (the halo column and the halo plane make each part one element larger).
-static std::vector<SweepShape> sweep_candidates(DType t, const Grid& g) {
+// Depths along x: a doubling series for the model to choose from; all of them, each
+// number of parts once, for the tuner (every), because the wave count hangs on it.
+static std::vector<SweepShape> sweep_candidates(DType t, const Grid& g, bool every) {
+  std::vector<int> depths = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
+  if (every) {
+    depths.clear();
+    for (int cx = 1; cx <= 32; ++cx)
+      if (cx == 1 || div_up(g.nx + 1, cx) != div_up(g.nx + 1, cx - 1)) depths.push_back(cx);
+  }
   std::vector<SweepShape> out;
   // a block takes 63 of the nz + 1 nodes along z at most (two rows of 64 threads)
   const int fewest = (int)div_up64(g.nz + 1, 63), most_parts = std::max(4, fewest + 1);
@@ -237,7 +245,7 @@ static std::vector<SweepShape> sweep_candidates(DType t, const Grid& g) {
       if (most < 2) continue;
       const int nb = (int)div_up64(g.ny + 1, most - 1);
       sh.bj = (int)div_up64(g.ny + 1, nb) + 1;
-      for (int cx : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {
+      for (int cx : depths) {
         sh.cx = cx;
         if (cx > 1 && cx >= 2 * (g.nx + 1)) continue;
         if (!fine_shape_ok(t, g, sh)) continue;
@@ -257,7 +265,7 @@ SweepShape default_shape(DType t, const Grid& g) {
   best.bk = 4;
   best.cx = 1;
   double best_cost = 1e300;
-  for (const SweepShape& sh : sweep_candidates(t, g)) {
+  for (const SweepShape& sh : sweep_candidates(t, g, false)) {
     const double cost = sweep_cost(t, g, sh);
     if (cost < best_cost) {
       best_cost = cost;
@@ -304,12 +312,17 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
   y.alloc(es * m.g.ndof);
   SF_CUDA(launch_fill_hash(t == F64 ? F64 : F32, m.g.ndof, 7u, u.p, s));
   SF_CUDA(launch_fill(t == F64 ? F64 : F32, m.g.ne(), 1.0, E.p, nullptr, s));
-  // the candidates of the lowest modelled time
-  std::vector<SweepShape> cands = sweep_candidates(t, m.g);
-  std::stable_sort(cands.begin(), cands.end(), [&](const SweepShape& a, const SweepShape& b) {
+  // the 48 candidates of the lowest modelled time, six of a cross section at most (with
+  // the model's ten depths alone 30.6 us a cold smoothing step of 512k elements, 28.8 so)
+  std::vector<SweepShape> all = sweep_candidates(t, m.g, true), cands;
+  std::stable_sort(all.begin(), all.end(), [&](const SweepShape& a, const SweepShape& b) {
     return sweep_cost(t, m.g, a) < sweep_cost(t, m.g, b);
   });
-  if (cands.size() > 48) cands.resize(48);
+  for (const SweepShape& sh : all) {
+    const auto same = std::count_if(cands.begin(), cands.end(),
+                                    [&](const SweepShape& o) { return o.bj == sh.bj && o.bk == sh.bk; });
+    if (same < 6 && cands.size() < 48) cands.push_back(sh);
+  }
   constexpr int kTuneReps = 8;
   cudaEvent_t e0, e1;
   SF_CUDA(cudaEventCreate(&e0));
