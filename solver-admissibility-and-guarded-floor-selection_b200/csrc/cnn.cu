@@ -363,6 +363,13 @@ __device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
                "l"(src), "r"(ok ? 16 : 0));
 }
+// the same from a source that is aligned to its type only
+__device__ __forceinline__ void cp16_by_float(float* dst, const float* src) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst + k)),
+                 "l"(src + k));
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int LEFT>
 __device__ __forceinline__ void cp_wait() {
@@ -472,11 +479,13 @@ __global__ void __launch_bounds__(256, 1) conv_s2_bwd_param_kernel(int N, const 
 
 // First layer's weight and bias gradients, in the same order of sums: a block takes
 // one output channel and one row ky of taps, thread t the position (y, x) of every
-// plane (256 positions a plane), sliding along z.
+// plane (256 positions a plane), sliding along z.  x is the caller's and may start at any
+// float: ALIGNED (to 16 bytes) copies it four floats at a time, otherwise one.
 struct Wgrad0 {
   static constexpr int TILE = 18 * 18 * 16, STEP = TILE + 4096;  // padded planes and rows of one sample, its gradients
   static constexpr size_t SMEM = sizeof(float) * kRing * STEP;
 };
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256, 1) conv0_bwd_param_kernel(int N, const float* __restrict__ dy,
                                                                  const float* __restrict__ x, float* __restrict__ gW,
                                                                  float* __restrict__ gb) {
@@ -489,7 +498,10 @@ __global__ void __launch_bounds__(256, 1) conv0_bwd_param_kernel(int N, const fl
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int e = tid + 256 * u, c = 4 * (e & 3), ry = (e >> 2) & 15, rz = e >> 6;
-      cp16(t + ((rz + 1) * 18 + ry + 1) * 16 + c, x + ((int64_t)n << 12) + 4 * e, true);
+      float* xd = t + ((rz + 1) * 18 + ry + 1) * 16 + c;
+      const float* xs = x + ((int64_t)n << 12) + 4 * e;
+      if (ALIGNED) cp16(xd, xs, true);
+      else cp16_by_float(xd, xs);
       cp16(t + Wgrad0::TILE + 4 * e, dy + (((int64_t)n * 16 + co) << 12) + 4 * e, true);
     }
   };
@@ -734,7 +746,8 @@ void set_attributes() {
     big_smem(conv_s2_bwd_param_kernel<16, 16, 16, 24>, G1::SMEM);
     big_smem(conv_s2_bwd_param_kernel<16, 32, 8, 12>, G2::SMEM);
     big_smem(conv_s2_bwd_param_kernel<32, 32, 4, 4>, G3::SMEM);
-    big_smem(conv0_bwd_param_kernel, Wgrad0::SMEM);
+    big_smem(conv0_bwd_param_kernel<true>, Wgrad0::SMEM);
+    big_smem(conv0_bwd_param_kernel<false>, Wgrad0::SMEM);
     return cudaSuccess;
   }));
 }
@@ -787,8 +800,8 @@ void backward(simpfem_cnn* h, const float* x, const int32_t* labels, int N, cuda
   conv_s2_bwd_data_kernel<16, 16, 16, 4, 1, 4><<<dim3(N, 4), D1::THREADS, D1::SMEM, s>>>(
       N, h->dact[2].as<float>(), wb + t_off(1), h->act[1].as<float>(), h->dact[1].as<float>());
   SF_CUDA(sf_launched(1));
-  conv0_bwd_param_kernel<<<48, 256, Wgrad0::SMEM, s>>>(N, h->dact[1].as<float>(), x, g + w_off(0),
-                                                                     g + b_off(0));
+  auto first = (uintptr_t)x % 16 == 0 ? conv0_bwd_param_kernel<true> : conv0_bwd_param_kernel<false>;
+  first<<<48, 256, Wgrad0::SMEM, s>>>(N, h->dact[1].as<float>(), x, g + w_off(0), g + b_off(0));
   SF_CUDA(sf_launched(1));
 }
 
