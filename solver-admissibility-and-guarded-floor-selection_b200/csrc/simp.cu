@@ -483,7 +483,8 @@ int simpfem_cone_filter(int nx, int ny, int nz, double rmin, int transpose, cons
   SIMP_API_END
 }
 
-size_t simpfem_oc_work_bytes(void) { return kGridCommBytes + sizeof(double) * 4; }
+// the exchange slots, the four results, and room to start the slots on 16 bytes
+size_t simpfem_oc_work_bytes(void) { return kGridCommBytes + sizeof(double) * 4 + 8; }
 
 int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
                       double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
@@ -500,8 +501,9 @@ int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const doub
   const int nb = (int)std::min<int64_t>(grid_sm_count(), div_up(n, 2 * kOcThreads));
   constexpr int kMaxKeep = 224 * 1024 / (4 * 8 * kOcThreads);
   int keep = (int)std::min<int64_t>(kMaxKeep, div_up(n, (int64_t)nb * kOcThreads));
-  ulonglong2* slots = (ulonglong2*)work;
-  double* out = work + kGridCommBytes / sizeof(double);
+  // the slots are read and written as pairs of words; work is aligned to its type only
+  ulonglong2* slots = (ulonglong2*)(((uintptr_t)work + 15) / 16 * 16);
+  double* out = (double*)slots + kGridCommBytes / sizeof(double);
   SF_CUDA(cudaMemsetAsync(slots, 0, kGridCommBytes, s));
   double target = volfrac * (double)n;
   void* args[] = {&n, (void*)&rho, (void*)&dc, (void*)&dv, (void*)&vol_w, &target, &move, &keep, &rho_new, &slots, &out};
