@@ -748,7 +748,7 @@ void solve_coarsest(Gmg& G, const void* rhs, void* x) {
   }
   if (G.coarse_mode == 2 && G.pcg_rows > 0) {
     SF_CUDA(launch_pcg_coop(G.cyc, G.pcg_rows, L.g, L.K64.as<double>(), L.dinv64.as<double>(), rhs, x,
-                            G.pz.as<double>(), coarse_pcg_count(G), G.pcomm.p, G.guard, G.st));
+                            coarse_pcg_count(G), G.pcomm.p, G.guard, G.st));
     return;
   }
   if (G.coarse_mode == 1) {
@@ -1372,15 +1372,15 @@ static void setup_coarsest(Gmg& G) {
   G.coarse_mode = 2;
   const int64_t nd = L.g.ndof;
   G.pcg_rows = pcg_coop_rows(nd, cooperative_available());
-  G.pz.alloc(8 * nd);
   if (G.pcg_rows > 0) {
     if (!G.pcomm.p) {
-      G.pcomm.alloc(pcg_coop_comm_bytes());
-      SF_CUDA(cudaMemsetAsync(G.pcomm.p, 0, pcg_coop_comm_bytes(), G.st));
+      G.pcomm.alloc(pcg_coop_comm_bytes(nd));
+      SF_CUDA(cudaMemsetAsync(G.pcomm.p, 0, pcg_coop_comm_bytes(nd), G.st));
     }
     return;
   }
   G.pr.alloc(8 * nd);
+  G.pz.alloc(8 * nd);
   G.pp.alloc(8 * nd);
   G.pAp.alloc(8 * nd);
 }

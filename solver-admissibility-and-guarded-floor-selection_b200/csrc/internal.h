@@ -293,13 +293,13 @@ cudaError_t launch_pcg_p(int64_t n, const double* z, double* p, const double* sc
                          cudaStream_t s);
 // The fixed-count Jacobi PCG of the coarsest level in one cooperative launch
 // (FP64 throughout; right-hand side and answer in t).  rows: pcg_coop_rows(), 0
-// where the system does not fit; comm: pcg_coop_comm_bytes() bytes zeroed once,
-// serving one stream at a time; z: ndof doubles of scratch.
-size_t pcg_coop_comm_bytes();
+// where the system does not fit; comm: pcg_coop_comm_bytes(ndof) bytes zeroed once,
+// serving one stream at a time.
+size_t pcg_coop_comm_bytes(int64_t n);
 int pcg_coop_rows(int64_t n, bool cooperative);
 bool cooperative_available();  // the device can run cooperative launches
 cudaError_t launch_pcg_coop(DType t, int rows, const Grid& g, const double* coef, const double* dinv, const void* b,
-                            void* x, double* z, int iters, void* comm, const int* guard, cudaStream_t s);
+                            void* x, int iters, void* comm, const int* guard, cudaStream_t s);
 cudaError_t launch_dmul(int64_t n, const double* dinv, const double* r, double* z, const int* guard,
                         cudaStream_t s);
 cudaError_t launch_select_vec(DType t, int64_t n, const void* trial, const void* r,

@@ -1298,17 +1298,22 @@ cudaError_t launch_pcg_p(int64_t n, const double* z, double* p, const double* sc
 // updates 1.7 each) around 0.6 MFLOP; here it is two grid exchanges.  A lane also
 // keeps the values of p at its 11 neighbours and updates them itself from the
 // published z (p = z + beta p is the same arithmetic wherever it is done), so p is
-// never exchanged: the exchange that sums <r, z> also publishes z, the one that
-// sums <p, Ap> carries no data.  The coefficients are read once per solve.
-// 7,098 unknowns, 200 iterations: 4.2 ms busy in 6.2 ms of launches -> 1.09 ms.
+// never exchanged.  z goes from block to block in words that carry the number of the
+// exchange that sums <r, z>, like the parts of the sum: a reader takes a value when it
+// carries that number, and no store has to be ordered before the sum (with z in plain
+// words a fence on both sides of block 0's relay is needed for that: 0.5 us an
+// iteration).  The next z is written after the sum <p, Ap>, whose parts hang on every read
+// of this one.  The coefficients are read once per solve.
+// 7,098 unknowns, 200 iterations: 4.2 ms busy in 6.2 ms of launches -> 0.87 ms; 14,196
+// (two rows a group) 1.16, 22,971 (three) 1.56.
 constexpr int kPcgThreads = 512, kPcgLanes = 8, kPcgRows = kPcgThreads / kPcgLanes, kPcgTerms = 11;
 
-// comm: the exchange slots, then the number of the last exchange (kept on the
-// device so that a captured launch can be replayed)
+// comm: the exchange slots, the number of the last exchange (kept on the device so
+// that a captured launch can be replayed), then z
 template <int P, typename T>
 __global__ void __launch_bounds__(kPcgThreads, 1)
     pcg_coop_kernel(Grid g, const double* __restrict__ coef, const double* __restrict__ dinv, const T* __restrict__ b,
-                    T* __restrict__ x, double* z, int iters, ulonglong2* slots, unsigned* last, const int* guard) {
+                    T* __restrict__ x, ulonglong2* z, int iters, ulonglong2* slots, unsigned* last, const int* guard) {
   if (guard_off(guard)) return;
   __shared__ double red[kPcgThreads / 32];
   __shared__ double total;
@@ -1321,13 +1326,12 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
   double* scf = psm + tid;
   int* sat = reinterpret_cast<int*>(psm + (size_t)P * kPcgTerms * kPcgThreads) + tid;
   double rcf[kPcgTerms], pn[P][kPcgTerms];
-  int rat[kPcgTerms], row[P];
-  double xr[P], r[P], zr[P], pr[P], di[P];
+  int rat[kPcgTerms];
 #pragma unroll
   for (int k = 0; k < P; ++k) {
-    row[k] = (blockIdx.x * P + k) * kPcgRows + tid / kPcgLanes;
-    const bool ok = row[k] < n;
-    const int node = ok ? row[k] / 3 : 0, c = ok ? row[k] - 3 * node : 0;
+    const int row = (blockIdx.x * P + k) * kPcgRows + tid / kPcgLanes;
+    const bool ok = row < n;
+    const int node = ok ? row / 3 : 0, c = ok ? row - 3 * node : 0;
     const int kz = node % NZ1, jq = node / NZ1, jy = jq % NY1, ix = jq / NY1;
 #pragma unroll
     for (int m = 0; m < kPcgTerms; ++m) {
@@ -1336,7 +1340,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
       const bool in = ok && t < 81 && ix + ox >= 0 && ix + ox <= g.nx && jy + oy >= 0 && jy + oy <= g.ny &&
                       kz + oz >= 0 && kz + oz <= g.nz;
       // a neighbour outside the grid has zero coefficients; its slot points at the row itself
-      const int idx = in ? 3 * (node + (ox * NY1 + oy) * NZ1 + oz) + q : (ok ? row[k] : 0);
+      const int idx = in ? 3 * (node + (ox * NY1 + oy) * NZ1 + oz) + q : (ok ? row : 0);
       const double cv = in ? coef[(int64_t)(o * 9 + c * 3 + q) * nn + node] : 0.0;
       if (P == 1) {
         rat[m] = idx;
@@ -1347,15 +1351,17 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
       }
       pn[k][m] = 0.0;
     }
-    xr[k] = 0.0;
-    pr[k] = 0.0;
-    r[k] = ok ? (double)b[row[k]] : 0.0;
-    di[k] = ok ? dinv[row[k]] : 0.0;
-    zr[k] = __dmul_rn(di[k], r[k]);
   }
-  // sum of the rows' v (held by every lane of a row) over the grid; with publish,
-  // everything stored before it is visible to every block after it
-  auto grid_sum = [&](double v, bool publish) -> double {
+  // lane k of a group keeps the vectors' entries of the group's row k (the lanes beyond P
+  // those of row 0 once more), which saves ten registers for every further row
+  const int own = sub < P ? sub : 0, row = (blockIdx.x * P + own) * kPcgRows + tid / kPcgLanes;
+  const bool mine = sub < P && row < n;
+  double xr = 0.0, pr = 0.0, r = row < n ? (double)b[row] : 0.0;
+  const double di = row < n ? dinv[row] : 0.0;
+  double zr = __dmul_rn(di, r);
+  auto of_row = [&](double v, int k) { return P == 1 ? v : __shfl_sync(0xffffffffu, v, k, kPcgLanes); };
+  // sum of the rows' v (held by every lane of a row) over the grid
+  auto grid_sum = [&](double v) -> double {
     v = sub == 0 ? v : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1366,9 +1372,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
       double s[1] = {lane < kPcgThreads / 32 ? red[lane] : 0.0};
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-      if (publish) __threadfence();
       const bool all = grid_allreduce_warp<1>(slots, epoch, s);
-      if (publish) __threadfence();
       if (lane == 0) {
         total = s[0];
         good = all ? 1 : 0;
@@ -1378,62 +1382,66 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
     return total;
   };
   auto publish_z = [&]() -> double {
+    if (mine) grid_put(z + row, zr, epoch + 1);
     double v = 0.0;
 #pragma unroll
-    for (int k = 0; k < P; ++k) {
-      if (sub == 0 && row[k] < n) __stcg(z + row[k], zr[k]);
-      v += r[k] * zr[k];
-    }
-    return grid_sum(v, true);
+    for (int k = 0; k < P; ++k) v += of_row(r, k) * of_row(zr, k);
+    return grid_sum(v);
   };
+  int polls = kGridPolls;  // of this thread for z, in the whole solve
   double rz = publish_z(), beta = 0.0;
   bool ok = good != 0;
   for (int it = 0; ok && it < iters; ++it) {
-    double pap = 0.0, Ap[P];
+    double pap = 0.0, Ap = 0.0;
+    pr = __dadd_rn(zr, __dmul_rn(beta, pr));
 #pragma unroll
     for (int k = 0; k < P; ++k) {
-      double zn[kPcgTerms], a0 = 0.0, a1 = 0.0;
+      double a0 = 0.0, a1 = 0.0;
+      constexpr int CH = P == 1 ? kPcgTerms : 6;  // words in flight (eleven of several rows spill)
 #pragma unroll
-      for (int m = 0; m < kPcgTerms; ++m)
-        zn[m] = __ldcg(z + (P == 1 ? rat[m] : sat[(k * kPcgTerms + m) * kPcgThreads]));
+      for (int c = 0; c < kPcgTerms; c += CH) {
+        double zn[CH];
+        bool in = false;
+        do {
+          in = true;
 #pragma unroll
-      for (int m = 0; m < kPcgTerms; ++m) {
-        pn[k][m] = __dadd_rn(zn[m], __dmul_rn(beta, pn[k][m]));
-        const double cv = P == 1 ? rcf[m] : scf[(k * kPcgTerms + m) * kPcgThreads];
-        if (m & 1) a1 += cv * pn[k][m];
-        else a0 += cv * pn[k][m];
+          for (int m = c; m < kPcgTerms && m < c + CH; ++m)
+            in = grid_get(z + (P == 1 ? rat[m] : sat[(k * kPcgTerms + m) * kPcgThreads]), zn[m - c], epoch) && in;
+        } while (!in && --polls > 0);
+        if (!in) zn[0] = NAN;  // carried into every row by the sums
+#pragma unroll
+        for (int m = c; m < kPcgTerms && m < c + CH; ++m) {
+          pn[k][m] = __dadd_rn(zn[m - c], __dmul_rn(beta, pn[k][m]));
+          const double cv = P == 1 ? rcf[m] : scf[(k * kPcgTerms + m) * kPcgThreads];
+          if (m & 1) a1 += cv * pn[k][m];
+          else a0 += cv * pn[k][m];
+        }
       }
       double a = a0 + a1;
 #pragma unroll
       for (int o = kPcgLanes / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      Ap[k] = a;
-      pr[k] = __dadd_rn(zr[k], __dmul_rn(beta, pr[k]));
-      pap += pr[k] * a;
+      if (own == k) Ap = a;
+      pap += of_row(pr, k) * a;
     }
-    const double s = grid_sum(pap, false);
+    const double s = grid_sum(pap);
     ok = good != 0;
     if (!ok) break;
     const double alpha = rz / (s + 1e-300);
-#pragma unroll
-    for (int k = 0; k < P; ++k) {
-      xr[k] = __dadd_rn(xr[k], __dmul_rn(alpha, pr[k]));
-      r[k] = __dsub_rn(r[k], __dmul_rn(alpha, Ap[k]));
-      zr[k] = __dmul_rn(di[k], r[k]);
-    }
+    xr = __dadd_rn(xr, __dmul_rn(alpha, pr));
+    r = __dsub_rn(r, __dmul_rn(alpha, Ap));
+    zr = __dmul_rn(di, r);
     if (it + 1 == iters) break;  // nothing reads the last z
     const double rzn = publish_z();
     ok = good != 0;
     beta = rzn / (rz + 1e-300);
     rz = rzn;
   }
-#pragma unroll
-  for (int k = 0; k < P; ++k)
-    // a solve whose exchange ran out of its wait answers NaN, which the outer solve's guard refuses
-    if (sub == 0 && row[k] < n) x[row[k]] = ok ? (T)xr[k] : (T)NAN;
+  // a solve whose exchange ran out of its wait answers NaN, which the outer solve's guard refuses
+  if (mine) x[row] = ok ? (T)xr : (T)NAN;
   if (blockIdx.x == 0 && tid == 0) *last = epoch;
 }
 
-size_t pcg_coop_comm_bytes() { return kGridCommBytes + 16; }
+size_t pcg_coop_comm_bytes(int64_t n) { return kGridCommBytes + 16 + 16 * (size_t)n; }
 
 // Rows a lane group holds (1..3) when the system fits the grid at one block per
 // SM, else 0: one row per group up to 148 x 64 = 9,472 unknowns, three up to 28,416
@@ -1446,12 +1454,13 @@ int pcg_coop_rows(int64_t n, bool cooperative) {
 
 template <typename T>
 static cudaError_t pcg_coop_dispatch(int rows, const Grid& g, const double* coef, const double* dinv, const T* b, T* x,
-                                     double* z, int iters, void* comm, const int* guard, cudaStream_t s) {
+                                     int iters, void* comm, const int* guard, cudaStream_t s) {
   const void* f = rows == 1 ? (const void*)pcg_coop_kernel<1, T>
                   : rows == 2 ? (const void*)pcg_coop_kernel<2, T>
                               : (const void*)pcg_coop_kernel<3, T>;
   ulonglong2* slots = (ulonglong2*)comm;
   unsigned* last = (unsigned*)((char*)comm + kGridCommBytes);
+  ulonglong2* z = (ulonglong2*)((char*)comm + kGridCommBytes + 16);
   Grid gg = g;
   void* args[] = {&gg, (void*)&coef, (void*)&dinv, (void*)&b, (void*)&x, &z, &iters, &slots, &last, (void*)&guard};
   const size_t smem = rows == 1 ? 0 : (size_t)rows * kPcgTerms * kPcgThreads * 12;
@@ -1470,11 +1479,11 @@ static cudaError_t pcg_coop_dispatch(int rows, const Grid& g, const double* coef
 }
 
 cudaError_t launch_pcg_coop(DType t, int rows, const Grid& g, const double* coef, const double* dinv, const void* b,
-                            void* x, double* z, int iters, void* comm, const int* guard, cudaStream_t s) {
+                            void* x, int iters, void* comm, const int* guard, cudaStream_t s) {
   if (rows < 1 || rows > 3 || g.ndof >= (int64_t(1) << 30)) return cudaErrorInvalidValue;
   if (t == F64)
-    return pcg_coop_dispatch<double>(rows, g, coef, dinv, (const double*)b, (double*)x, z, iters, comm, guard, s);
-  return pcg_coop_dispatch<float>(rows, g, coef, dinv, (const float*)b, (float*)x, z, iters, comm, guard, s);
+    return pcg_coop_dispatch<double>(rows, g, coef, dinv, (const double*)b, (double*)x, iters, comm, guard, s);
+  return pcg_coop_dispatch<float>(rows, g, coef, dinv, (const float*)b, (float*)x, iters, comm, guard, s);
 }
 
 // z = dinv * r (elementwise), guarded
