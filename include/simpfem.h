@@ -205,6 +205,17 @@ int simpfem_gmg_apply(simpfem_gmg* g, const double* rhs_free, double* z_free, vo
 int simpfem_gmg_cycle_trace(simpfem_gmg* g, const double* rhs_free, int cycle_type, double* visits,
                             int max_visits, int* n_visits, double* summary, void* stream);
 int simpfem_gmg_props_get(simpfem_gmg* g, simpfem_gmg_props* out);
+/* Kernels that sum over their whole grid in one launch (Arnoldi column, fixed-count
+ * coarse PCG, OC bisection; no reference counterpart).  A block that has polled for the
+ * others' parts this often without success gives up: a solve then ends unconverged,
+ * simpfem_oc_update returns SIMPFEM_EINTERNAL, and the next call starts afresh. */
+typedef struct simpfem_grid_opts {
+  int polls;       /* of every block but the first; default 2^21, about two seconds */
+  int polls_first; /* of the first block; below 0 counts as 0 in both */
+} simpfem_grid_opts;
+void simpfem_grid_default_opts(simpfem_grid_opts* o);
+/* Options of the hierarchy's solves from the next call on (opts NULL: the defaults). */
+void simpfem_gmg_set_grid_opts(simpfem_gmg* g, const simpfem_grid_opts* opts);
 /* Average device time (ms) of one fused smoothing step of `level` (below the
  * coarsest) -- the operator kernel with the smoother's update fused into its
  * store, the kernel the cycle launches most -- over `reps` launches, each timed by
@@ -385,6 +396,11 @@ size_t simpfem_oc_work_bytes(void);
 int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
                       double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
                       double* change_host, double* lambda_host, int* steps_host, void* stream);
+/* The same with options of its launch (opts NULL: the defaults); its status in *status. */
+void simpfem_oc_update_opts(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
+                            double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
+                            double* change_host, double* lambda_host, int* steps_host,
+                            const simpfem_grid_opts* opts, void* stream, int* status);
 
 /* Heaviside projection proj = (tanh(b eta) + tanh(b (x - eta))) / den and its
  * derivative dproj = b (1 - tanh(b (x - eta))^2) / den, den = tanh(b eta) +

@@ -465,6 +465,19 @@ int simpfem_gmg_props_get(simpfem_gmg* g, simpfem_gmg_props* p) {
   SF_API_END
 }
 
+void simpfem_grid_default_opts(simpfem_grid_opts* o) {
+  o->polls = kGridPolls;
+  o->polls_first = kGridPolls;
+}
+
+void simpfem_gmg_set_grid_opts(simpfem_gmg* g, const simpfem_grid_opts* opts) {
+  if (!g) return;
+  Gmg& G = *g->impl;
+  G.wait = grid_wait(opts);
+  for (KrylovWs* k : {&G.ik, &G.rl, &G.outer}) k->wait = G.wait;
+  ++G.setup_epoch;  // captured cycles hold the former options
+}
+
 int simpfem_gmg_reset_lambda_cache(simpfem_gmg* g) {
   SF_API_BEGIN
   if (!g) throw InvalidArg{"null gmg"};

@@ -70,6 +70,15 @@ bool cooperative_available() {
   return v == 2;
 }
 
+GridWait grid_wait(const simpfem_grid_opts* o) {
+  GridWait w;
+  if (o) {
+    w.polls = std::max(o->polls, 0);
+    w.polls0 = std::max(o->polls_first, 0);
+  }
+  return w;
+}
+
 static size_t dsize(DType t) { return t == F64 ? 8 : (t == F32 ? 4 : 2); }
 
 // ----------------------------------------------------------------------------
@@ -748,7 +757,7 @@ void solve_coarsest(Gmg& G, const void* rhs, void* x) {
   }
   if (G.coarse_mode == 2 && G.pcg_rows > 0) {
     SF_CUDA(launch_pcg_coop(G.cyc, G.pcg_rows, L.g, L.K64.as<double>(), L.dinv64.as<double>(), rhs, x,
-                            coarse_pcg_count(G), G.pcomm.p, G.guard, G.st));
+                            coarse_pcg_count(G), G.pcomm.p, G.wait, G.guard, G.st));
     return;
   }
   if (G.coarse_mode == 1) {

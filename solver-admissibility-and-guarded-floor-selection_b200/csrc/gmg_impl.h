@@ -107,6 +107,7 @@ struct KrylovWs {
   int64_t n = 0;
   DevBuf V, Z, w, r, H, cs, sn, g, y, sc, Zptr;
   DevBuf comm;      // exchange slots of the one-launch Arnoldi column
+  GridWait wait;
   ColumnPlan plan;
   DevBuf flags_dev;     // device-side control flags (read by every guarded kernel)
   PinnedBuf flags_pin;  // host mirror, refreshed by sync_flags()
@@ -209,6 +210,7 @@ struct Gmg {
   DevBuf pr, pz, pp, pAp;
   DevBuf pcomm;        // exchange slots of the one-launch form
   int pcg_rows = 0;    // its rows per lane group; 0: the launched form
+  GridWait wait;
 
   DevBuf sc;         // scalar scratch of the corrections
   DevBuf rhs64, out64, tmp64a, tmp64b, tmp64c, tmp64d;  // apply-level FP64 vectors
@@ -254,6 +256,8 @@ struct Gmg {
 
   int64_t nfull() const { return m->g.ndof; }
 };
+
+GridWait grid_wait(const simpfem_grid_opts* o);  // null: the defaults
 
 using PrecFn = std::function<void(const double* in, double* out, const int* guard)>;
 

@@ -14,16 +14,18 @@
 // alternate between two halves: a block writes exchange e + 2 only after it has
 // seen the sum of e + 1, to which every block adds only after it has read e.
 //
-// Every wait is bounded: after kGridPolls unsuccessful polls the exchange
+// Every wait is bounded: after GridExchange's number of unsuccessful polls the exchange
 // reports failure, the block leaves its loop and the others, no longer served,
-// do the same; the host reads the flag.
+// do the same; the host reads the flag.  Block 0 keeps the number of the last
+// exchange for the next launch on the buffer.  With up to kGridFlat blocks the others
+// may have passed an exchange that block 0 gave up and left parts of the next, so
+// after a failure it keeps a number beyond any in the slots (grid_last).
 #pragma once
 
 #include "common.cuh"
 
 namespace simpfem {
 
-constexpr int kGridPolls = 1 << 21;  // about two seconds
 constexpr int kGridSlots = 256;
 constexpr int kGridCopies = 8;       // copies of a sum published by block 0
 constexpr int kGridMaxBlocks = 160;  // blocks of one exchange: a multiple of 32 (a B200 has 148 SMs)
@@ -32,6 +34,18 @@ constexpr int kGridMaxVals = 4;
 // one exchange buffer: [2 halves][kGridMaxVals][kGridSlots] slots of two words
 constexpr size_t kGridCommBytes = (size_t)2 * kGridMaxVals * kGridSlots * 16;
 static_assert(kGridMaxBlocks + kGridCopies <= kGridSlots, "slots");
+
+// An exchange buffer and how often a block polls it before it gives up (block 0 by
+// itself, so that a test can make one side of an exchange give up alone).
+struct GridExchange {
+  ulonglong2* slots = nullptr;
+  unsigned* last = nullptr;  // number of the last exchange
+  int polls = kGridPolls, polls0 = kGridPolls;
+  __device__ __forceinline__ int limit() const { return blockIdx.x == 0 ? polls0 : polls; }
+};
+
+// what *last becomes when block 0 leaves at exchange epoch
+__device__ __forceinline__ unsigned grid_last(unsigned epoch, bool ok) { return ok ? epoch : epoch + 2; }
 
 __device__ __forceinline__ void grid_put(ulonglong2* slot, double v, unsigned epoch) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v), e = epoch;
@@ -50,9 +64,9 @@ __device__ __forceinline__ bool grid_get(const ulonglong2* slot, double& v, unsi
 // block (its 32 lanes call this together): v[k] of lane 0 is the block's part; on
 // return every lane holds the result.  False when a wait ran out.
 template <int NV, bool MAX = false>
-__device__ __forceinline__ bool grid_allreduce_warp(ulonglong2* slots, unsigned epoch, double (&v)[NV]) {
-  const int lane = threadIdx.x & 31, nb = (int)gridDim.x;
-  ulonglong2* half = slots + (size_t)(epoch & 1) * kGridMaxVals * kGridSlots;
+__device__ __forceinline__ bool grid_allreduce_warp(const GridExchange& x, unsigned epoch, double (&v)[NV]) {
+  const int lane = threadIdx.x & 31, nb = (int)gridDim.x, polls = x.limit();
+  ulonglong2* half = x.slots + (size_t)(epoch & 1) * kGridMaxVals * kGridSlots;
 #pragma unroll
   for (int k = 0; k < NV; ++k)
     if (lane == 0) grid_put(half + k * kGridSlots + blockIdx.x, v[k], epoch);
@@ -60,7 +74,7 @@ __device__ __forceinline__ bool grid_allreduce_warp(ulonglong2* slots, unsigned 
   if (nb <= kGridFlat || blockIdx.x == 0) {
     constexpr int PER = kGridMaxBlocks / 32;
     double got[NV][PER];
-    for (int tries = 0; tries < kGridPolls && !all; ++tries) {
+    for (int tries = 0; tries < polls && !all; ++tries) {
       bool ok = true;
 #pragma unroll
       for (int k = 0; k < NV; ++k)
@@ -86,7 +100,7 @@ __device__ __forceinline__ bool grid_allreduce_warp(ulonglong2* slots, unsigned 
       if (all && nb > kGridFlat && lane < kGridCopies) grid_put(half + k * kGridSlots + kGridMaxBlocks + lane, s, epoch);
     }
   } else {
-    for (int tries = 0; tries < kGridPolls && !all; ++tries) {
+    for (int tries = 0; tries < polls && !all; ++tries) {
       bool ok = true;
 #pragma unroll
       for (int k = 0; k < NV; ++k)
@@ -104,13 +118,13 @@ __device__ __forceinline__ bool grid_allreduce_warp(ulonglong2* slots, unsigned 
 constexpr int kGridParts = 2 * kGridMaxBlocks;
 static_assert(kGridParts + kGridCopies <= kGridMaxVals * kGridSlots && kGridParts % 16 == 0, "slots");
 
-__device__ __forceinline__ bool grid_sum_parts_warp(ulonglong2* half, unsigned epoch, int nparts, double* stage,
-                                                    double& v) {
+__device__ __forceinline__ bool grid_sum_parts_warp(ulonglong2* half, int polls, unsigned epoch, int nparts,
+                                                    double* stage, double& v) {
   const int lane = threadIdx.x & 31, nb = (int)gridDim.x;
   bool all = false;
   if (nb <= kGridFlat || blockIdx.x == 0) {
     constexpr int PER = kGridParts / 32;
-    for (int tries = 0; tries < kGridPolls && !all; ++tries) {
+    for (int tries = 0; tries < polls && !all; ++tries) {
       bool ok = true;
 #pragma unroll
       for (int p = 0; p < PER; ++p) {
@@ -127,7 +141,7 @@ __device__ __forceinline__ bool grid_sum_parts_warp(ulonglong2* half, unsigned e
     v = s;
     if (all && nb > kGridFlat && lane < kGridCopies) grid_put(half + kGridParts + lane, s, epoch);
   } else {
-    for (int tries = 0; tries < kGridPolls && !all; ++tries)
+    for (int tries = 0; tries < polls && !all; ++tries)
       all = __all_sync(0xffffffffu, grid_get(half + kGridParts + blockIdx.x % kGridCopies, v, epoch));
   }
   return all;

@@ -67,6 +67,14 @@ struct Grid {
   }
 };
 
+// Unsuccessful polls after which a block gives up an exchange over its grid
+// (gridcomm.cuh), by default about two seconds' worth.
+constexpr int kGridPolls = 1 << 21;
+struct GridWait {
+  int polls = kGridPolls;   // every block but the first
+  int polls0 = kGridPolls;  // the first block
+};
+
 // Tile shape of the fine-operator sweep kernel (chosen by the tuner).
 struct SweepShape {
   int bj = 8;   // element columns along y per block (one of them is a halo column)
@@ -273,7 +281,8 @@ size_t arnoldi_comm_bytes();
 ColumnPlan arnoldi_plan(int64_t n, bool cooperative);
 // comm: arnoldi_comm_bytes() bytes zeroed once, serving one stream at a time
 cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
-                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm, cudaStream_t s);
+                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm,
+                           const GridWait& wait, cudaStream_t s);
 cudaError_t launch_scale_vec(int64_t n, const double* src, const double* denom_dev, double* dst,
                              const int* guard, cudaStream_t s);
 cudaError_t launch_backsolve(KrylovDev k, cudaStream_t s);
@@ -299,7 +308,7 @@ size_t pcg_coop_comm_bytes(int64_t n);
 int pcg_coop_rows(int64_t n, bool cooperative);
 bool cooperative_available();  // the device can run cooperative launches
 cudaError_t launch_pcg_coop(DType t, int rows, const Grid& g, const double* coef, const double* dinv, const void* b,
-                            void* x, int iters, void* comm, const int* guard, cudaStream_t s);
+                            void* x, int iters, void* comm, const GridWait& wait, const int* guard, cudaStream_t s);
 cudaError_t launch_dmul(int64_t n, const double* dinv, const double* r, double* z, const int* guard,
                         cudaStream_t s);
 cudaError_t launch_select_vec(DType t, int64_t n, const void* trial, const void* r,

@@ -74,7 +74,7 @@ void fgmres_core(const KrylovEnv& E, KrylovWs& K, const double* b, double* x, bo
       E.A(K.Zj(j), K.w.as<double>(), cyc);
       if (K.plan.per > 0) {
         SF_CUDA(launch_arnoldi(n, kd, j, K.Vj(0), K.w.as<double>(), K.Vj(j + 1), tol, hist_dev, hist_cap, K.plan,
-                               K.comm.p, st));
+                               K.comm.p, K.wait, st));
       } else {
         double* Hc = kd.H + (size_t)j * ld;
         SF_CUDA(launch_mgs_first(n, K.Vj(0), K.w.as<double>(), E.rw, Hc, cyc, st));

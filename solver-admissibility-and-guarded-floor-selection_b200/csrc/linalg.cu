@@ -811,7 +811,7 @@ template <int MP, int PER, bool WSMEM>
 __global__ void __launch_bounds__(kColThreads, 1)
     arnoldi_kernel(int64_t n, KrylovDev k, int j, const double* __restrict__ V, const double* __restrict__ w,
                    double* __restrict__ vnew, double tol, double* hist, int hist_cap, int per, int parts,
-                   ulonglong2* slots, unsigned* last) {
+                   GridExchange x) {
   if (!k.flags[F_CYC]) return;
   extern __shared__ __align__(16) double csm[];  // WSMEM: w [per][threads]; else two vectors [2][MP * PER][threads]
   __shared__ double red[MP * kColThreads / 32];
@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(kColThreads, 1)
     const int e = base + q * stride;
     return base < stride && e < len ? e : len;
   };
-  unsigned epoch = *(volatile unsigned*)last;
+  unsigned epoch = *(volatile unsigned*)x.last;
   double wr[NE];
   auto fetch = [&](int i) {  // V_i into slot i & 1
     const double* src = V + (int64_t)i * n;
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(kColThreads, 1)
     __syncthreads();
     ++epoch;
     if (wid == 0) {
-      ulonglong2* half = slots + (size_t)(epoch & 1) * kGridMaxVals * kGridSlots;
+      ulonglong2* half = x.slots + (size_t)(epoch & 1) * kGridMaxVals * kGridSlots;
 #pragma unroll
       for (int z = 0; z < (MP + 1) / 2; ++z) {  // eight warps a part, four parts a round
         const int r = z * 32 + lane;
@@ -870,7 +870,7 @@ __global__ void __launch_bounds__(kColThreads, 1)
         if (r % 8 == 0 && mine < 2 * MP && part0 + mine < parts) grid_put(half + part0 + mine, s, epoch);
       }
       double s = 0.0;
-      const bool all = grid_sum_parts_warp(half, epoch, parts, stage, s);
+      const bool all = grid_sum_parts_warp(half, x.limit(), epoch, parts, stage, s);
       if (lane == 0) {
         total = s;
         good = all ? 1 : 0;
@@ -959,16 +959,30 @@ __global__ void __launch_bounds__(kColThreads, 1)
         }
     }
   }
-  if (blockIdx.x == 0 && tid == 0) {
-    if (ok) {
-      givens_update(k, j, hn, tol, hist, hist_cap);
-    } else {  // the solve ends unconverged; its caller's recomputed residual refuses the iterate
+  if (tid == 0) {
+    // a block that gave up (any: block 0 may have seen the last sum) has not written its
+    // part of V_{j+1}: the solve ends with the columns that block 0 has rotated
+    if (!ok) {
       k.flags[F_DONE] = 1;
       k.flags[F_NOTDONE] = 0;
       k.flags[F_CYC] = 0;
     }
-    *last = epoch;
+    if (blockIdx.x == 0) {
+      if (ok) givens_update(k, j, hn, tol, hist, hist_cap);
+      *x.last = grid_last(epoch, ok);
+    }
   }
+}
+
+// comm: the exchange slots, then the number of the last exchange (kept on the device so
+// that a captured launch can be replayed)
+static GridExchange grid_exchange(void* comm, const GridWait& wait) {
+  GridExchange x;
+  x.slots = (ulonglong2*)comm;
+  x.last = (unsigned*)((char*)comm + kGridCommBytes);
+  x.polls = wait.polls;
+  x.polls0 = wait.polls0;
+  return x;
 }
 
 size_t arnoldi_comm_bytes() { return kGridCommBytes + 16; }
@@ -1011,7 +1025,8 @@ static ColumnKernel column_kernel(const ColumnPlan& p) {
 }
 
 cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
-                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm, cudaStream_t s) {
+                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm,
+                           const GridWait& wait, cudaStream_t s) {
   static std::atomic<uint64_t> attr_done;
   cudaError_t e = once_per_device(attr_done, [] {
     for (const void* f : {(const void*)arnoldi_kernel<1, 1, true>, (const void*)arnoldi_kernel<8, 1, false>,
@@ -1026,11 +1041,10 @@ cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V
   if (e != cudaSuccess) return e;
   const ColumnKernel c = column_kernel(p);
   const size_t smem = (size_t)(p.wsmem ? p.per : 2 * c.elements) * kColThreads * sizeof(double);
-  ulonglong2* slots = (ulonglong2*)comm;
-  unsigned* last = (unsigned*)((char*)comm + kGridCommBytes);
+  GridExchange x = grid_exchange(comm, wait);
   KrylovDev kd = k;
   int per = p.per, parts = p.parts;
-  void* args[] = {&n, &kd, &j, (void*)&V, (void*)&w, &vnew, &tol, &hist, &hist_cap, &per, &parts, &slots, &last};
+  void* args[] = {&n, &kd, &j, (void*)&V, (void*)&w, &vnew, &tol, &hist, &hist_cap, &per, &parts, &x};
   e = cudaLaunchCooperativeKernel(c.fn, dim3(p.blocks), dim3(kColThreads), args, smem, s);
   return e != cudaSuccess ? e : sf_launched(1);
 }
@@ -1308,19 +1322,17 @@ cudaError_t launch_pcg_p(int64_t n, const double* z, double* p, const double* sc
 // (two rows a group) 1.16, 22,971 (three) 1.56.
 constexpr int kPcgThreads = 512, kPcgLanes = 8, kPcgRows = kPcgThreads / kPcgLanes, kPcgTerms = 11;
 
-// comm: the exchange slots, the number of the last exchange (kept on the device so
-// that a captured launch can be replayed), then z
 template <int P, typename T>
 __global__ void __launch_bounds__(kPcgThreads, 1)
     pcg_coop_kernel(Grid g, const double* __restrict__ coef, const double* __restrict__ dinv, const T* __restrict__ b,
-                    T* __restrict__ x, ulonglong2* z, int iters, ulonglong2* slots, unsigned* last, const int* guard) {
+                    T* __restrict__ x, ulonglong2* z, int iters, GridExchange gx, const int* guard) {
   if (guard_off(guard)) return;
   __shared__ double red[kPcgThreads / 32];
   __shared__ double total;
   __shared__ int good;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, sub = tid & (kPcgLanes - 1);
   const int nn = (int)g.nn, n = 3 * nn, NZ1 = g.nz + 1, NY1 = g.ny + 1;
-  unsigned epoch = *(volatile unsigned*)last;
+  unsigned epoch = *(volatile unsigned*)gx.last;
   // one row: coefficients and neighbour indices in registers; more: in shared memory
   extern __shared__ __align__(16) double psm[];  // P > 1: [P][kPcgTerms][kPcgThreads] doubles, then as many ints
   double* scf = psm + tid;
@@ -1372,7 +1384,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
       double s[1] = {lane < kPcgThreads / 32 ? red[lane] : 0.0};
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-      const bool all = grid_allreduce_warp<1>(slots, epoch, s);
+      const bool all = grid_allreduce_warp<1>(gx, epoch, s);
       if (lane == 0) {
         total = s[0];
         good = all ? 1 : 0;
@@ -1388,7 +1400,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
     for (int k = 0; k < P; ++k) v += of_row(r, k) * of_row(zr, k);
     return grid_sum(v);
   };
-  int polls = kGridPolls;  // of this thread for z, in the whole solve
+  int polls = gx.limit();  // of this thread for z, in the whole solve
   double rz = publish_z(), beta = 0.0;
   bool ok = good != 0;
   for (int it = 0; ok && it < iters; ++it) {
@@ -1438,9 +1450,10 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
   }
   // a solve whose exchange ran out of its wait answers NaN, which the outer solve's guard refuses
   if (mine) x[row] = ok ? (T)xr : (T)NAN;
-  if (blockIdx.x == 0 && tid == 0) *last = epoch;
+  if (blockIdx.x == 0 && tid == 0) *gx.last = grid_last(epoch, ok);
 }
 
+// the exchange, then z
 size_t pcg_coop_comm_bytes(int64_t n) { return kGridCommBytes + 16 + 16 * (size_t)n; }
 
 // Rows a lane group holds (1..3) when the system fits the grid at one block per
@@ -1454,15 +1467,14 @@ int pcg_coop_rows(int64_t n, bool cooperative) {
 
 template <typename T>
 static cudaError_t pcg_coop_dispatch(int rows, const Grid& g, const double* coef, const double* dinv, const T* b, T* x,
-                                     int iters, void* comm, const int* guard, cudaStream_t s) {
+                                     int iters, void* comm, const GridWait& wait, const int* guard, cudaStream_t s) {
   const void* f = rows == 1 ? (const void*)pcg_coop_kernel<1, T>
                   : rows == 2 ? (const void*)pcg_coop_kernel<2, T>
                               : (const void*)pcg_coop_kernel<3, T>;
-  ulonglong2* slots = (ulonglong2*)comm;
-  unsigned* last = (unsigned*)((char*)comm + kGridCommBytes);
+  GridExchange gx = grid_exchange(comm, wait);
   ulonglong2* z = (ulonglong2*)((char*)comm + kGridCommBytes + 16);
   Grid gg = g;
-  void* args[] = {&gg, (void*)&coef, (void*)&dinv, (void*)&b, (void*)&x, &z, &iters, &slots, &last, (void*)&guard};
+  void* args[] = {&gg, (void*)&coef, (void*)&dinv, (void*)&b, (void*)&x, &z, &iters, &gx, (void*)&guard};
   const size_t smem = rows == 1 ? 0 : (size_t)rows * kPcgTerms * kPcgThreads * 12;
   static std::atomic<uint64_t> attr_done;
   cudaError_t e = once_per_device(attr_done, [] {
@@ -1479,11 +1491,11 @@ static cudaError_t pcg_coop_dispatch(int rows, const Grid& g, const double* coef
 }
 
 cudaError_t launch_pcg_coop(DType t, int rows, const Grid& g, const double* coef, const double* dinv, const void* b,
-                            void* x, int iters, void* comm, const int* guard, cudaStream_t s) {
+                            void* x, int iters, void* comm, const GridWait& wait, const int* guard, cudaStream_t s) {
   if (rows < 1 || rows > 3 || g.ndof >= (int64_t(1) << 30)) return cudaErrorInvalidValue;
   if (t == F64)
-    return pcg_coop_dispatch<double>(rows, g, coef, dinv, (const double*)b, (double*)x, iters, comm, guard, s);
-  return pcg_coop_dispatch<float>(rows, g, coef, dinv, (const float*)b, (float*)x, iters, comm, guard, s);
+    return pcg_coop_dispatch<double>(rows, g, coef, dinv, (const double*)b, (double*)x, iters, comm, wait, guard, s);
+  return pcg_coop_dispatch<float>(rows, g, coef, dinv, (const float*)b, (float*)x, iters, comm, wait, guard, s);
 }
 
 // z = dinv * r (elementwise), guarded

@@ -288,7 +288,7 @@ __device__ __forceinline__ void oc_bounds(double rho, double move, double& lo, d
 __global__ void __launch_bounds__(kOcThreads, 1)
     oc_bisect_kernel(int64_t n, const double* __restrict__ rho, const double* __restrict__ dc,
                      const double* __restrict__ dv, const double* __restrict__ vw, double target, double move,
-                     int keep, double* rn, ulonglong2* slots, double* __restrict__ out) {
+                     int keep, double* rn, GridExchange x, double* __restrict__ out) {
   extern __shared__ __align__(16) double osm[];  // [4][keep][kOcThreads]
   __shared__ double red[3][kOcThreads / 32];
   __shared__ double sums[3];
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kOcThreads, 1)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
       }
-      const bool all = grid_allreduce_warp<3>(slots, epoch, v);
+      const bool all = grid_allreduce_warp<3>(x, epoch, v);
       if (lane == 0) {
         sums[0] = v[0];
         sums[1] = v[1];
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kOcThreads, 1)
     ch[0] = lane < kOcThreads / 32 ? red[0][lane] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ch[0] = fmax(ch[0], __shfl_down_sync(0xffffffffu, ch[0], o));
-    ok = grid_allreduce_warp<1, true>(slots, epoch + 1, ch);
+    ok = grid_allreduce_warp<1, true>(x, epoch + 1, ch);
   }
   if (blockIdx.x == 0 && tid == 0) {
     out[0] = ch[0];
@@ -486,9 +486,9 @@ int simpfem_cone_filter(int nx, int ny, int nz, double rmin, int transpose, cons
 // the exchange slots, the four results, and room to start the slots on 16 bytes
 size_t simpfem_oc_work_bytes(void) { return kGridCommBytes + sizeof(double) * 4 + 8; }
 
-int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
-                      double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
-                      double* change_host, double* lambda_host, int* steps_host, void* stream) {
+static int oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
+                     double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
+                     double* change_host, double* lambda_host, int* steps_host, const GridWait& wait, void* stream) {
   SIMP_API_BEGIN
   if (n < 1 || !rho || !dc || !vol_w || !rho_new || !work) throw InvalidArg{"simpfem_oc_update: null argument"};
   if (work_bytes < simpfem_oc_work_bytes()) throw InvalidArg{"simpfem_oc_update: workspace too small"};
@@ -502,11 +502,14 @@ int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const doub
   constexpr int kMaxKeep = 224 * 1024 / (4 * 8 * kOcThreads);
   int keep = (int)std::min<int64_t>(kMaxKeep, div_up(n, (int64_t)nb * kOcThreads));
   // the slots are read and written as pairs of words; work is aligned to its type only
-  ulonglong2* slots = (ulonglong2*)(((uintptr_t)work + 15) / 16 * 16);
-  double* out = (double*)slots + kGridCommBytes / sizeof(double);
-  SF_CUDA(cudaMemsetAsync(slots, 0, kGridCommBytes, s));
+  GridExchange x;
+  x.slots = (ulonglong2*)(((uintptr_t)work + 15) / 16 * 16);
+  x.polls = wait.polls;
+  x.polls0 = wait.polls0;
+  double* out = (double*)x.slots + kGridCommBytes / sizeof(double);
+  SF_CUDA(cudaMemsetAsync(x.slots, 0, kGridCommBytes, s));
   double target = volfrac * (double)n;
-  void* args[] = {&n, (void*)&rho, (void*)&dc, (void*)&dv, (void*)&vol_w, &target, &move, &keep, &rho_new, &slots, &out};
+  void* args[] = {&n, (void*)&rho, (void*)&dc, (void*)&dv, (void*)&vol_w, &target, &move, &keep, &rho_new, &x, &out};
   SF_CUDA(cudaLaunchCooperativeKernel((const void*)oc_bisect_kernel, dim3(nb), dim3(kOcThreads), args,
                                       sizeof(double) * 4 * (size_t)keep * kOcThreads, s));
   SF_CUDA(sf_launched(1));
@@ -518,6 +521,22 @@ int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const doub
   if (lambda_host) *lambda_host = h[1];
   if (steps_host) *steps_host = (int)h[2];
   SIMP_API_END
+}
+
+int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
+                      double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
+                      double* change_host, double* lambda_host, int* steps_host, void* stream) {
+  return oc_update(n, rho, dc, dv, vol_w, volfrac, move, rho_new, work, work_bytes, change_host, lambda_host,
+                   steps_host, GridWait(), stream);
+}
+
+void simpfem_oc_update_opts(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
+                            double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
+                            double* change_host, double* lambda_host, int* steps_host,
+                            const simpfem_grid_opts* opts, void* stream, int* status) {
+  const int st = oc_update(n, rho, dc, dv, vol_w, volfrac, move, rho_new, work, work_bytes, change_host, lambda_host,
+                           steps_host, grid_wait(opts), stream);
+  if (status) *status = st;
 }
 
 int simpfem_heaviside(int64_t n, const double* x, double beta, double eta, double* proj, double* dproj,

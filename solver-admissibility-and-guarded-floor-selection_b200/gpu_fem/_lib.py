@@ -82,6 +82,10 @@ class GmgProps(ctypes.Structure):
     ]
 
 
+class GridOpts(ctypes.Structure):
+    _fields_ = [("polls", ctypes.c_int), ("polls_first", ctypes.c_int)]
+
+
 class PolicyOpts(ctypes.Structure):
     _fields_ = [
         ("penal", ctypes.c_double),
@@ -161,6 +165,8 @@ _SIGS = {
     "simpfem_gmg_apply": (_I, [_P, _P, _P, _P]),
     "simpfem_gmg_cycle_trace": (_I, [_P, _P, _I, _P, _I, _P, _P, _P]),
     "simpfem_gmg_props_get": (_I, [_P, _P]),
+    "simpfem_grid_default_opts": (None, [_P]),
+    "simpfem_gmg_set_grid_opts": (None, [_P, _P]),
     "simpfem_gmg_reset_lambda_cache": (_I, [_P]),
     "simpfem_gmg_fine_E": (_I, [_P, _P]),
     "simpfem_fgmres": (_I, [_P, _P, _P, _P, _D, _I, _I, _P, _I, _P, _P, _P, _P]),
@@ -175,6 +181,7 @@ _SIGS = {
     "simpfem_cone_filter": (_I, [_I, _I, _I, _D, _I, _P, _P, _P]),
     "simpfem_oc_work_bytes": (ctypes.c_size_t, []),
     "simpfem_oc_update": (_I, [_I64, _P, _P, _P, _P, _D, _D, _P, _P, ctypes.c_size_t, _P, _P, _P, _P]),
+    "simpfem_oc_update_opts": (None, [_I64, _P, _P, _P, _P, _D, _D, _P, _P, ctypes.c_size_t, _P, _P, _P, _P, _P, _P]),
     "simpfem_heaviside": (_I, [_I64, _P, _D, _D, _P, _P, _P]),
     "simpfem_oc_projected_work_bytes": (ctypes.c_size_t, [_I64]),
     "simpfem_oc_update_projected": (_I, [_I, _I, _I, _D, _P, _P, _P, _D, _D, _D, _D, _P, _P, ctypes.c_size_t, _P, _P,
