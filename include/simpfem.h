@@ -212,6 +212,8 @@ int simpfem_gmg_props_get(simpfem_gmg* g, simpfem_gmg_props* out);
 typedef struct simpfem_grid_opts {
   int polls;       /* of every block but the first; default 2^21, about two seconds */
   int polls_first; /* of the first block; below 0 counts as 0 in both */
+  int one_launch;  /* 0: step by step in a launch each, which is also what runs where the
+                      device cannot hold the whole grid at once; default 1 */
 } simpfem_grid_opts;
 void simpfem_grid_default_opts(simpfem_grid_opts* o);
 /* Options of the hierarchy's solves from the next call on (opts NULL: the defaults). */
@@ -392,7 +394,8 @@ size_t simpfem_oc_work_bytes(void);
  * rho, dc, dv, vol_w, rho_new: device arrays of n doubles; work: device workspace of
  * at least simpfem_oc_work_bytes() bytes.  *change_host = max |rho_new - rho|,
  * *lambda_host the final multiplier, *steps_host the bisection steps (each may be
- * NULL).  The bisection is one cooperative launch; the stream is synchronised once. */
+ * NULL).  The bisection is one cooperative launch and the stream is synchronised once;
+ * where the device cannot hold its grid, a launch and a synchronisation per step. */
 int simpfem_oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
                       double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
                       double* change_host, double* lambda_host, int* steps_host, void* stream);

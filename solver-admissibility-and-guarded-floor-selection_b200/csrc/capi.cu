@@ -468,6 +468,7 @@ int simpfem_gmg_props_get(simpfem_gmg* g, simpfem_gmg_props* p) {
 void simpfem_grid_default_opts(simpfem_grid_opts* o) {
   o->polls = kGridPolls;
   o->polls_first = kGridPolls;
+  o->one_launch = 1;
 }
 
 void simpfem_gmg_set_grid_opts(simpfem_gmg* g, const simpfem_grid_opts* opts) {

@@ -57,17 +57,20 @@ int grid_sm_count() {
   return v;
 }
 
-bool cooperative_available() {
-  static std::atomic<int> cached[64];  // 0 unknown, 1 no, 2 yes
-  int dev = 0;
+int grid_coresident(const void* kernel, int threads, size_t smem) {
+  int dev = 0, coop = 0, sms = 0, per = 0;
   SF_CUDA(cudaGetDevice(&dev));
-  int v = dev < 64 ? cached[dev].load(std::memory_order_relaxed) : 0;
-  if (v == 0) {
-    SF_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev));
-    v = v ? 2 : 1;
-    if (dev < 64) cached[dev].store(v, std::memory_order_relaxed);
-  }
-  return v == 2;
+  SF_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  if (!coop) return 0;
+  SF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  SF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
+  return std::min(per * sms, kGridMaxBlocks);
+}
+
+bool grid_refused(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return false;
+  cudaGetLastError();
+  return true;
 }
 
 GridWait grid_wait(const simpfem_grid_opts* o) {
@@ -75,6 +78,7 @@ GridWait grid_wait(const simpfem_grid_opts* o) {
   if (o) {
     w.polls = std::max(o->polls, 0);
     w.polls0 = std::max(o->polls_first, 0);
+    w.one_launch = o->one_launch != 0;
   }
   return w;
 }
@@ -755,10 +759,14 @@ void solve_coarsest(Gmg& G, const void* rhs, void* x) {
     if (r != x) SF_CUDA(launch_copy(G.cyc, n, r, x, G.guard, G.st));
     return;
   }
-  if (G.coarse_mode == 2 && G.pcg_rows > 0) {
-    SF_CUDA(launch_pcg_coop(G.cyc, G.pcg_rows, L.g, L.K64.as<double>(), L.dinv64.as<double>(), rhs, x,
-                            coarse_pcg_count(G), G.pcomm.p, G.wait, G.guard, G.st));
-    return;
+  if (G.coarse_mode == 2 && G.pcg_rows > 0 && G.wait.one_launch) {
+    const cudaError_t e = launch_pcg_coop(G.cyc, G.pcg_rows, L.g, L.K64.as<double>(), L.dinv64.as<double>(), rhs, x,
+                                          coarse_pcg_count(G), G.pcomm.p, G.wait, G.guard, G.st);
+    if (!grid_refused(e)) {
+      SF_CUDA(e);
+      return;
+    }
+    G.pcg_rows = 0;
   }
   if (G.coarse_mode == 1) {
     SF_CUDA(launch_gather_idx(G.cyc, G.nc, G.c_idx.as<int32_t>(), rhs, G.cb.as<double>(), G.guard, G.st));
@@ -1380,13 +1388,10 @@ static void setup_coarsest(Gmg& G) {
   }
   G.coarse_mode = 2;
   const int64_t nd = L.g.ndof;
-  G.pcg_rows = pcg_coop_rows(nd, cooperative_available());
-  if (G.pcg_rows > 0) {
-    if (!G.pcomm.p) {
-      G.pcomm.alloc(pcg_coop_comm_bytes(nd));
-      SF_CUDA(cudaMemsetAsync(G.pcomm.p, 0, pcg_coop_comm_bytes(nd), G.st));
-    }
-    return;
+  if (G.pcg_rows < 0) G.pcg_rows = pcg_coop_rows(nd);
+  if (G.pcg_rows > 0 && !G.pcomm.p) {
+    G.pcomm.alloc(pcg_coop_comm_bytes(nd));
+    SF_CUDA(cudaMemsetAsync(G.pcomm.p, 0, pcg_coop_comm_bytes(nd), G.st));
   }
   G.pr.alloc(8 * nd);
   G.pz.alloc(8 * nd);

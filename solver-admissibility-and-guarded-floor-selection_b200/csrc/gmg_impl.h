@@ -128,7 +128,7 @@ struct KrylovWs {
     g.alloc(sizeof(double) * (restart + 1));
     y.alloc(sizeof(double) * restart);
     sc.alloc(sizeof(double) * 16);
-    plan = arnoldi_plan(n, cooperative_available());
+    plan = arnoldi_plan(n);
     if (plan.per > 0 && !comm.p) {
       comm.alloc(arnoldi_comm_bytes());
       SF_CUDA(cudaMemset(comm.p, 0, arnoldi_comm_bytes()));
@@ -209,7 +209,7 @@ struct Gmg {
   // iterative coarse (fixed PCG) vectors
   DevBuf pr, pz, pp, pAp;
   DevBuf pcomm;        // exchange slots of the one-launch form
-  int pcg_rows = 0;    // its rows per lane group; 0: the launched form
+  int pcg_rows = -1;   // its rows per lane group; 0: the launched form, -1: not planned yet
   GridWait wait;
 
   DevBuf sc;         // scalar scratch of the corrections

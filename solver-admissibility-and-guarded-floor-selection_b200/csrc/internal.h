@@ -73,7 +73,14 @@ constexpr int kGridPolls = 1 << 21;
 struct GridWait {
   int polls = kGridPolls;   // every block but the first
   int polls0 = kGridPolls;  // the first block
+  bool one_launch = true;   // false: the launched forms
 };
+// Blocks of a kernel that the current device holds at once (at most kGridMaxBlocks); 0
+// where it has no cooperative launches.  Launches of more are refused.
+int grid_coresident(const void* kernel, int threads, size_t smem);
+// A launch that was refused for the size of its grid after all (a context with fewer
+// SMs than the device): nothing ran, and the error is cleared.
+bool grid_refused(cudaError_t e);
 
 // Tile shape of the fine-operator sweep kernel (chosen by the tuner).
 struct SweepShape {
@@ -278,7 +285,7 @@ struct ColumnPlan {
   bool wsmem = false;  // w in shared memory instead of registers
 };
 size_t arnoldi_comm_bytes();
-ColumnPlan arnoldi_plan(int64_t n, bool cooperative);
+ColumnPlan arnoldi_plan(int64_t n);
 // comm: arnoldi_comm_bytes() bytes zeroed once, serving one stream at a time
 cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
                            double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm,
@@ -305,8 +312,7 @@ cudaError_t launch_pcg_p(int64_t n, const double* z, double* p, const double* sc
 // where the system does not fit; comm: pcg_coop_comm_bytes(ndof) bytes zeroed once,
 // serving one stream at a time.
 size_t pcg_coop_comm_bytes(int64_t n);
-int pcg_coop_rows(int64_t n, bool cooperative);
-bool cooperative_available();  // the device can run cooperative launches
+int pcg_coop_rows(int64_t n);
 cudaError_t launch_pcg_coop(DType t, int rows, const Grid& g, const double* coef, const double* dinv, const void* b,
                             void* x, int iters, void* comm, const GridWait& wait, const int* guard, cudaStream_t s);
 cudaError_t launch_dmul(int64_t n, const double* dinv, const double* r, double* z, const int* guard,

@@ -72,10 +72,15 @@ void fgmres_core(const KrylovEnv& E, KrylovWs& K, const double* b, double* x, bo
     for (int j = 0; j < inner; ++j) {
       M(K.Vj(j), K.Zj(j), cyc);
       E.A(K.Zj(j), K.w.as<double>(), cyc);
-      if (K.plan.per > 0) {
-        SF_CUDA(launch_arnoldi(n, kd, j, K.Vj(0), K.w.as<double>(), K.Vj(j + 1), tol, hist_dev, hist_cap, K.plan,
-                               K.comm.p, K.wait, st));
-      } else {
+      bool done = false;
+      if (K.plan.per > 0 && K.wait.one_launch) {
+        const cudaError_t e = launch_arnoldi(n, kd, j, K.Vj(0), K.w.as<double>(), K.Vj(j + 1), tol, hist_dev, hist_cap,
+                                             K.plan, K.comm.p, K.wait, st);
+        done = !grid_refused(e);
+        if (done) SF_CUDA(e);
+        else K.plan.per = 0;
+      }
+      if (!done) {
         double* Hc = kd.H + (size_t)j * ld;
         SF_CUDA(launch_mgs_first(n, K.Vj(0), K.w.as<double>(), E.rw, Hc, cyc, st));
         for (int i = 0; i <= j; ++i) {

@@ -987,28 +987,6 @@ static GridExchange grid_exchange(void* comm, const GridWait& wait) {
 
 size_t arnoldi_comm_bytes() { return kGridCommBytes + 16; }
 
-// The variant of the one-launch column; per = 0: the vectors are too long (or the
-// device cannot), the launched form runs.
-ColumnPlan arnoldi_plan(int64_t n, bool cooperative) {
-  ColumnPlan p;
-  if (!cooperative || n < 1) return p;
-  // Longer vectors take every SM, and eight solves in flight then wait for all of them at
-  // once: 512k elements (1.6 M unknowns) ran 173 batched solves/s with one launch a column
-  // against 186-198 launched step by step; one solve alone gains about 3 %.
-  if (n > 1000000) return p;
-  const int parts = red_blocks(n);
-  const int64_t per = div_up(n, (int64_t)parts * kRedThreads);
-  if (per * kColThreads * 8 > 216 * 1024) return p;
-  const int mp = per == 1 ? 8 : (per == 2 ? 4 : (per <= 4 ? 2 : 1));
-  const int blocks = (parts + 2 * mp - 1) / (2 * mp);
-  if (blocks > grid_sm_count()) return p;
-  p.per = (int)per;
-  p.parts = parts;
-  p.blocks = blocks;
-  p.wsmem = per > 24;
-  return p;
-}
-
 struct ColumnKernel {
   const void* fn;
   int elements;  // a thread
@@ -1023,29 +1001,57 @@ static ColumnKernel column_kernel(const ColumnPlan& p) {
   if (p.per <= 12) return {(const void*)arnoldi_kernel<1, 12, false>, 12};
   return {(const void*)arnoldi_kernel<1, 24, false>, 24};
 }
+static size_t column_smem(const ColumnPlan& p) {
+  return (size_t)(p.wsmem ? p.per : 2 * column_kernel(p).elements) * kColThreads * sizeof(double);
+}
 
-cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
-                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm,
-                           const GridWait& wait, cudaStream_t s) {
+static cudaError_t column_attributes() {
   static std::atomic<uint64_t> attr_done;
-  cudaError_t e = once_per_device(attr_done, [] {
+  return once_per_device(attr_done, [] {
     for (const void* f : {(const void*)arnoldi_kernel<1, 1, true>, (const void*)arnoldi_kernel<8, 1, false>,
                           (const void*)arnoldi_kernel<4, 2, false>, (const void*)arnoldi_kernel<2, 4, false>,
                           (const void*)arnoldi_kernel<1, 8, false>, (const void*)arnoldi_kernel<1, 12, false>,
                           (const void*)arnoldi_kernel<1, 24, false>}) {
-      const cudaError_t e2 = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
-      if (e2 != cudaSuccess) return e2;
+      const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+      if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
   });
+}
+
+// The variant of the one-launch column; per = 0: the vectors are too long (or the
+// device cannot hold its grid), the launched form runs.
+ColumnPlan arnoldi_plan(int64_t n) {
+  ColumnPlan p;
+  if (n < 1) return p;
+  // Longer vectors take every SM, and eight solves in flight then wait for all of them at
+  // once: 512k elements (1.6 M unknowns) ran 173 batched solves/s with one launch a column
+  // against 186-198 launched step by step; one solve alone gains about 3 %.
+  if (n > 1000000) return p;
+  const int parts = red_blocks(n);
+  const int64_t per = div_up(n, (int64_t)parts * kRedThreads);
+  if (per * kColThreads * 8 > 216 * 1024) return p;
+  const int mp = per == 1 ? 8 : (per == 2 ? 4 : (per <= 4 ? 2 : 1));
+  const int blocks = (parts + 2 * mp - 1) / (2 * mp);
+  p.per = (int)per;
+  p.parts = parts;
+  p.blocks = blocks;
+  p.wsmem = per > 24;
+  SF_CUDA(column_attributes());
+  if (blocks > grid_coresident(column_kernel(p).fn, kColThreads, column_smem(p))) p.per = 0;
+  return p;
+}
+
+cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
+                           double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm,
+                           const GridWait& wait, cudaStream_t s) {
+  cudaError_t e = column_attributes();
   if (e != cudaSuccess) return e;
-  const ColumnKernel c = column_kernel(p);
-  const size_t smem = (size_t)(p.wsmem ? p.per : 2 * c.elements) * kColThreads * sizeof(double);
   GridExchange x = grid_exchange(comm, wait);
   KrylovDev kd = k;
   int per = p.per, parts = p.parts;
   void* args[] = {&n, &kd, &j, (void*)&V, (void*)&w, &vnew, &tol, &hist, &hist_cap, &per, &parts, &x};
-  e = cudaLaunchCooperativeKernel(c.fn, dim3(p.blocks), dim3(kColThreads), args, smem, s);
+  e = cudaLaunchCooperativeKernel(column_kernel(p).fn, dim3(p.blocks), dim3(kColThreads), args, column_smem(p), s);
   return e != cudaSuccess ? e : sf_launched(1);
 }
 
@@ -1456,46 +1462,54 @@ __global__ void __launch_bounds__(kPcgThreads, 1)
 // the exchange, then z
 size_t pcg_coop_comm_bytes(int64_t n) { return kGridCommBytes + 16 + 16 * (size_t)n; }
 
+static const void* pcg_coop_fn(DType t, int rows) {
+  if (t == F64)
+    return rows == 1   ? (const void*)pcg_coop_kernel<1, double>
+           : rows == 2 ? (const void*)pcg_coop_kernel<2, double>
+                       : (const void*)pcg_coop_kernel<3, double>;
+  return rows == 1   ? (const void*)pcg_coop_kernel<1, float>
+         : rows == 2 ? (const void*)pcg_coop_kernel<2, float>
+                     : (const void*)pcg_coop_kernel<3, float>;
+}
+static size_t pcg_coop_smem(int rows) { return rows == 1 ? 0 : (size_t)rows * kPcgTerms * kPcgThreads * 12; }
+static cudaError_t pcg_coop_attributes() {
+  static std::atomic<uint64_t> attr_done;
+  return once_per_device(attr_done, [] {
+    for (DType t : {F64, F32})
+      for (int rows : {2, 3}) {
+        const cudaError_t e = cudaFuncSetAttribute(pcg_coop_fn(t, rows), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)pcg_coop_smem(rows));
+        if (e != cudaSuccess) return e;
+      }
+    return cudaSuccess;
+  });
+}
+
 // Rows a lane group holds (1..3) when the system fits the grid at one block per
 // SM, else 0: one row per group up to 148 x 64 = 9,472 unknowns, three up to 28,416
 // (each row takes 68 KB of a block's shared memory and, for p, 22 registers).
-int pcg_coop_rows(int64_t n, bool cooperative) {
-  if (!cooperative) return 0;
-  const int64_t per = div_up(n, (int64_t)grid_sm_count() * kPcgRows);
-  return per <= 3 ? (int)per : 0;
-}
-
-template <typename T>
-static cudaError_t pcg_coop_dispatch(int rows, const Grid& g, const double* coef, const double* dinv, const T* b, T* x,
-                                     int iters, void* comm, const GridWait& wait, const int* guard, cudaStream_t s) {
-  const void* f = rows == 1 ? (const void*)pcg_coop_kernel<1, T>
-                  : rows == 2 ? (const void*)pcg_coop_kernel<2, T>
-                              : (const void*)pcg_coop_kernel<3, T>;
-  GridExchange gx = grid_exchange(comm, wait);
-  ulonglong2* z = (ulonglong2*)((char*)comm + kGridCommBytes + 16);
-  Grid gg = g;
-  void* args[] = {&gg, (void*)&coef, (void*)&dinv, (void*)&b, (void*)&x, &z, &iters, &gx, (void*)&guard};
-  const size_t smem = rows == 1 ? 0 : (size_t)rows * kPcgTerms * kPcgThreads * 12;
-  static std::atomic<uint64_t> attr_done;
-  cudaError_t e = once_per_device(attr_done, [] {
-    const int most = 3 * kPcgTerms * kPcgThreads * 12;
-    const cudaError_t e2 =
-        cudaFuncSetAttribute(pcg_coop_kernel<2, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    return e2 != cudaSuccess
-               ? e2
-               : cudaFuncSetAttribute(pcg_coop_kernel<3, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  });
-  if (e != cudaSuccess) return e;
-  e = cudaLaunchCooperativeKernel(f, dim3(div_up(g.ndof, (int64_t)kPcgRows * rows)), dim3(kPcgThreads), args, smem, s);
-  return e != cudaSuccess ? e : sf_launched(1);
+int pcg_coop_rows(int64_t n) {
+  const int64_t rows = div_up(n, (int64_t)grid_sm_count() * kPcgRows);
+  if (rows > 3) return 0;
+  SF_CUDA(pcg_coop_attributes());
+  const int64_t blocks = div_up(n, (int64_t)kPcgRows * rows);
+  for (DType t : {F64, F32})
+    if (blocks > grid_coresident(pcg_coop_fn(t, (int)rows), kPcgThreads, pcg_coop_smem((int)rows))) return 0;
+  return (int)rows;
 }
 
 cudaError_t launch_pcg_coop(DType t, int rows, const Grid& g, const double* coef, const double* dinv, const void* b,
                             void* x, int iters, void* comm, const GridWait& wait, const int* guard, cudaStream_t s) {
   if (rows < 1 || rows > 3 || g.ndof >= (int64_t(1) << 30)) return cudaErrorInvalidValue;
-  if (t == F64)
-    return pcg_coop_dispatch<double>(rows, g, coef, dinv, (const double*)b, (double*)x, iters, comm, wait, guard, s);
-  return pcg_coop_dispatch<float>(rows, g, coef, dinv, (const float*)b, (float*)x, iters, comm, wait, guard, s);
+  cudaError_t e = pcg_coop_attributes();
+  if (e != cudaSuccess) return e;
+  GridExchange gx = grid_exchange(comm, wait);
+  ulonglong2* z = (ulonglong2*)((char*)comm + kGridCommBytes + 16);
+  Grid gg = g;
+  void* args[] = {&gg, (void*)&coef, (void*)&dinv, (void*)&b, (void*)&x, &z, &iters, &gx, (void*)&guard};
+  e = cudaLaunchCooperativeKernel(pcg_coop_fn(t, rows), dim3(div_up(g.ndof, (int64_t)kPcgRows * rows)),
+                                  dim3(kPcgThreads), args, pcg_coop_smem(rows), s);
+  return e != cudaSuccess ? e : sf_launched(1);
 }
 
 // z = dinv * r (elementwise), guarded

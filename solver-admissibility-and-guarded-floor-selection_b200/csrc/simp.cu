@@ -203,6 +203,20 @@ __device__ __forceinline__ double oc_candidate(double rho, double dc, double dv,
   return fmin(fmax(r, 1e-3), 1.0);
 }
 
+// partial sums of vw rn(lm): the volume of a candidate, a launch per bisection step
+__global__ void __launch_bounds__(kSimpThreads) oc_volume_kernel(int64_t n, const double* __restrict__ rho,
+                                                                 const double* __restrict__ dc,
+                                                                 const double* __restrict__ dv,
+                                                                 const double* __restrict__ vw, double lm, double move,
+                                                                 double* __restrict__ partials) {
+  __shared__ double sh[32];
+  double v = 0.0;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
+    v += vw[e] * oc_candidate(rho[e], dc[e], dv ? dv[e] : 1.0, lm, move);
+  const double t = block_reduce_sum(v, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = t;
+}
+
 // rn(lm) and partial maxima of |rn - rho|
 __global__ void __launch_bounds__(kSimpThreads) oc_candidate_kernel(int64_t n, const double* __restrict__ rho,
                                                                     const double* __restrict__ dc,
@@ -212,7 +226,7 @@ __global__ void __launch_bounds__(kSimpThreads) oc_candidate_kernel(int64_t n, c
   __shared__ double sh[32];
   double v = 0.0;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    const double r = oc_candidate(rho[e], dc[e], dv[e], lm, move);
+    const double r = oc_candidate(rho[e], dc[e], dv ? dv[e] : 1.0, lm, move);
     rn[e] = r;
     v = fmax(v, fabs(r - rho[e]));
   }
@@ -486,6 +500,53 @@ int simpfem_cone_filter(int nx, int ny, int nz, double rmin, int transpose, cons
 // the exchange slots, the four results, and room to start the slots on 16 bytes
 size_t simpfem_oc_work_bytes(void) { return kGridCommBytes + sizeof(double) * 4 + 8; }
 
+// The bisection by a launch and a synchronisation per step, for devices that cannot hold
+// the grid of the one launch: h = {change, lm, steps}.
+static void oc_bisect_launched(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
+                               double target, double move, double* rho_new, double* partials, double* out,
+                               cudaStream_t s, double (&h)[4]) {
+  const int nb = (int)std::min<int64_t>(kSimpBlocks, div_up(n, kSimpThreads));
+  auto finish = [&](int max) {
+    oc_finish_kernel<<<1, kSimpThreads, 0, s>>>(nb, max, partials, out);
+    SF_CUDA(sf_launched(2));
+    double v = 0.0;
+    SF_CUDA(cudaMemcpyAsync(&v, out, sizeof(v), cudaMemcpyDeviceToHost, s));
+    SF_CUDA(cudaStreamSynchronize(s));
+    return v;
+  };
+  double l1 = 0.0, l2 = 1e9, lm = 0.5 * (l1 + l2);
+  int steps = 0;
+  for (int it = 0; it < 100; ++it) {
+    lm = 0.5 * (l1 + l2);
+    oc_volume_kernel<<<nb, kSimpThreads, 0, s>>>(n, rho, dc, dv, vol_w, lm, move, partials);
+    const double vol = finish(0);
+    ++steps;
+    if (vol > target) l1 = lm;
+    else l2 = lm;
+    if (l2 - l1 < 1e-9) break;
+  }
+  oc_candidate_kernel<<<nb, kSimpThreads, 0, s>>>(n, rho, dc, dv, lm, move, rho_new, partials);
+  h[0] = finish(1);
+  h[1] = lm;
+  h[2] = steps;
+  h[3] = 0.0;
+}
+
+// blocks of the one-launch bisection that the device holds at once
+static int oc_coresident() {
+  constexpr int kMost = 224 * 1024;
+  static std::atomic<int> cached[64];  // 0 unknown, else the number + 1
+  int dev = 0;
+  SF_CUDA(cudaGetDevice(&dev));
+  int v = dev < 64 ? cached[dev].load(std::memory_order_relaxed) : 0;
+  if (v == 0) {
+    SF_CUDA(cudaFuncSetAttribute(oc_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+    v = grid_coresident((const void*)oc_bisect_kernel, kOcThreads, kMost) + 1;
+    if (dev < 64) cached[dev].store(v, std::memory_order_relaxed);
+  }
+  return v - 1;
+}
+
 static int oc_update(int64_t n, const double* rho, const double* dc, const double* dv, const double* vol_w,
                      double volfrac, double move, double* rho_new, double* work, size_t work_bytes,
                      double* change_host, double* lambda_host, int* steps_host, const GridWait& wait, void* stream) {
@@ -493,30 +554,36 @@ static int oc_update(int64_t n, const double* rho, const double* dc, const doubl
   if (n < 1 || !rho || !dc || !vol_w || !rho_new || !work) throw InvalidArg{"simpfem_oc_update: null argument"};
   if (work_bytes < simpfem_oc_work_bytes()) throw InvalidArg{"simpfem_oc_update: workspace too small"};
   cudaStream_t s = (cudaStream_t)stream;
-  static std::atomic<uint64_t> attr_done;
-  SF_CUDA(once_per_device(attr_done, [] {
-    return cudaFuncSetAttribute(oc_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-  }));
-  // two elements a thread or more before another block joins (an exchange costs more the more blocks take part)
-  const int nb = (int)std::min<int64_t>(grid_sm_count(), div_up(n, 2 * kOcThreads));
-  constexpr int kMaxKeep = 224 * 1024 / (4 * 8 * kOcThreads);
-  int keep = (int)std::min<int64_t>(kMaxKeep, div_up(n, (int64_t)nb * kOcThreads));
   // the slots are read and written as pairs of words; work is aligned to its type only
   GridExchange x;
   x.slots = (ulonglong2*)(((uintptr_t)work + 15) / 16 * 16);
   x.polls = wait.polls;
   x.polls0 = wait.polls0;
+  static_assert(kGridCommBytes >= sizeof(double) * kSimpBlocks, "partial sums of the launched form");
   double* out = (double*)x.slots + kGridCommBytes / sizeof(double);
-  SF_CUDA(cudaMemsetAsync(x.slots, 0, kGridCommBytes, s));
-  double target = volfrac * (double)n;
-  void* args[] = {&n, (void*)&rho, (void*)&dc, (void*)&dv, (void*)&vol_w, &target, &move, &keep, &rho_new, &x, &out};
-  SF_CUDA(cudaLaunchCooperativeKernel((const void*)oc_bisect_kernel, dim3(nb), dim3(kOcThreads), args,
-                                      sizeof(double) * 4 * (size_t)keep * kOcThreads, s));
-  SF_CUDA(sf_launched(1));
-  double h[4];
-  SF_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
-  SF_CUDA(cudaStreamSynchronize(s));
-  if (h[3] != 0.0) throw std::runtime_error("simpfem_oc_update: a grid exchange ran out of its wait");
+  double target = volfrac * (double)n, h[4];
+  const int most = wait.one_launch ? oc_coresident() : 0;
+  bool done = false;
+  if (most > 0) {
+    // two elements a thread or more before another block joins (an exchange costs more the more blocks take part)
+    const int nb = (int)std::min<int64_t>(std::min(most, grid_sm_count()), div_up(n, 2 * kOcThreads));
+    constexpr int kMaxKeep = 224 * 1024 / (4 * 8 * kOcThreads);
+    int keep = (int)std::min<int64_t>(kMaxKeep, div_up(n, (int64_t)nb * kOcThreads));
+    SF_CUDA(cudaMemsetAsync(x.slots, 0, kGridCommBytes, s));
+    void* args[] = {&n,      (void*)&rho, (void*)&dc, (void*)&dv, (void*)&vol_w, &target,
+                    &move,   &keep,       &rho_new,   &x,         &out};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)oc_bisect_kernel, dim3(nb), dim3(kOcThreads), args,
+                                                      sizeof(double) * 4 * (size_t)keep * kOcThreads, s);
+    done = !grid_refused(e);
+    if (done) {
+      SF_CUDA(e);
+      SF_CUDA(sf_launched(1));
+      SF_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
+      SF_CUDA(cudaStreamSynchronize(s));
+      if (h[3] != 0.0) throw std::runtime_error("simpfem_oc_update: a grid exchange ran out of its wait");
+    }
+  }
+  if (!done) oc_bisect_launched(n, rho, dc, dv, vol_w, target, move, rho_new, (double*)x.slots, out, s, h);
   if (change_host) *change_host = h[0];
   if (lambda_host) *lambda_host = h[1];
   if (steps_host) *steps_host = (int)h[2];

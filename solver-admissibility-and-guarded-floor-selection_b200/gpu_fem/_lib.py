@@ -83,7 +83,7 @@ class GmgProps(ctypes.Structure):
 
 
 class GridOpts(ctypes.Structure):
-    _fields_ = [("polls", ctypes.c_int), ("polls_first", ctypes.c_int)]
+    _fields_ = [("polls", ctypes.c_int), ("polls_first", ctypes.c_int), ("one_launch", ctypes.c_int)]
 
 
 class PolicyOpts(ctypes.Structure):
