@@ -14,7 +14,6 @@
 // Element index e = (i * ny + j) * nz + k.  Reductions are deterministic: every
 // block writes a partial, one block sums them in block order.
 #include <algorithm>
-#include <mutex>
 #include <stdexcept>
 
 #include "common.cuh"
@@ -28,13 +27,14 @@ namespace {
 constexpr int kMaxOff = 343;  // offsets within radius <= 3.5 in a 7^3 box
 constexpr int kSimpBlocks = 296, kSimpThreads = 256;
 
+// Neighbours within the radius: a kernel argument, so that calls of different radii on
+// other streams or from other threads do not meet.
 struct FilterOffsets {
-  int n;
-  int dx[kMaxOff], dy[kMaxOff], dz[kMaxOff];
   double w[kMaxOff];
+  int n;
+  int8_t dx[kMaxOff], dy[kMaxOff], dz[kMaxOff];
 };
-
-__constant__ FilterOffsets c_off;
+static_assert(sizeof(FilterOffsets) <= 3900, "kernel arguments");
 
 // y = H x (transpose = 0) or y = H^T x (transpose = 1); H symmetric in its
 // weights, so (H^T x)_e = sum over neighbours f of w(e, f) x_f / rowsum_f.
@@ -59,9 +59,9 @@ struct FilterTile {
 
 __device__ __forceinline__ int axis_code(int i, int n, int r) { return min(i, r) * (r + 1) + min(n - 1 - i, r); }
 
-__global__ void __launch_bounds__(kFilterThreads) cone_filter_kernel(int nx, int ny, int nz, FilterTile ft,
-                                                                     int transpose, const double* __restrict__ x,
-                                                                     double* __restrict__ y) {
+__global__ void __launch_bounds__(kFilterThreads) cone_filter_kernel(
+    const __grid_constant__ FilterOffsets nb, int nx, int ny, int nz, FilterTile ft, int transpose,
+    const double* __restrict__ x, double* __restrict__ y) {
   extern __shared__ __align__(16) double fsm[];
   const int r = ft.r, NC = (r + 1) * (r + 1), HY = ft.ty + 2 * r, HZ = ft.tz + 2 * r, HX = ft.tx + 2 * r;
   const int ntile = HX * HY * HZ;
@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(kFilterThreads) cone_filter_kernel(int nx, int
   int* off = reinterpret_cast<int*>(tile + ntile);
   const int bz = blockIdx.x % ft.bz, bq = blockIdx.x / ft.bz, by = bq % ft.by, bx = bq / ft.by;
   const int i0 = bx * ft.tx, j0 = by * ft.ty, k0 = bz * ft.tz;
-  for (int q = threadIdx.x; q < c_off.n; q += kFilterThreads)
-    off[q] = (c_off.dx[q] * HY + c_off.dy[q]) * HZ + c_off.dz[q];
+  for (int q = threadIdx.x; q < nb.n; q += kFilterThreads)
+    off[q] = (nb.dx[q] * HY + nb.dy[q]) * HZ + nb.dz[q];
   for (int c = threadIdx.x; c < NC * NC * NC; c += kFilterThreads) {
     const int cz = c % NC, cy = (c / NC) % NC, cx = c / (NC * NC);
     const int xa = cx / (r + 1), xb = cx % (r + 1), ya = cy / (r + 1), yb = cy % (r + 1), za = cz / (r + 1),
@@ -81,9 +81,9 @@ __global__ void __launch_bounds__(kFilterThreads) cone_filter_kernel(int nx, int
                         (za == r || zb == r || nz <= 2 * r);
     double s = 0.0;
     if (occurs)
-      for (int q = 0; q < c_off.n; ++q) {
-        const int dx = c_off.dx[q], dy = c_off.dy[q], dz = c_off.dz[q];
-        if (dx >= -xa && dx <= xb && dy >= -ya && dy <= yb && dz >= -za && dz <= zb) s += c_off.w[q];
+      for (int q = 0; q < nb.n; ++q) {
+        const int dx = nb.dx[q], dy = nb.dy[q], dz = nb.dz[q];
+        if (dx >= -xa && dx <= xb && dy >= -ya && dy <= yb && dz >= -za && dz <= zb) s += nb.w[q];
       }
     rs[c] = s;
   }
@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(kFilterThreads) cone_filter_kernel(int nx, int
     at[m] = ((lx + r) * HY + ly + r) * HZ + lz + r;
     acc[m] = 0.0;
   }
-  for (int q = 0; q < c_off.n; ++q) {
-    const double w = c_off.w[q];
+  for (int q = 0; q < nb.n; ++q) {
+    const double w = nb.w[q];
     const int o = off[q];
 #pragma unroll
     for (int m = 0; m < kFilterPer; ++m) acc[m] += w * tile[at[m] + o];
@@ -155,17 +155,16 @@ FilterTile filter_tile(int nx, int ny, int nz, int r) {
   return f;
 }
 
-cudaError_t launch_filter(int nx, int ny, int nz, double rmin, int transpose, const double* x, double* y,
+cudaError_t launch_filter(const FilterOffsets& nb, int nx, int ny, int nz, int transpose, const double* x, double* y,
                           cudaStream_t s) {
-  const int r = (int)floor(rmin);
-  const FilterTile f = filter_tile(nx, ny, nz, r);
+  const FilterTile f = filter_tile(nx, ny, nz, (int)floor(nb.w[0]));  // the element's own weight is the radius
   const size_t smem = filter_smem(f);
   static std::atomic<uint64_t> attr_done;
   const cudaError_t e = once_per_device(attr_done, [] {
     return cudaFuncSetAttribute(cone_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterSmem);
   });
   if (e != cudaSuccess) return e;
-  cone_filter_kernel<<<f.bx * f.by * f.bz, kFilterThreads, smem, s>>>(nx, ny, nz, f, transpose, x, y);
+  cone_filter_kernel<<<f.bx * f.by * f.bz, kFilterThreads, smem, s>>>(nb, nx, ny, nz, f, transpose, x, y);
   return sf_launched(1);
 }
 
@@ -434,9 +433,9 @@ FilterOffsets make_offsets(double rmin) {
         if (a == 0 && b == 0 && c == 0) continue;
         const double d = sqrt((double)(a * a + b * b + c * c));
         if (d > rmin - 1e-10) continue;
-        o.dx[o.n] = a;
-        o.dy[o.n] = b;
-        o.dz[o.n] = c;
+        o.dx[o.n] = (int8_t)a;
+        o.dy[o.n] = (int8_t)b;
+        o.dz[o.n] = (int8_t)c;
         o.w[o.n] = rmin - d;
         ++o.n;
       }
@@ -464,26 +463,6 @@ using namespace simpfem;
   }                                         \
   return SIMPFEM_OK;
 
-namespace {
-// the offsets live in constant memory, loaded when the radius or device changes
-// (one radius at a time: a call with a new radius must not overlap filter
-// launches of another radius on other streams)
-std::mutex g_filter_mutex;
-void set_filter(double rmin, cudaStream_t s) {
-  std::lock_guard<std::mutex> lk(g_filter_mutex);
-  static double cur = -1.0;
-  static int dev_set = -1;
-  int dev = 0;
-  SF_CUDA(cudaGetDevice(&dev));
-  if (cur == rmin && dev_set == dev) return;
-  const FilterOffsets o = make_offsets(rmin);
-  SF_CUDA(cudaMemcpyToSymbolAsync(c_off, &o, sizeof(o), 0, cudaMemcpyHostToDevice, s));
-  SF_CUDA(cudaStreamSynchronize(s));
-  cur = rmin;
-  dev_set = dev;
-}
-}  // namespace
-
 extern "C" {
 
 int simpfem_cone_filter(int nx, int ny, int nz, double rmin, int transpose, const double* x, double* y,
@@ -492,8 +471,7 @@ int simpfem_cone_filter(int nx, int ny, int nz, double rmin, int transpose, cons
   if (nx < 1 || ny < 1 || nz < 1 || !x || !y || x == y) throw InvalidArg{"simpfem_cone_filter: bad argument"};
   if (!(rmin >= 1.0 && rmin <= 3.5)) throw InvalidArg{"simpfem_cone_filter: rmin must be in [1, 3.5]"};
   cudaStream_t s = (cudaStream_t)stream;
-  set_filter(rmin, s);
-  SF_CUDA(launch_filter(nx, ny, nz, rmin, transpose ? 1 : 0, x, y, s));
+  SF_CUDA(launch_filter(make_offsets(rmin), nx, ny, nz, transpose ? 1 : 0, x, y, s));
   SIMP_API_END
 }
 
@@ -635,7 +613,7 @@ int simpfem_oc_update_projected(int nx, int ny, int nz, double rmin, const doubl
   if (!(beta > 1e-6)) throw InvalidArg{"simpfem_oc_update_projected: beta must exceed 1e-6 (else simpfem_oc_update)"};
   if (!(rmin >= 1.0 && rmin <= 3.5)) throw InvalidArg{"simpfem_oc_update_projected: rmin must be in [1, 3.5]"};
   cudaStream_t s = (cudaStream_t)stream;
-  set_filter(rmin, s);
+  const FilterOffsets around = make_offsets(rmin);
   double* dh = work;
   double* dcdh = dh + n;  // dc * dh, then reused for the filtered candidate
   double* dcd = dcdh + n;
@@ -648,8 +626,8 @@ int simpfem_oc_update_projected(int nx, int ny, int nz, double rmin, const doubl
   // sensitivities in the design space (simp_gpu.py:245-258): H^T (dc dh), H^T dh
   heaviside_kernel<<<eb, 256, 0, s>>>(n, rho_f, beta, eta, tbe, den, nullptr, dh, dc_phys, dcdh);
   SF_CUDA(sf_launched(1));
-  SF_CUDA(launch_filter(nx, ny, nz, rmin, 1, dcdh, dcd, s));
-  SF_CUDA(launch_filter(nx, ny, nz, rmin, 1, dh, dvd, s));
+  SF_CUDA(launch_filter(around, nx, ny, nz, 1, dcdh, dcd, s));
+  SF_CUDA(launch_filter(around, nx, ny, nz, 1, dh, dvd, s));
   double* rnf = dcdh;
   const int nb = (int)std::min<int64_t>(kSimpBlocks, div_up(n, kSimpThreads));
   const double target = volfrac * (double)n;
@@ -660,7 +638,7 @@ int simpfem_oc_update_projected(int nx, int ny, int nz, double rmin, const doubl
   for (int it = 0; it < 100; ++it) {
     lm = 0.5 * (l1 + l2);
     oc_candidate_kernel<<<nb, kSimpThreads, 0, s>>>(n, rho, dcd, dvd, lm, move, rn, partials);
-    SF_CUDA(launch_filter(nx, ny, nz, rmin, 0, rn, rnf, s));
+    SF_CUDA(launch_filter(around, nx, ny, nz, 0, rn, rnf, s));
     projected_sum_kernel<<<nb, kSimpThreads, 0, s>>>(n, rnf, beta, eta, tbe, partials);
     oc_finish_kernel<<<1, kSimpThreads, 0, s>>>(nb, 0, partials, out);
     SF_CUDA(sf_launched(3));
