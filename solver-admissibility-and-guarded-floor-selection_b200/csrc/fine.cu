@@ -71,10 +71,20 @@ void set_fine_constants(const double* ke576, const WhtBlocks& wb) {
         for (int c2 = 0; c2 < 3; ++c2)
           kem[(q * 3 + c) * 24 + q2 * 3 + c2] =
               ke576[(3 * kRefNodeOfCorner[q] + c) * 24 + 3 * kRefNodeOfCorner[q2] + c2];
-  // KE with bf16-rounded entries keeps the reflection symmetry (mirrored entries
-  // round alike), so it has Walsh blocks of its own
+  // KE with bf16-rounded entries has Walsh blocks of its own as long as mirrored entries
+  // round alike.  An accepted KE may be off its reflection symmetry by up to 1e-9, and
+  // entries on two sides of a rounding boundary would then part by 2^-8, terms that the
+  // blocks cannot hold: so the entries of corner 0 are rounded and mirrored.
   double keb[576];
-  for (int i = 0; i < 576; ++i) keb[i] = (double)__bfloat162float(__float2bfloat16_rn((float)ke576[i]));
+  for (int q = 0; q < 8; ++q)
+    for (int c = 0; c < 3; ++c)
+      for (int q2 = 0; q2 < 8; ++q2)
+        for (int c2 = 0; c2 < 3; ++c2) {
+          const bool odd = ((q & (4 >> c)) != 0) != ((q & (4 >> c2)) != 0);  // a component changes sign along its own axis
+          const double v = ke576[(3 * kRefNodeOfCorner[0] + c) * 24 + 3 * kRefNodeOfCorner[q ^ q2] + c2];
+          const double r = (double)__bfloat162float(__float2bfloat16_rn((float)v));
+          keb[(3 * kRefNodeOfCorner[q] + c) * 24 + 3 * kRefNodeOfCorner[q2] + c2] = odd ? -r : r;
+        }
   double boff = 0.0;
   const WhtBlocks wbb = make_wht_blocks(keb, &boff);
   double kd[24];
