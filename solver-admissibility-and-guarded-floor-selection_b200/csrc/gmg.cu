@@ -1401,6 +1401,7 @@ static void setup_coarsest(Gmg& G) {
 
 void gmg_setup(Gmg& G, const double* E, const double* fine_diag_free) {
   ++G.setup_epoch;  // captured cycles hold the previous setup's launch arguments
+  const Flying flying(true);
   Mesh& m = *G.m;
   const int64_t n = m.g.ndof;
   const int64_t ne = m.g.ne();

@@ -102,6 +102,19 @@ struct Mesh {
   }
 };
 
+// Hierarchy setups and outer solves that the process has in flight on a device: what the
+// choice between the two forms of an Arnoldi column goes by (arnoldi_one_launch; the
+// results do not depend on it).
+struct Flying {
+  int dev = 0;
+  bool counted = false;
+  explicit Flying(bool outer);
+  ~Flying();
+  Flying(const Flying&) = delete;
+  Flying& operator=(const Flying&) = delete;
+  int count() const;
+};
+
 struct KrylovWs {
   int restart = 0;
   int64_t n = 0;

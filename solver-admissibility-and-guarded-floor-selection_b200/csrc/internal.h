@@ -286,6 +286,7 @@ struct ColumnPlan {
 };
 size_t arnoldi_comm_bytes();
 ColumnPlan arnoldi_plan(int64_t n);
+bool arnoldi_one_launch(const ColumnPlan& p, int64_t n, int flying);
 // comm: arnoldi_comm_bytes() bytes zeroed once, serving one stream at a time
 cudaError_t launch_arnoldi(int64_t n, const KrylovDev& k, int j, const double* V, const double* w, double* vnew,
                            double tol, double* hist, int hist_cap, const ColumnPlan& p, void* comm,

@@ -17,6 +17,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <atomic>
 #include <vector>
 
 #include "gmg_impl.h"
@@ -28,12 +29,24 @@ static void kdots(const KrylovEnv& E, const DotSet& ds, double* out, const int* 
   SF_CUDA(launch_dots(F64, E.n, ds, E.rw, out, guard, E.st));
 }
 
+static std::atomic<int> g_flying[64];
+Flying::Flying(bool outer) {
+  SF_CUDA(cudaGetDevice(&dev));
+  counted = outer && dev < 64;
+  if (counted) g_flying[dev].fetch_add(1, std::memory_order_relaxed);
+}
+Flying::~Flying() {
+  if (counted) g_flying[dev].fetch_sub(1, std::memory_order_relaxed);
+}
+int Flying::count() const { return dev < 64 ? g_flying[dev].load(std::memory_order_relaxed) : 1; }
+
 void fgmres_core(const KrylovEnv& E, KrylovWs& K, const double* b, double* x, bool x0_zero, double tol,
                  int maxiter, int restart, const PrecFn& M, const int* parent, bool host_control, double* hist_dev,
                  int hist_cap, const CheckHook* check) {
   const int64_t n = E.n;
   cudaStream_t st = E.st;
   K.ensure(n, restart);
+  const Flying flying(host_control);
   KrylovDev& kd = K.kd;
   const int ld = restart + 1;
   {
@@ -73,7 +86,7 @@ void fgmres_core(const KrylovEnv& E, KrylovWs& K, const double* b, double* x, bo
       M(K.Vj(j), K.Zj(j), cyc);
       E.A(K.Zj(j), K.w.as<double>(), cyc);
       bool done = false;
-      if (K.plan.per > 0 && K.wait.one_launch) {
+      if (K.wait.one_launch && arnoldi_one_launch(K.plan, n, flying.count())) {
         const cudaError_t e = launch_arnoldi(n, kd, j, K.Vj(0), K.w.as<double>(), K.Vj(j + 1), tol, hist_dev, hist_cap,
                                              K.plan, K.comm.p, K.wait, st);
         done = !grid_refused(e);

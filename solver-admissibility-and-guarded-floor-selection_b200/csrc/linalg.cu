@@ -103,10 +103,7 @@ __global__ void __launch_bounds__(kRedThreads) dots_kernel(int64_t n, DotSet ds,
     for (int k = 0; k < ND; ++k) {
       const double t0 = dot_term<T>(ds, k, i), t1 = dot_term<T>(ds, k, i + stride);
       const double t2 = dot_term<T>(ds, k, i + 2 * stride), t3 = dot_term<T>(ds, k, i + 3 * stride);
-      v[k] += t0;
-      v[k] += t1;
-      v[k] += t2;
-      v[k] += t3;
+      v[k] = add_rn(add_rn(add_rn(add_rn(v[k], t0), t1), t2), t3);  // arnoldi_kernel repeats this rounding
     }
   }
   for (; i < n; i += stride) {
@@ -672,13 +669,13 @@ __global__ void __launch_bounds__(kRedThreads) mgs_step_kernel(int64_t n, const 
     for (int q = 0; q < 4; ++q) {
       const double wn = sub_rn(wv[q], mul_rn(h, vv[q]));
       w[i + q * stride] = wn;
-      v[0] += (vnext != nullptr ? nv[q] : wn) * wn;
+      v[0] = fma(vnext != nullptr ? nv[q] : wn, wn, v[0]);
     }
   }
   for (; i < n; i += stride) {
     const double wn = sub_rn(w[i], mul_rn(h, vi[i]));
     w[i] = wn;
-    v[0] += (vnext != nullptr ? vnext[i] : wn) * wn;
+    v[0] = fma(vnext != nullptr ? vnext[i] : wn, wn, v[0]);
   }
   block_sum<1>(v, sh);
   last_block_finalize<1>(v, rw, out);
@@ -797,9 +794,9 @@ __global__ void givens_kernel(KrylovDev k, int j, double tol, double* hist, int 
 // exchange of the step before (WSMEM: twice, through L2), and the step is that one
 // exchange.  The block that gathers the exchanges is the one that rotates.
 //
-// The sums are the launched kernels' to the last bit (nested solves and FP32 cycles
-// amplify a difference of 1e-16 beyond 1e-9 of the solution): the vectors are split
-// into the same parts, part p owning the elements p * kRedThreads + t, + parts *
+// The sums are the launched kernels' to the last bit, so a solve may take either form
+// from column to column (nested solves and FP32 cycles amplify a difference of 1e-16
+// beyond 1e-9 of the solution): the vectors are split into the same parts, part p owning the elements p * kRedThreads + t, + parts *
 // kRedThreads, ..., and one chain adds the parts in order (1.2 us of an exchange's
 // 3).  A block holds 2 * MP parts; MP is chosen for about eight elements a thread,
 // because fewer blocks exchange faster and leave SMs to other streams (45 x 30 x 30,
@@ -830,6 +827,12 @@ __global__ void __launch_bounds__(kColThreads, 1)
     const int base = first + m * kColThreads;
     const int e = base + q * stride;
     return base < stride && e < len ? e : len;
+  };
+  // <v_0, w> is dots_kernel's sum: products rounded by themselves where a thread has four
+  // elements of a pass, fused with the addition behind the last such pass
+  auto first_dot = [&](double acc, double a, double b, int m, int q) -> double {
+    const bool pass = (int64_t)first + m * kColThreads + (int64_t)(q / 4 * 4 + 3) * stride < len;
+    return pass ? add_rn(acc, mul_rn(a, b)) : fma(a, b, acc);
   };
   unsigned epoch = *(volatile unsigned*)x.last;
   double wr[NE];
@@ -890,7 +893,7 @@ __global__ void __launch_bounds__(kColThreads, 1)
       const int e = element(0, q);
       const double x = e < len ? w[e] : 0.0;
       csm[q * kColThreads + tid] = x;
-      if (e < len) part[0] = fma(V[e], x, part[0]);
+      if (e < len) part[0] = first_dot(part[0], V[e], x, 0, q);
     }
   } else {
     fetch(0);
@@ -907,7 +910,8 @@ __global__ void __launch_bounds__(kColThreads, 1)
 #pragma unroll
     for (int m = 0; m < MP; ++m)
 #pragma unroll
-      for (int q = 0; q < PER; ++q) part[m] = fma(csm[(m * PER + q) * kColThreads + tid], wr[m * PER + q], part[m]);
+      for (int q = 0; q < PER; ++q)
+        part[m] = first_dot(part[m], csm[(m * PER + q) * kColThreads + tid], wr[m * PER + q], m, q);
   }
   bool ok = grid_sum(part, h);
   for (int i = 0; ok && i <= j; ++i) {
@@ -942,6 +946,7 @@ __global__ void __launch_bounds__(kColThreads, 1)
     }
     ok = grid_sum(part, h);
   }
+  asm volatile("cp.async.wait_group 0;\n" ::);  // copies of a loop that a failed exchange ended
   const double hn = sqrt(h);  // h = <w, w>
   if (ok) {
     if constexpr (WSMEM) {
@@ -987,6 +992,23 @@ static GridExchange grid_exchange(void* comm, const GridWait& wait) {
 
 size_t arnoldi_comm_bytes() { return kGridCommBytes + 16; }
 
+// Whether a column of one of `flying` setups and solves takes the one launch.  Its blocks must all be
+// resident at once, so solves in flight queue for the SMs, which costs more than the
+// launches it saves once they ask for more than twice as many blocks as there are; with
+// vectors beyond a million unknowns, whose blocks stay longest, as soon as there are two.
+// Milliseconds a state, one launch against launched, mixed solves:
+//   unknowns (blocks)   alone          2 in flight   4 in flight   8 in flight
+//   132,618    (37)     4.8 / 5.2                                  1.36 / 1.48
+//   209,223    (74)     4.4 / 4.8      2.57 / 2.81   1.75 / 1.90   1.4 / 1.4
+//   450,765   (148)     5.2 / 5.7      3.53 / 3.9    2.67 / 2.52   2.5 / 2.1
+//   686,433   (148)     6.9 / 7.8                                  3.6 / 3.1
+//   1,610,739 (148)     8.25 / 8.72    6.3 / 6.06    5.7 / 4.9     5.65 / 4.67
+// Both forms add in the same order: the choice changes no bit.
+bool arnoldi_one_launch(const ColumnPlan& p, int64_t n, int flying) {
+  if (p.per == 0) return false;
+  return flying <= 1 || (n <= 1000000 && (int64_t)flying * p.blocks <= 2 * grid_sm_count());
+}
+
 struct ColumnKernel {
   const void* fn;
   int elements;  // a thread
@@ -1024,10 +1046,6 @@ static cudaError_t column_attributes() {
 ColumnPlan arnoldi_plan(int64_t n) {
   ColumnPlan p;
   if (n < 1) return p;
-  // Longer vectors take every SM, and eight solves in flight then wait for all of them at
-  // once: 512k elements (1.6 M unknowns) ran 173 batched solves/s with one launch a column
-  // against 186-198 launched step by step; one solve alone gains about 3 %.
-  if (n > 1000000) return p;
   const int parts = red_blocks(n);
   const int64_t per = div_up(n, (int64_t)parts * kRedThreads);
   if (per * kColThreads * 8 > 216 * 1024) return p;
