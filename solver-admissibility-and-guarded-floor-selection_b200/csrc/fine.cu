@@ -159,9 +159,9 @@ __device__ __forceinline__ float2 zbutterfly(float2 a) { return make_float2(__fa
 __device__ __forceinline__ float2 swap2(float2 a) { return make_float2(a.y, a.x); }
 
 // The eight blocks: w[c][2 sx + sy] (component 2 swapped) -> v in the same layout.
-// RN: each row is product, fused multiply-add, fused multiply-add; otherwise the
-// order that contracting c0 in0 + c1 in1 + c2 in2 from the left gives.
-template <bool RN, bool BF>
+// A row is a product and two fused multiply-adds; the element form begins with the
+// second term, the face form with the first.
+template <bool FACES, bool BF>
 __device__ __forceinline__ void blocks2(const float2 (&w)[3][4], float2 (&v)[3][4]) {
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
@@ -170,7 +170,7 @@ __device__ __forceinline__ void blocks2(const float2 (&w)[3][4], float2 (&v)[3][
     for (int r = 0; r < 3; ++r) {
       const float2* c = BF ? c_whtb32[h] : c_wht32[h];
       float2 a;
-      if (RN) {
+      if (FACES) {
         a = __fmul2_rn(c[3 * r], in0);
         a = __ffma2_rn(c[3 * r + 1], in1, a);
       } else {
@@ -184,9 +184,7 @@ __device__ __forceinline__ void blocks2(const float2 (&w)[3][4], float2 (&v)[3][
 }
 
 // f = E * KE * u for one element: lo and hi are its faces at dx = 0 and 1, node pairs
-// [component][dy].  RN: every operation is rounded by itself; otherwise the modulus
-// is contracted into the first back-transform butterfly.
-template <bool RN>
+// [component][dy].  The modulus is contracted into the first back-transform butterfly.
 __device__ __forceinline__ void element_product2(const float2 (&ulo)[3][2], const float2 (&uhi)[3][2], float E,
                                                  float2 (&flo)[3][2], float2 (&fhi)[3][2]) {
   float2 w[3][4], v[3][4];
@@ -203,7 +201,7 @@ __device__ __forceinline__ void element_product2(const float2 (&ulo)[3][2], cons
       for (int s = 0; s < 4; ++s) w[q][s] = swap2(w[q][s]);
     }
   }
-  blocks2<RN, false>(w, v);
+  blocks2<false, false>(w, v);
   const float2 E2 = make_float2(E, E);
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
@@ -211,14 +209,8 @@ __device__ __forceinline__ void element_product2(const float2 (&ulo)[3][2], cons
 #pragma unroll
     for (int y = 0; y < 2; ++y) {
       const float2 r = __fmul2_rn(E2, v[q][2 + y]);
-      if (RN) {
-        const float2 p = __fmul2_rn(E2, v[q][y]);
-        s[y] = add2(p, r);
-        d[y] = sub2(p, r);
-      } else {
-        s[y] = __ffma2_rn(E2, v[q][y], r);
-        d[y] = __ffma2_rn(E2, v[q][y], make_float2(-r.x, -r.y));
-      }
+      s[y] = __ffma2_rn(E2, v[q][y], r);
+      d[y] = __ffma2_rn(E2, v[q][y], make_float2(-r.x, -r.y));
     }
     const float2 a0 = add2(s[0], s[1]), a1 = sub2(s[0], s[1]), b0 = add2(d[0], d[1]), b1 = sub2(d[0], d[1]);
     flo[q][0] = zbutterfly(q == 2 ? swap2(a0) : a0);
@@ -306,7 +298,7 @@ __device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.a
 // One face of an element column at a node plane (12 values): with FORM kFaces
 // transformed along z and y -- v[component][2 a + b], a the y and b the z parity
 // (FP32: component 2 with b swapped) --, else its node values v[component][2 dy + dz].
-enum SweepForm { kFaces = 0, kElementRn = 1, kElement = 2 };
+enum SweepForm { kFaces = 0, kElement = 1 };
 
 template <bool BF, int FORM>
 __device__ __forceinline__ void face_values(const double* r0, const double* r1, double (&v)[3][4], double (&own)[3]) {
@@ -428,7 +420,7 @@ __device__ __forceinline__ void element_faces(const float (&p)[3][4], const floa
         h[q][y] = __ffma2_rn(E2, v[q][y], make_float2(-r.x, -r.y));
       }
   } else {
-    element_product2<FORM == kElementRn>(a, b, E, l, h);
+    element_product2(a, b, E, l, h);
   }
 #pragma unroll
   for (int q = 0; q < 3; ++q)
@@ -574,18 +566,13 @@ constexpr int sweep_resident() { return sizeof(T) == 8 ? (FORM == kFaces && DENS
 // and the hierarchy's own FP64 operator -- keep the element-by-element evaluation
 // instead: FP32 cycles turn a difference of 1e-16 in a Krylov vector into 1e-8 of the
 // displacement of nodes that hang in void alone, the nested Krylov solves of the FP64
-// stacks into 1e-9 of all of it, and their answers are to stay the same to the last
-// bit.  FP32 has two such forms, by grid size (launch_sweep): the compiler's
-// contraction of the plain expressions up to kFusedElements, every operation rounded
-// by itself beyond.  They take about 1.4 times the arithmetic of kFaces.
+// stacks into 1e-9 of all of it.  It takes about 1.4 times the arithmetic of kFaces.
 //
 // COMPACT: u and y are the free-DOF vectors of the C interface, so neither an
 // expanded copy of u nor a full result is written.  pinfo[plane] is the free index
 // of the first DOF of a node plane that is wholly free -- its values then lie as in
 // the full layout --, -1 otherwise; on those planes (supports) ninfo[node] gives 8 *
 // (free index of the node's first free DOF) + its three free bits.
-constexpr int64_t kFusedElements = 250000;
-
 template <typename T, int EPI, bool DENSE, bool BF, bool COMPACT, int FORM>
 __global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE, FORM>())
     sweep_kernel(Grid g, SweepShape sh, const T* __restrict__ E, const uint8_t* __restrict__ nmask,
@@ -828,11 +815,8 @@ static cudaError_t launch_sweep(const Grid& g, const SweepShape& sh, const void*
                                                                    nullptr, ea, s);
   }
   if constexpr (sizeof(T) == 4 && !BF && EPI != EPI_APPLY) {
-    return g.ne() <= kFusedElements
-               ? launch_sweep_as<T, EPI, true, false, false, kElement>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
-                                                                       nullptr, ea, s)
-               : launch_sweep_as<T, EPI, true, false, false, kElementRn>(g, sh, (const T*)E, nmask, (const T*)u,
-                                                                         nullptr, nullptr, ea, s);
+    return launch_sweep_as<T, EPI, true, false, false, kElement>(g, sh, (const T*)E, nmask, (const T*)u, nullptr,
+                                                                 nullptr, ea, s);
   } else if constexpr (sizeof(T) == 4) {
     return launch_sweep_as<T, EPI, true, BF, false, kFaces>(g, sh, (const T*)E, nmask, (const T*)u, nullptr, nullptr,
                                                             ea, s);
