@@ -501,8 +501,7 @@ constexpr int epi_operands() {
 }
 
 // The epilogues of one node: operands o[0..2] = b, o[3..5] = dinv, o[6..8] = d,
-// staged by the thread itself; evaluates epilogue()'s expressions.  off: first DOF
-// of the node, fr its free bits.
+// staged by the thread itself.  off: first DOF of the node, fr its free bits.
 template <typename T, int EPI>
 __device__ __forceinline__ void node_epilogue(const EpiArgs& ea, int64_t off, unsigned fr, const T* o, const T (&ku)[3],
                                               const T (&x)[3]) {

@@ -543,20 +543,13 @@ void level_op(Gmg& G, int l, DType vt, int precsel, Epi epi, const void* u, EpiA
     return;
   }
   Level& L = G.lv[l];
-  DType ct = F64;
-  const void* coef = L.K64.p;
-  if (vt == F32) {
-    if (precsel == BF16 && L.K16.p) {
-      // BF16 copy node-major by neighbour column, nine lanes per node
-      SF_CUDA(launch_stencil_col_bf16(epi, L.g, L.K16.as<__nv_bfloat16>(), L.mask.as<uint8_t>(), (const float*)u,
-                                      ea, G.st));
-      return;
-    } else {
-      ct = F32;
-      coef = L.K32.p;
-    }
+  if (vt == F32 && precsel == BF16 && L.K16.p) {
+    // BF16 copy node-major by neighbour column, nine lanes per node
+    SF_CUDA(launch_stencil_col_bf16(epi, L.g, L.K16.as<__nv_bfloat16>(), L.mask.as<uint8_t>(), (const float*)u, ea,
+                                    G.st));
+    return;
   }
-  SF_CUDA(launch_stencil(vt, ct, epi, L.g, coef, L.mask.as<uint8_t>(), u, ea, G.st));
+  SF_CUDA(launch_stencil(vt, epi, L.g, vt == F32 ? L.K32.p : L.K64.p, L.mask.as<uint8_t>(), u, ea, G.st));
 }
 
 const void* level_dinv(Gmg& G, int l, DType t) {
@@ -1184,7 +1177,7 @@ static void fixed_pcg_coarse(Gmg& G, int l, const double* b, double* x) {
     EpiArgs ea;
     ea.y = Ap;
     ea.guard = G.guard;
-    SF_CUDA(launch_stencil(F64, F64, EPI_APPLY, L.g, L.K64.p, L.mask.as<uint8_t>(), p, ea, G.st));
+    SF_CUDA(launch_stencil(F64, EPI_APPLY, L.g, L.K64.p, L.mask.as<uint8_t>(), p, ea, G.st));
     DotSet dp;
     dp.a[0] = p; dp.b[0] = Ap; dp.nd = 1;
     dots(G, F64, n, dp, sc + 1, G.guard);
@@ -1309,7 +1302,7 @@ static double sparse_lambda(Gmg& G, int l) {
   for (int it = 0; it < 10; ++it) {
     EpiArgs ea;
     ea.y = Kv;
-    SF_CUDA(launch_stencil(F64, F64, EPI_APPLY, L.g, L.K64.p, mask, v, ea, G.st));
+    SF_CUDA(launch_stencil(F64, EPI_APPLY, L.g, L.K64.p, mask, v, ea, G.st));
     SF_CUDA(launch_vec_op(n, 3, Kv, dinv, nullptr, 0.0, nullptr, Av, G.st));
     DotSet d;
     d.a[0] = v; d.b[0] = Kv;

@@ -168,8 +168,8 @@ size_t stencil_colmajor_bytes(int64_t nn);
 cudaError_t launch_stencil_colmajor_bf16(int64_t nn, const double* K64, __nv_bfloat16* out, cudaStream_t s);
 cudaError_t launch_stencil_col_bf16(Epi epi, const Grid& g, const __nv_bfloat16* coefC, const uint8_t* mask,
                                     const float* u, const EpiArgs& ea, cudaStream_t s);
-cudaError_t launch_stencil(DType vt, DType ct, Epi epi, const Grid& g, const void* coef,
-                           const uint8_t* mask, const void* u, const EpiArgs& ea, cudaStream_t s);
+cudaError_t launch_stencil(DType t, Epi epi, const Grid& g, const void* coef, const uint8_t* mask, const void* u,
+                           const EpiArgs& ea, cudaStream_t s);
 cudaError_t launch_level1_assemble(const Grid& gc, const Grid& gf, const double* E_fine,
                                    const double* Q /*8*576*/, const uint8_t* mask_c, double* coef,
                                    cudaStream_t s);

@@ -26,15 +26,6 @@ __device__ __forceinline__ int64_t node_id(const Grid& g, int i, int j, int k) {
   return ((int64_t)i * (g.ny + 1) + j) * (g.nz + 1) + k;
 }
 
-template <typename VT, typename CT>
-__device__ __forceinline__ VT coef_to(CT c) {
-  return (VT)to_d(c);
-}
-template <>
-__device__ __forceinline__ float coef_to<float, __nv_bfloat16>(__nv_bfloat16 c) {
-  return __bfloat162float(c);
-}
-
 // Unsigned division by an invariant d >= 1 for dividends below 2^31: one multiply
 // instead of the twenty instructions of an integer division.
 struct FastDiv {
@@ -76,9 +67,9 @@ __device__ __forceinline__ void node_ijk(const Grid& g, const FastDiv& dz, const
 // 3 * nn < 2^31).
 constexpr int kStencilNodes = 32, kStencilThreads = 9 * 32;
 
-template <typename VT, typename CT, int EPI>
+template <typename VT, int EPI>
 __global__ void __launch_bounds__(kStencilThreads) stencil_kernel(Grid g, FastDiv dz, FastDiv dy,
-                                                                  const CT* __restrict__ coef,
+                                                                  const VT* __restrict__ coef,
                                                                   const uint8_t* __restrict__ mask,
                                                                   const VT* __restrict__ u, EpiArgs ea) {
   if (guard_off(ea.guard)) return;
@@ -101,8 +92,8 @@ __global__ void __launch_bounds__(kStencilThreads) stencil_kernel(Grid g, FastDi
   const int ox = col / 3, oy = col - 3 * ox;
   const int sx = ox == 0 ? (i > 0 ? -NY1 * NZ1 : 0) : (ox == 2 ? (i < g.nx ? NY1 * NZ1 : 0) : 0);
   const int sy = oy == 0 ? (j > 0 ? -NZ1 : 0) : (oy == 2 ? (j < g.ny ? NZ1 : 0) : 0);
-  const CT* cp = coef + (int64_t)(col * 27) * nn + n;
-  CT cf[27];
+  const VT* cp = coef + (int64_t)(col * 27) * nn + n;
+  VT cf[27];
 #pragma unroll
   for (int e = 0; e < 27; ++e) cf[e] = cp[(int64_t)e * nn];
   VT uv[9];
@@ -119,7 +110,7 @@ __global__ void __launch_bounds__(kStencilThreads) stencil_kernel(Grid g, FastDi
       for (int r = 0; r < 3; ++r) {
         VT acc = c > 0 ? part[3 * nl + r] : VT(0);
 #pragma unroll
-        for (int e = 0; e < 9; ++e) acc = fma(coef_to<VT, CT>(cf[e / 3 * 9 + r * 3 + e % 3]), uv[e], acc);
+        for (int e = 0; e < 9; ++e) acc = fma(cf[e / 3 * 9 + r * 3 + e % 3], uv[e], acc);
         part[3 * nl + r] = acc;
       }
     }
@@ -147,32 +138,29 @@ __global__ void __launch_bounds__(kStencilThreads) stencil_kernel(Grid g, FastDi
   if (EPI == EPI_CHEB1 || EPI == EPI_CHEB) ((VT*)ea.d)[dof] = f ? dn : VT(0);
 }
 
-template <typename VT, typename CT>
+template <typename VT>
 static cudaError_t stencil_dispatch(Epi epi, const Grid& g, const void* coef, const uint8_t* mask,
                                     const void* u, const EpiArgs& ea, cudaStream_t s) {
   if (3 * g.nn >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
   const int bs = kStencilThreads, nb = div_up(g.nn, kStencilNodes);
   const FastDiv dz = FastDiv::make(g.nz + 1), dy = FastDiv::make(g.ny + 1);
-  const CT* c = (const CT*)coef;
+  const VT* c = (const VT*)coef;
   const VT* uu = (const VT*)u;
   switch (epi) {
-    case EPI_APPLY: stencil_kernel<VT, CT, EPI_APPLY><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
-    case EPI_RESID: stencil_kernel<VT, CT, EPI_RESID><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
-    case EPI_CHEB1: stencil_kernel<VT, CT, EPI_CHEB1><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
-    case EPI_CHEB: stencil_kernel<VT, CT, EPI_CHEB><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
-    case EPI_JAC: stencil_kernel<VT, CT, EPI_JAC><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_APPLY: stencil_kernel<VT, EPI_APPLY><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_RESID: stencil_kernel<VT, EPI_RESID><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_CHEB1: stencil_kernel<VT, EPI_CHEB1><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_CHEB: stencil_kernel<VT, EPI_CHEB><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
+    case EPI_JAC: stencil_kernel<VT, EPI_JAC><<<nb, bs, 0, s>>>(g, dz, dy, c, mask, uu, ea); break;
     default: return cudaErrorInvalidValue;
   }
   return sf_launched(1);
 }
 
-cudaError_t launch_stencil(DType vt, DType ct, Epi epi, const Grid& g, const void* coef,
-                           const uint8_t* mask, const void* u, const EpiArgs& ea, cudaStream_t s) {
-  if (vt == F64 && ct == F64) return stencil_dispatch<double, double>(epi, g, coef, mask, u, ea, s);
-  if (vt == F32 && ct == F32) return stencil_dispatch<float, float>(epi, g, coef, mask, u, ea, s);
-  if (vt == F32 && ct == BF16)
-    return stencil_dispatch<float, __nv_bfloat16>(epi, g, coef, mask, u, ea, s);
-  if (vt == F64 && ct == F32) return stencil_dispatch<double, float>(epi, g, coef, mask, u, ea, s);
+cudaError_t launch_stencil(DType t, Epi epi, const Grid& g, const void* coef, const uint8_t* mask, const void* u,
+                           const EpiArgs& ea, cudaStream_t s) {
+  if (t == F64) return stencil_dispatch<double>(epi, g, coef, mask, u, ea, s);
+  if (t == F32) return stencil_dispatch<float>(epi, g, coef, mask, u, ea, s);
   return cudaErrorInvalidValue;
 }
 
