@@ -491,11 +491,11 @@ def run_native(args):
     # the FP64 operator product of every FGMRES iteration and of the guard
     avg64 = ctypes.c_float()
     _lib.call("simpfem_gmg_time_operator", fp64.gmg._h, 50, ctypes.byref(avg64), _lib.stream_ptr())
-    op_bytes = 8 * ne + 2 * 8 * ndof + ndof  # read E and u, write y (FP64), 1-byte DOF mask
+    op_bytes = 8 * ne + 2 * 8 * ndof + ndof // 3  # read E and u, write y (FP64), 1-byte node mask
     op_flops = 1152 * ne                     # 2 x 24 x 24 per element, the reference's convention
-    # fp32 vectors read u, rhs, dinv (plus d for Chebyshev) and write x (plus d); E (fp32); 1-byte DOF mask
+    # fp32 vectors read u, rhs, dinv (plus d for Chebyshev) and write x (plus d); E (fp32); 1-byte node mask
     nvec = 4 if args.stack == "plain" else 6
-    alg_bytes = nvec * 4 * ndof + 4 * ne + ndof
+    alg_bytes = nvec * 4 * ndof + 4 * ne + ndof // 3
     achieved = alg_bytes / (avg.value * 1e-3) / 1e9
     traffic = _traffic_per_launch().get(f"fine_step_{args.stack}_mixed")
     result = {

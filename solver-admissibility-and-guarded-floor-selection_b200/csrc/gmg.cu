@@ -234,9 +234,10 @@ static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
   return us;
 }
 
-// Candidate tiles of a grid: the z extent in one to four equal parts, blocks of up to
-// 256, 128 or 64 threads filled with equal parts of the y extent, cx node planes a
-// block (the halo column and the halo plane make each part one element larger).
+// Candidate tiles of a grid: the z extent in as few equal parts as two rows of 64 threads
+// take up to four (one more than the fewest on longer rows), blocks of up to 128, 96 or 64
+// threads filled with equal parts of the y extent, cx node planes a block (the halo column
+// and the halo plane make each part one element larger).
 // Depths along x: a doubling series for the model to choose from; all of them, each
 // number of parts once, for the tuner (every), because the wave count hangs on it.
 static std::vector<SweepShape> sweep_candidates(DType t, const Grid& g, bool every) {
@@ -1582,8 +1583,8 @@ float time_fine_operator(Gmg& G, int reps) {
   SF_CUDA(launch_fill_hash(F64, n, 21u, u, G.st));
   EpiArgs ea;
   ea.y = y;
-  fine_apply(*G.m, F64, EPI_APPLY, G.E64.p, u, ea, G.st);
-  return time_cold([&]() { fine_apply(*G.m, F64, EPI_APPLY, G.E64.p, u, ea, G.st); }, reps, G.st);
+  fine_apply64(G, EPI_APPLY, u, ea, G.st);
+  return time_cold([&]() { fine_apply64(G, EPI_APPLY, u, ea, G.st); }, reps, G.st);
 }
 
 // Outer FGMRES: host-controlled (one synchronisation per iteration to read the
