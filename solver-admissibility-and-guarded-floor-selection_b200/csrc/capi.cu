@@ -180,6 +180,9 @@ int simpfem_mesh_create(int nelx, int nely, int nelz, const int32_t* free_dofs_h
       SF_CUDA(cudaMemcpy(m.ninfo.p, info.data(), 4 * m.g.nn, cudaMemcpyHostToDevice));
       SF_CUDA(cudaMemcpy(m.pinfo.p, planes.data(), 4 * planes.size(), cudaMemcpyHostToDevice));
     }
+    // a copy from pageable memory may return before its last bytes have arrived; the
+    // operator takes addresses from these tables on whatever stream it is called
+    SF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   }
   m.init_red();
   m.sh[0] = default_shape(F64, m.g);

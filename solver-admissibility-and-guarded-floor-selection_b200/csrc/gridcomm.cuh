@@ -4,7 +4,8 @@
 // Every block publishes its part of a sum as two 64-bit words, each holding 32
 // bits of the value and the 32-bit number of the exchange; a reader polls the
 // words until they carry that number, so a value and its arrival are one load
-// and no counter, fence or second read is needed.  Up to kGridFlat blocks each
+// and no counter, fence or second read is needed (data and flag in one word, as in the
+// low-latency "LL" protocol of NCCL).  Up to kGridFlat blocks each
 // block reads all parts; beyond that block 0 reads them and publishes the sum in
 // a few copies for the others, because the polls of every block on every part
 // load the L2 slices that hold them (one value, with the block-wide sum before

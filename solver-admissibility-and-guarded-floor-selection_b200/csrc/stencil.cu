@@ -27,7 +27,8 @@ __device__ __forceinline__ int64_t node_id(const Grid& g, int i, int j, int k) {
 }
 
 // Unsigned division by an invariant d >= 1 for dividends below 2^31: one multiply
-// instead of the twenty instructions of an integer division.
+// instead of the twenty instructions of an integer division (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994, figure 4.1).
 struct FastDiv {
   unsigned d = 1, mul = 0, shift = 0;
   static FastDiv make(unsigned d) {
