@@ -320,17 +320,24 @@ __device__ __forceinline__ void face_values(const double* r0, const double* r1, 
     v[q][3] = d0 - d1;
   }
 }
+// a pair of operands, which the BF16 operator rounds (one conversion for both)
 template <bool BF>
-__device__ __forceinline__ float operand(float v) {  // the BF16 operator rounds its operands
-  return BF ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+__device__ __forceinline__ float2 operands(float x, float y) {
+  if constexpr (BF) {
+    unsigned p;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(y), "f"(x));  // y in the upper half
+    return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+  } else {
+    return make_float2(x, y);
+  }
 }
 template <bool BF, int FORM>
 __device__ __forceinline__ void face_values(const float* r0, const float* r1, float (&v)[3][4], float (&own)[3]) {
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     own[q] = r0[q];
-    const float2 a = make_float2(operand<BF>(own[q]), operand<BF>(r0[3 + q]));
-    const float2 b = make_float2(operand<BF>(r1[q]), operand<BF>(r1[3 + q]));
+    const float2 a = operands<BF>(own[q], r0[3 + q]);
+    const float2 b = operands<BF>(r1[q], r1[3 + q]);
     float2 p = a, m = b;
     if (FORM == kFaces) {
       p = zbutterfly(add2(a, b));
@@ -471,26 +478,39 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   const float t = __fsub_rn(s, a);
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
 }
+__device__ __forceinline__ void two_sum(float2 a, float2 b, float2& s, float2& e) {
+  s = add2(a, b);
+  const float2 t = sub2(s, a);
+  e = add2(sub2(a, sub2(s, t)), sub2(b, t));
+}
 // A node's sum over its four face corners: its own thread's, the z and y neighbours'
 // and the diagonal one's.  The element forms keep the order that the solves' bits rest
 // on; kFaces adds in pairs, which rounds smaller sums (relative 2-norm against 64 bits,
 // FP32 at 512k elements: 6.04e-8, one after the other 6.19e-8, element by element 6.13e-8).
 // The BF16 operator also adds what these three additions lose and transforms its faces
 // back element by element (sweep_kernel): 4.35e-8, where faces summed first gave 5.31e-8
-// and a dense product of the rounded matrix gives 4.56e-8, for 61.7 us at 2M elements
+// and a dense product of the rounded matrix gives 4.56e-8, for 59.7 us at 2M elements
 // against 55.6.
 template <bool BF, int FORM, typename T>
-__device__ __forceinline__ T corner_sum(T own, T z, T y, T yz) {
+__device__ __forceinline__ void corner_sums(const T (&own)[3], const T* z, const T* y, const T* yz, T (&ku)[3]) {
   if constexpr (BF) {
-    T a, b, s, ea, eb, e;
-    two_sum(own, z, a, ea);
-    two_sum(y, yz, b, eb);
-    two_sum(a, b, s, e);
-    return add_rn(s, add_rn(add_rn(ea, eb), e));
-  } else if constexpr (FORM == kFaces) {
-    return add_rn(add_rn(own, z), add_rn(y, yz));
+    float2 s[3], e[3];  // pairs: (own + y, z + yz)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) two_sum(make_float2(own[q], z[q]), make_float2(y[q], yz[q]), s[q], e[q]);
+    float2 s01, e01;
+    two_sum(make_float2(s[0].x, s[1].x), make_float2(s[0].y, s[1].y), s01, e01);
+    const float2 l01 = add2(add2(make_float2(e[0].x, e[1].x), make_float2(e[0].y, e[1].y)), e01);
+    const float2 k01 = add2(s01, l01);
+    ku[0] = k01.x;
+    ku[1] = k01.y;
+    float s2, e2;
+    two_sum(s[2].x, s[2].y, s2, e2);
+    ku[2] = add_rn(s2, add_rn(add_rn(e[2].x, e[2].y), e2));
   } else {
-    return add_rn(add_rn(add_rn(own, y), z), yz);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      ku[q] = FORM == kFaces ? add_rn(add_rn(own[q], z[q]), add_rn(y[q], yz[q]))
+                             : add_rn(add_rn(add_rn(own[q], y[q]), z[q]), yz[q]);
   }
 }
 
@@ -750,8 +770,7 @@ __global__ void __launch_bounds__(kSweepThreads, sweep_resident<T, DENSE, FORM>(
       const T* bz = buf - 9;
       const T* by = buf - 9 * sh.bk;
       T ku[3];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) ku[q] = corner_sum<BF, FORM>(f0[q], bz[q], by[3 + q], by[6 + q - 9]);
+      corner_sums<BF, FORM>(f0, bz, by + 3, by + 6 - 9, ku);
       if constexpr (COMPACT) {
         if (bits >= 0) {
           T* py = (T*)ea.y + bits + 3 * (je * NZ1 + ke);
