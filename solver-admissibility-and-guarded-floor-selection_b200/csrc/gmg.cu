@@ -234,6 +234,13 @@ static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
   return us;
 }
 
+// Warps times node planes that a sweep issues, halos included.
+static int64_t sweep_work(const Grid& g, const SweepShape& sh) {
+  const int64_t blocks =
+      div_up64(g.ny + 1, sh.bj - 1) * div_up64(g.nz + 1, sh.bk - 1) * div_up64(g.nx + 1, sh.cx);
+  return blocks * div_up64((int64_t)sh.bj * sh.bk, 32) * (sh.cx + 1);
+}
+
 // Candidate tiles of a grid: the z extent in as few equal parts as two rows of 64 threads
 // take up to four (one more than the fewest on longer rows), blocks of up to 128, 96 or 64
 // threads filled with equal parts of the y extent, cx node planes a block (the halo column
@@ -341,8 +348,7 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
   cudaEvent_t e0, e1;
   SF_CUDA(cudaEventCreate(&e0));
   SF_CUDA(cudaEventCreate(&e1));
-  float best = 1e30f;
-  SweepShape best_sh = default_shape(t, m.g);
+  std::vector<float> time(cands.size(), 1e30f);
   // SIMPFEM_TUNE_VERBOSE=1 prints every candidate's time (stderr)
   const char* vb = getenv("SIMPFEM_TUNE_VERBOSE");
   const bool verbose = vb != nullptr && vb[0] != '\0' && vb[0] != '0';
@@ -351,7 +357,8 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
   ea.by_element = t == F64;
   ea.y = y.p;
   ea.b = u.p;
-  for (const SweepShape& sh : cands) {
+  for (size_t c = 0; c < cands.size(); ++c) {
+    const SweepShape& sh = cands[c];
     cudaError_t err = launch_fine(t, EPI_RESID, m.g, sh, E.p, m.nmask.as<uint8_t>(), u.p, ea, s);
     if (err != cudaSuccess) {
       cudaGetLastError();
@@ -368,11 +375,20 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
       fprintf(stderr, "[simpfem tune] %s %dx%dx%d bj=%d bk=%d cx=%d: %.1f us (model %.1f)\n",
               t == F64 ? "f64" : "f32", m.g.nx, m.g.ny, m.g.nz, sh.bj, sh.bk, sh.cx, ms * 1000.f / kTuneReps,
               sweep_cost(t, m.g, sh));
-    if (ms < best) {
-      best = ms;
-      best_sh = sh;
-    }
+    time[c] = ms;
   }
+  // Of the tiles within a hundredth of the fastest, which the events hardly tell apart,
+  // the one that issues the least: alone they run alike, but solves in flight share the
+  // SMs (eight of 512k: ten tiles between 22.8 and 22.9 us gave 221 guarded solves/s in
+  // the order of their work down to 212, the last with a quarter more of it).
+  SweepShape best_sh = default_shape(t, m.g);
+  const float best = cands.empty() ? 0.f : *std::min_element(time.begin(), time.end());
+  int64_t least = INT64_MAX;
+  for (size_t c = 0; c < cands.size(); ++c)
+    if (time[c] < 1e30f && time[c] <= 1.01f * best && sweep_work(m.g, cands[c]) < least) {
+      least = sweep_work(m.g, cands[c]);
+      best_sh = cands[c];
+    }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   m.sh[idx] = best_sh;
