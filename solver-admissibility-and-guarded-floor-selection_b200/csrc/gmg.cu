@@ -209,6 +209,9 @@ static std::vector<double> make_w1(int nf, int nc) {
 // ----------------------------------------------------------------------------
 
 static int64_t div_up64(int64_t a, int64_t b) { return (a + b - 1) / b; }
+static int64_t sweep_blocks(const Grid& g, const SweepShape& sh) {
+  return div_up64(g.ny + 1, sh.bj - 1) * div_up64(g.nz + 1, sh.bk - 1) * div_up64(g.nx + 1, sh.cx);
+}
 
 // Time model of a tile (microseconds): the blocks of an SM run in rounds of as many
 // as registers and shared memory hold; a round walks cx node planes after about two
@@ -225,9 +228,7 @@ static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
   const int64_t smem = es * (18 * nt + 4 * 3 * (sh.bj + 1) * (sh.bk + 1)) + 1024;
   const int64_t resident =
       std::max<int64_t>(1, std::min({65536 / (regs * 32 * warps), 233472 / smem, int64_t(32), 64 / warps}));
-  const int64_t blocks =
-      div_up64(g.ny + 1, sh.bj - 1) * div_up64(g.nz + 1, sh.bk - 1) * div_up64(g.nx + 1, sh.cx);
-  const int64_t per_sm = div_up64(blocks, grid_sm_count()), full = per_sm / resident, rest = per_sm % resident;
+  const int64_t per_sm = div_up64(sweep_blocks(g, sh), grid_sm_count()), full = per_sm / resident, rest = per_sm % resident;
   const double planes = sh.cx + startup;
   double us = launch + full * planes * std::max(latency, issue * resident * warps);
   if (rest) us += planes * std::max(latency, issue * rest * warps);
@@ -236,9 +237,7 @@ static double sweep_cost(DType t, const Grid& g, const SweepShape& sh) {
 
 // Warps times node planes that a sweep issues, halos included.
 static int64_t sweep_work(const Grid& g, const SweepShape& sh) {
-  const int64_t blocks =
-      div_up64(g.ny + 1, sh.bj - 1) * div_up64(g.nz + 1, sh.bk - 1) * div_up64(g.nx + 1, sh.cx);
-  return blocks * div_up64((int64_t)sh.bj * sh.bk, 32) * (sh.cx + 1);
+  return sweep_blocks(g, sh) * div_up64((int64_t)sh.bj * sh.bk, 32) * (sh.cx + 1);
 }
 
 // Candidate tiles of a grid: the z extent in as few equal parts as two rows of 64 threads
@@ -307,6 +306,8 @@ void fine_apply64(Gmg& G, Epi epi, const void* u, EpiArgs ea, cudaStream_t s) {
   ea.by_element = true;
   fine_apply(*G.m, F64, epi, G.E64.p, u, ea, s);
 }
+
+constexpr int64_t kFlushFloats = int64_t(64) << 20;  // 256 MB, twice the L2
 
 // Tuner: time candidate sweep shapes on this mesh and keep the fastest.  The
 // choice is cached per process by grid size and precision, so every mesh of a
@@ -377,18 +378,46 @@ void tune_mesh(Mesh& m, DType t, cudaStream_t s) {
               sweep_cost(t, m.g, sh));
     time[c] = ms;
   }
-  // Of the tiles within a hundredth of the fastest, which the events hardly tell apart,
-  // the one that issues the least: alone they run alike, but solves in flight share the
-  // SMs (eight of 512k: ten tiles between 22.8 and 22.9 us gave 221 guarded solves/s in
-  // the order of their work down to 212, the last with a quarter more of it).
+  // Tiles within a hundredth of the fastest the events hardly tell apart, but from a cold
+  // L2, as among solves in flight that evict each other, they are not alike (512k: ten
+  // tiles between 22.8 and 22.9 us take 28.7 to 33 cold, and eight solves in flight ran
+  // 212 to 220 guarded solves/s with them).  Of these the fastest cold, and of those that
+  // tie again the one that issues the least, in the fewest blocks.
   SweepShape best_sh = default_shape(t, m.g);
   const float best = cands.empty() ? 0.f : *std::min_element(time.begin(), time.end());
-  int64_t least = INT64_MAX;
+  std::vector<size_t> ties;
   for (size_t c = 0; c < cands.size(); ++c)
-    if (time[c] < 1e30f && time[c] <= 1.01f * best && sweep_work(m.g, cands[c]) < least) {
-      least = sweep_work(m.g, cands[c]);
+    if (time[c] < 1e30f && time[c] <= 1.01f * best) ties.push_back(c);
+  if (ties.size() > 1) {
+    DevBuf flush;
+    flush.alloc(sizeof(float) * kFlushFloats);
+    for (size_t c : ties) {
+      time[c] = 1e30f;
+      for (int r = 0; r < 3; ++r) {
+        SF_CUDA(launch_fill_hash(F32, kFlushFloats, 0x9e3779b9u * (uint32_t)(r + 1), flush.p, s));
+        SF_CUDA(cudaEventRecord(e0, s));
+        SF_CUDA(launch_fine(t, EPI_RESID, m.g, cands[c], E.p, m.nmask.as<uint8_t>(), u.p, ea, s));
+        SF_CUDA(cudaEventRecord(e1, s));
+        SF_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.f;
+        SF_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        time[c] = std::min(time[c], ms);
+      }
+    }
+  }
+  float cold = 1e30f;
+  for (size_t c : ties) cold = std::min(cold, time[c]);
+  std::pair<int64_t, int64_t> least(INT64_MAX, 0);
+  for (size_t c : ties) {
+    const std::pair<int64_t, int64_t> cost(sweep_work(m.g, cands[c]), sweep_blocks(m.g, cands[c]));
+    if (verbose)
+      fprintf(stderr, "[simpfem tune] tie bj=%d bk=%d cx=%d: %.1f us, work %lld\n", cands[c].bj, cands[c].bk,
+              cands[c].cx, time[c] * 1000.f, (long long)cost.first);
+    if (time[c] <= 1.01f * cold && cost < least) {
+      least = cost;
       best_sh = cands[c];
     }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   m.sh[idx] = best_sh;
@@ -1569,12 +1598,11 @@ float time_smoother_step(Gmg& G, int l, int reps) {
 // inside its event pair.
 float time_cold(const std::function<void()>& launch, int reps, cudaStream_t st) {
   DevBuf flush;
-  const int64_t flush_vals = int64_t(64) << 20;  // 64 Mi floats = 256 MB
-  flush.alloc(sizeof(float) * flush_vals);
+  flush.alloc(sizeof(float) * kFlushFloats);
   std::vector<cudaEvent_t> ev(2 * reps);
   for (auto& e : ev) SF_CUDA(cudaEventCreate(&e));
   for (int r = 0; r < reps; ++r) {
-    SF_CUDA(launch_fill_hash(F32, flush_vals, 0x9e3779b9u * (uint32_t)(r + 1), flush.p, st));
+    SF_CUDA(launch_fill_hash(F32, kFlushFloats, 0x9e3779b9u * (uint32_t)(r + 1), flush.p, st));
     SF_CUDA(cudaEventRecord(ev[2 * r], st));
     launch();
     SF_CUDA(cudaEventRecord(ev[2 * r + 1], st));
