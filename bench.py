@@ -120,10 +120,10 @@ def run_kernel(args) -> None:
         if args.kernel == "smoother-step":
             _lib.call("simpfem_gmg_time_smoother_step", gmg._h, 0, args.reps, ctypes.byref(avg), _lib.stream_ptr())
             s = 4 if args.precision == "fp32" else 8
-            alg = (4 if args.stack == "plain" else 6) * s * ndof + s * ne + ndof
+            alg = (4 if args.stack == "plain" else 6) * s * ndof + s * ne + ndof // 3
         else:
             _lib.call("simpfem_gmg_time_operator", gmg._h, args.reps, ctypes.byref(avg), _lib.stream_ptr())
-            alg = 8 * ne + 2 * 8 * ndof + ndof
+            alg = 8 * ne + 2 * 8 * ndof + ndof // 3
         torch.cuda.synchronize()
         torch.cuda.profiler.stop()
         print(json.dumps({"kernel": args.kernel, "grid": [nx, ny, nz], "precision": args.precision,

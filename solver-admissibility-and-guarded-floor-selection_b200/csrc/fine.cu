@@ -572,15 +572,15 @@ constexpr int sweep_resident() { return sizeof(T) == 8 ? (FORM == kFaces && DENS
 // which alternate between two buffers.
 //
 // The kernel is bound by latency, not by memory or issue: the grid holds some three
-// blocks of four warps an SM (512k elements: 12-16 % of the warps, issue in 35 % of the
-// cycles in FP64 and 42 % in FP32, reads at the compulsory bytes), and a plane is a chain
+// blocks of three or four warps an SM (512k elements: 16-19 % of the warps, issue in 42 %
+// of the cycles in FP64 and 50 % in FP32, reads at the compulsory bytes), and a plane is a chain
 // of ~300 instructions a warp around one barrier.  Addresses are running pointers and
 // immediate offsets to keep that chain short (the face sums are stored nine to an
 // element for that reason: 9 words apart is also free of bank conflicts in both types).
 //
 // Operator of 1M elements: FP64 87 us before (42 now; its 58 MB at 6.6 TB/s take
 // 9), FP32 45 (28); 512k: FP64 50 (31), FP32 24 (20); 2M in FP32 101 (49).  The element
-// form of the solves from a cold L2, 512k: FP64 product 40.8 us, FP32 Jacobi step 28.7.
+// form of the solves from a cold L2, 512k: FP64 product 39.3 us, FP32 Jacobi step 28.7.
 //
 // FORM: how an element's product is evaluated.  kFaces transforms a face once for
 // two elements, as above.  The products inside a solve -- smoothing steps, residuals
