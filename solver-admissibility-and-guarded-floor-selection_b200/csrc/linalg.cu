@@ -1343,7 +1343,10 @@ cudaError_t launch_pcg_p(int64_t n, const double* z, double* p, const double* sc
 // iteration).  The next z is written after the sum <p, Ap>, whose parts hang on every read
 // of this one.  The coefficients are read once per solve.
 // 7,098 unknowns, 200 iterations: 4.2 ms busy in 6.2 ms of launches -> 0.87 ms; 14,196
-// (two rows a group) 1.16, 22,971 (three) 1.56.
+// (two rows a group) 1.16, 22,971 (three) 1.56.  Its sums are split where the launched
+// form's are chains; against the same iterations in 80 bits (7,260 unknowns, 200 iterations,
+// 180 systems of SIMP contrast 1e-12 and 1e-3) its error is 0.93 of the launched form's
+// (geometric mean, standard error 0.08).
 constexpr int kPcgThreads = 512, kPcgLanes = 8, kPcgRows = kPcgThreads / kPcgLanes, kPcgTerms = 11;
 
 template <int P, typename T>
